@@ -304,13 +304,12 @@ struct oshun_ctx {
     int* d_plane_l = nullptr;    // [nplanes]
     int* d_plane_m = nullptr;    // [nplanes]
     int* d_hplane = nullptr;     // [2*nh]: plane of Re (or -1 for f00), complex flag
-    int* d_seq = nullptr;        // [nh]: source harmonics in stream order, l | (m << 16)
     double* d_ptab = nullptr;    // inv_pr, vr, wj
     double* d_vtab = nullptr;    // vr, U4, U4m1, U2, U2m1, U1, U1m1, U3, Qn, Pn, v^5, v^7
     double* d_dense_ws = nullptr;
     int dense_blocks = 0;
     int* d_status = nullptr;
-    double* d_jw = nullptr;      // [cells][3][8] current partial sums of the pipelined stage
+    double* d_jw = nullptr;      // [cells][3][8] current partial sums of the one-point stage kernels
     Clock* d_clock = nullptr;
     double2* d_stage = nullptr;  // host-layout staging for transfers and slopes
     std::vector<CoefLM> coef_host;   // the coupling table on the host
@@ -356,7 +355,7 @@ struct oshun_ctx {
     double dp = 0, idx = 0, idy = 0, g00_s = 0, g00_inv = 0, g00_gr = 0, c_kpre = 0, kpre = 0;
 
     template <typename TS>
-    StageArgs<TS> stage_args(int in_set, int out_set, int mode) const;
+    StageArgs<TS> stage_args(int in_set, int kind) const;
 };
 
 namespace {
@@ -442,7 +441,7 @@ int pick_mc(int m0) {
 }  // namespace
 
 template <typename TS>
-StageArgs<TS> oshun_ctx::stage_args(int in_set, int out_set, int mode) const {
+StageArgs<TS> oshun_ctx::stage_args(int in_set, int kind) const {
     StageArgs<TS> a;
     std::memset(&a, 0, sizeof(a));
     a.f00_in = f00[in_set]; a.pl_in = (const TS*)pl[in_set]; a.fld_in = (const TS*)fld[in_set];
@@ -453,15 +452,14 @@ StageArgs<TS> oshun_ctx::stage_args(int in_set, int out_set, int mode) const {
     a.inv_pr = d_ptab; a.vr = d_ptab + cfg.nump; a.wj = d_ptab + 2 * cfg.nump;
     a.cells = cells; a.pstride = pstride;
     a.np = cfg.nump; a.nx = cfg.numx; a.ny = cfg.numy; a.l0 = cfg.l0; a.m0 = cfg.m0;
-    a.mode = mode;
+    a.kind = kind;
     a.g00_s = g00_s; a.g00_inv = g00_inv; a.g00_gr = g00_gr;
     a.idx = idx; a.idy = idy;
-    a.seq = d_seq; a.nh = nh; a.err = d_status;
+    a.err = d_status;
+    a.jw = d_jw;
     a.parts = kPartAll;
     a.wait_ns = inject_active ? inject_wait_ns : 1000000000ull;
     a.withhold = inject_active ? inject_withhold : -1;
-    a.jw = d_jw;
-    (void)out_set;
     return a;
 }
 
@@ -623,11 +621,6 @@ int build_tables(oshun_ctx* h) {
         CK(cudaMemcpy(h->d_plane_l, plane_l.data(), sizeof(int) * plane_l.size(), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(h->d_plane_m, plane_m.data(), sizeof(int) * plane_m.size(), cudaMemcpyHostToDevice));
     }
-    std::vector<int> seq;
-    for (int l = 0; l <= l0; ++l)
-        for (int m = 0; m <= std::min(l, m0); ++m) seq.push_back(l | (m << 16));
-    CK(cudaMalloc(&h->d_seq, sizeof(int) * seq.size()));
-    CK(cudaMemcpy(h->d_seq, seq.data(), sizeof(int) * seq.size(), cudaMemcpyHostToDevice));
     CK(cudaMalloc(&h->d_hplane, sizeof(int) * hplane.size()));
     CK(cudaMemcpy(h->d_hplane, hplane.data(), sizeof(int) * hplane.size(), cudaMemcpyHostToDevice));
     CK(cudaMalloc(&h->d_ptab, sizeof(double) * ptab.size()));
@@ -637,26 +630,49 @@ int build_tables(oshun_ctx* h) {
     return OSHUN_OK;
 }
 
-int launch_stage(oshun_ctx* h, int in_set, int B_set, int A_set, int out_set, int mode, int first, double c1,
-                 double c2) {
+// one stage launch: the state sets it reads and writes (out < 0: no stage
+// output) and its weights in units of the step
+struct StageSets {
+    int in, B, A, out, kind;
+    double c1, c2;
+};
+template <typename TS>
+StageArgs<TS> stage_launch_args(const oshun_ctx* h, const StageSets& q, double dt) {
+    StageArgs<TS> a = h->stage_args<TS>(q.in, q.kind);
+    a.f00_B = h->f00[q.B]; a.pl_B = (const TS*)h->pl[q.B]; a.fld_B = (const TS*)h->fld[q.B];
+    a.f00_A = h->f00[q.A]; a.pl_A = (TS*)h->pl[q.A]; a.fld_A = (TS*)h->fld[q.A];
+    if (q.out >= 0) { a.f00_out = h->f00[q.out]; a.pl_out = (TS*)h->pl[q.out]; a.fld_out = (TS*)h->fld[q.out]; }
+    a.c1 = dt * q.c1; a.c2 = q.c2;
+    return a;
+}
+
+// parts, coef, fld_in: a partial right-hand side (the implicit-E actions)
+int launch_stage(oshun_ctx* h, const StageSets& q, int parts = kPartAll, const CoefLM* coef = nullptr,
+                 const void* fld_in = nullptr) {
     cudaError_t e;
-    if (h->fp32) {
-        StageArgs<float> a = h->stage_args<float>(in_set, out_set, mode);
-        a.f00_B = h->f00[B_set]; a.pl_B = (const float*)h->pl[B_set]; a.fld_B = (const float*)h->fld[B_set];
-        a.f00_A = h->f00[A_set]; a.pl_A = (float*)h->pl[A_set]; a.fld_A = (float*)h->fld[A_set];
-        if (out_set >= 0) { a.f00_out = h->f00[out_set]; a.pl_out = (float*)h->pl[out_set]; a.fld_out = (float*)h->fld[out_set]; }
-        a.first = first; a.c1 = c1; a.c2 = c2;
-        e = launch_stage_fp32(a, h->mc, h->stream);
-    } else {
-        StageArgs<double> a = h->stage_args<double>(in_set, out_set, mode);
-        a.f00_B = h->f00[B_set]; a.pl_B = (const double*)h->pl[B_set]; a.fld_B = (const double*)h->fld[B_set];
-        a.f00_A = h->f00[A_set]; a.pl_A = (double*)h->pl[A_set]; a.fld_A = (double*)h->fld[A_set];
-        if (out_set >= 0) { a.f00_out = h->f00[out_set]; a.pl_out = (double*)h->pl[out_set]; a.fld_out = (double*)h->fld[out_set]; }
-        a.first = first; a.c1 = c1; a.c2 = c2;
-        e = launch_stage_fp64(a, h->mc, h->stream);
-    }
+    auto go = [&](auto ts, auto launch) {
+        using TS = decltype(ts);
+        StageArgs<TS> a = stage_launch_args<TS>(h, q, h->cfg.dt);
+        a.parts = parts;
+        if (coef) a.coef = coef;
+        if (fld_in) a.fld_in = (const TS*)fld_in;
+        return launch(a, h->mc, h->stream);
+    };
+    if (h->fp32) e = go(float{}, launch_stage_fp32);
+    else e = go(double{}, launch_stage_fp64);
     if (e != cudaSuccess) { set_error(std::string("rk stage launch: ") + cudaGetErrorString(e)); return OSHUN_ERR_CUDA; }
     return OSHUN_OK;
+}
+
+// RK4 stage k (1..4) of Runge_Kutta_4::advance_p1 (def-RK.cpp:116-142) from
+// set B into set A: the stage inputs are B, Sa, Sb, Sa
+StageSets rk4_sets(int k, int B, int A, int Sa, int Sb) {
+    switch (k) {
+        case 1: return {B, B, A, Sa, kStageFirst, 0.5, 1.0 / 3.0};
+        case 2: return {Sa, B, A, Sb, kStageMid, 0.5, 2.0 / 3.0};
+        case 3: return {Sb, B, A, Sa, kStageMid, 1.0, 1.0 / 3.0};
+        default: return {Sa, B, A, -1, kStageLast, 1.0 / 6.0, 1.0};
+    }
 }
 
 HaloGrid halo_grid(const oshun_ctx* h) {
@@ -677,20 +693,12 @@ int fill_mirror(oshun_ctx* h, int set) {
     return OSHUN_OK;
 }
 
-// RK4 stage k (1..4) of Runge_Kutta_4::advance_p1 (def-RK.cpp:116-142) on set
-// cur: inputs cur, Sa, Sb, Sa; the fourth writes the step's result to cur ^ 1
+// RK4 stage k (1..4) on set cur: inputs cur, 2, 3, 2; the step's result is in cur ^ 1
 int stage_input(const oshun_ctx* h, int k) { return k == 1 ? h->cur : (k == 3 ? 3 : 2); }
 int enqueue_stage(oshun_ctx* h, int k) {
-    const double dt = h->cfg.dt;
-    const int B = h->cur, A = h->cur ^ 1, Sa = 2, Sb = 3;
-    int rc = fill_mirror(h, stage_input(h, k));
+    const int rc = fill_mirror(h, stage_input(h, k));
     if (rc) return rc;
-    switch (k) {
-        case 1: return launch_stage(h, B, B, A, Sa, 0, 1, 0.5 * dt, 1.0 / 3.0);
-        case 2: return launch_stage(h, Sa, B, A, Sb, 0, 0, 0.5 * dt, 2.0 / 3.0);
-        case 3: return launch_stage(h, Sb, B, A, Sa, 0, 0, dt, 1.0 / 3.0);
-        default: return launch_stage(h, Sa, B, A, -1, 0, 0, dt / 6.0, 1.0);
-    }
+    return launch_stage(h, rk4_sets(k, h->cur, h->cur ^ 1, 2, 3));
 }
 
 // Runge_Kutta_4::advance_p1 on set cur -> set cur ^ 1
@@ -874,39 +882,13 @@ ImplicitArgs implicit_args(const oshun_ctx* h) {
     return a;
 }
 
-// one stage launch of a partial right-hand side (the implicit actions)
-int launch_stage_part(oshun_ctx* h, int in_set, int B_set, int A_set, int out_set, int first, double c1, double c2,
-                      int parts, const CoefLM* coef, const void* fld_in) {
-    cudaError_t e;
-    if (h->fp32) {
-        StageArgs<float> a = h->stage_args<float>(in_set, out_set, 0);
-        a.f00_B = h->f00[B_set]; a.pl_B = (const float*)h->pl[B_set]; a.fld_B = (const float*)h->fld[B_set];
-        a.f00_A = h->f00[A_set]; a.pl_A = (float*)h->pl[A_set]; a.fld_A = (float*)h->fld[A_set];
-        if (out_set >= 0) { a.f00_out = h->f00[out_set]; a.pl_out = (float*)h->pl[out_set]; a.fld_out = (float*)h->fld[out_set]; }
-        a.first = first; a.c1 = c1; a.c2 = c2; a.parts = parts; a.coef = coef;
-        if (fld_in) a.fld_in = (const float*)fld_in;
-        e = launch_stage_fp32(a, h->mc, h->stream);
-    } else {
-        StageArgs<double> a = h->stage_args<double>(in_set, out_set, 0);
-        a.f00_B = h->f00[B_set]; a.pl_B = (const double*)h->pl[B_set]; a.fld_B = (const double*)h->fld[B_set];
-        a.f00_A = h->f00[A_set]; a.pl_A = (double*)h->pl[A_set]; a.fld_A = (double*)h->fld[A_set];
-        if (out_set >= 0) { a.f00_out = h->f00[out_set]; a.pl_out = (double*)h->pl[out_set]; a.fld_out = (double*)h->fld[out_set]; }
-        a.first = first; a.c1 = c1; a.c2 = c2; a.parts = parts; a.coef = coef;
-        if (fld_in) a.fld_in = (const double*)fld_in;
-        e = launch_stage_fp64(a, h->mc, h->stream);
-    }
-    if (e != cudaSuccess) { set_error(std::string("rk2 stage launch: ") + cudaGetErrorString(e)); return OSHUN_ERR_CUDA; }
-    return OSHUN_OK;
-}
-
 // One Runge_Kutta_2_Imp update (def-RK.cpp:463-493 and the advance_IE*
 // forms, :515-588) from set S into set T through set U:
 //   Y0 = Y; Yh = F(Y0) h; Y0 += Yh; Yh *= 0.5; Y += Yh; Yh = F(Y0) h/2; Y += Yh
 int enqueue_rk2(oshun_ctx* h, int S, int T, int U, int parts, const CoefLM* coef, const void* fld_in) {
-    const double dt = h->cfg.dt;
-    int rc = launch_stage_part(h, S, S, T, U, 1, dt, 0.5, parts, coef, fld_in);
+    int rc = launch_stage(h, {S, S, T, U, kStageFirst, 1.0, 0.5}, parts, coef, fld_in);
     if (rc) return rc;
-    return launch_stage_part(h, U, S, T, -1, 0, 0.5 * dt, 1.0, parts, coef, fld_in);
+    return launch_stage(h, {U, S, T, -1, kStageLast, 0.5, 1.0}, parts, coef, fld_in);
 }
 
 // Implicit_E_Field::advance (def-ImplicitE.cpp:471-676) on set cur at RK time t
@@ -972,7 +954,7 @@ void free_ctx(oshun_ctx* h) {
             if (h->graph[p][c]) cudaGraphExecDestroy(h->graph[p][c]);
     for (int i = 0; i < 4; ++i) { cudaFree(h->f00[i]); cudaFree(h->pl[i]); cudaFree(h->fld[i]); }
     cudaFree(h->d_coef); cudaFree(h->d_plane_of); cudaFree(h->d_plane_l); cudaFree(h->d_plane_m);
-    cudaFree(h->d_hplane); cudaFree(h->d_seq); cudaFree(h->d_ptab); cudaFree(h->d_vtab); cudaFree(h->d_dense_ws);
+    cudaFree(h->d_hplane); cudaFree(h->d_ptab); cudaFree(h->d_vtab); cudaFree(h->d_dense_ws);
     cudaFree(h->d_status); cudaFree(h->d_clock); cudaFree(h->d_stage); cudaFree(h->d_jw);
     cudaFree(h->d_mom_tab); cudaFree(h->d_mom);
     cudaFree(h->d_ref64); cudaFree(h->d_ref_ts); cudaFree(h->d_refpart); cudaFree(h->d_refkeep); cudaFree(h->d_hx);
@@ -1225,7 +1207,7 @@ int oshun_rhs(oshun_handle h, double* slope_harmonics, double* slope_fields) {
     // slope written to set 2 (scratch), in plane layout
     int rc = fill_mirror(h, h->cur);
     if (rc) return rc;
-    rc = launch_stage(h, h->cur, h->cur, h->cur, 2, 1, 0, 1.0, 1.0);
+    rc = launch_stage(h, {h->cur, h->cur, h->cur, 2, kStageSlope, 1.0, 1.0});
     if (rc) return rc;
     return gather_to_host(h, 2, slope_harmonics, slope_fields, false);
 }
@@ -1670,17 +1652,7 @@ void free_batch(oshun_batch_ctx* b) {
 // of problem h for state parity c, as launch_stage builds it
 template <typename TS>
 StageArgs<TS> batch_stage_args(const oshun_ctx* h, int c, int k, const void* coef_ts) {
-    const double dt = h->cfg.dt;
-    const int B = c, A = c ^ 1, Sa = 2, Sb = 3;
-    const int in_set[4] = {B, Sa, Sb, Sa}, out_set[4] = {Sa, Sb, Sa, -1};
-    const double c1[4] = {0.5 * dt, 0.5 * dt, dt, dt / 6.0}, c2[4] = {1.0 / 3.0, 2.0 / 3.0, 1.0 / 3.0, 1.0};
-    StageArgs<TS> a = h->stage_args<TS>(in_set[k], out_set[k], 0);
-    a.f00_B = h->f00[B]; a.pl_B = (const TS*)h->pl[B]; a.fld_B = (const TS*)h->fld[B];
-    a.f00_A = h->f00[A]; a.pl_A = (TS*)h->pl[A]; a.fld_A = (TS*)h->fld[A];
-    if (out_set[k] >= 0) {
-        a.f00_out = h->f00[out_set[k]]; a.pl_out = (TS*)h->pl[out_set[k]]; a.fld_out = (TS*)h->fld[out_set[k]];
-    }
-    a.first = k == 0; a.c1 = c1[k]; a.c2 = c2[k];
+    StageArgs<TS> a = stage_launch_args<TS>(h, rk4_sets(k + 1, c, c ^ 1, 2, 3), h->cfg.dt);
     a.coef_ts = coef_ts;
     return a;
 }
@@ -2440,13 +2412,13 @@ int oshun_adjoint_vjp(oshun_adjoint a, const double* y, const double* lam_next, 
     int rc;
     // stage inputs of the step (the production stage kernels)
     if ((rc = adj_copy_in(h, B, y))) return rc;
-    if ((rc = launch_stage(h, B, B, A, Sa, 0, 1, 0.5 * dt, 1.0 / 3.0))) return rc;
+    if ((rc = launch_stage(h, rk4_sets(1, B, A, Sa, Sb)))) return rc;
     if ((rc = adj_copy_out(h, Sa, a->s2))) return rc;
-    if ((rc = launch_stage(h, Sa, B, A, Sb, 0, 0, 0.5 * dt, 2.0 / 3.0))) return rc;
+    if ((rc = launch_stage(h, rk4_sets(2, B, A, Sa, Sb)))) return rc;
     if ((rc = adj_copy_out(h, Sb, a->s3))) return rc;
-    if ((rc = launch_stage(h, Sb, B, A, Sa, 0, 0, dt, 1.0 / 3.0))) return rc;
+    if ((rc = launch_stage(h, rk4_sets(3, B, A, Sa, Sb)))) return rc;
     if ((rc = adj_copy_out(h, Sa, a->s4))) return rc;
-    if ((rc = launch_stage(h, Sa, B, A, -1, 0, 0, dt / 6.0, 1.0))) return rc;
+    if ((rc = launch_stage(h, rk4_sets(4, B, A, Sa, Sb)))) return rc;
     if ((rc = adj_copy_out(h, A, a->y1))) return rc;
     CK(cudaMemcpyAsync(a->lam1, lam_next, sizeof(double) * a->n, cudaMemcpyDeviceToDevice, h->stream));
     // collision step transpose at y1

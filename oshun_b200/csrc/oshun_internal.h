@@ -53,7 +53,17 @@ enum : int {
     kPartAll = 255
 };
 
-// Arguments of one fused RHS + RK4 stage launch.  TS is the storage and
+// What a stage launch makes of the slope k of a target, t = k c1 (Runge_Kutta_4::
+// advance_p1's order of roundings, def-RK.cpp:116-142): B the step base
+// (f00_B, pl_B, fld_B), A the RK accumulator, out the next stage input
+enum : int {
+    kStageSlope = 0,   // out = k
+    kStageFirst = 1,   // out = B + t, A = B + t c2
+    kStageMid = 2,     // out = B + t, A += t c2
+    kStageLast = 3     // A += t c2
+};
+
+// Arguments of one fused RHS + RK stage launch.  TS is the storage and
 // arithmetic type of the l >= 1 planes and the fields; f00 is always FP64.
 template <typename TS>
 struct StageArgs {
@@ -73,21 +83,16 @@ struct StageArgs {
     long long cells;      // numx*numy
     long long pstride;    // cells*nump (elements per plane)
     int np, nx, ny, l0, m0;
-    int mode;             // 0: RK stage; 1: write the slope to *_out
-    int first;            // stage 1: A = B + t*c2 instead of A += t*c2
-    double c1, c2;        // t = k*c1; out = B + t; A (+)= t*c2
+    int kind;             // kStage*
+    double c1, c2;        // t = k*c1; A takes t*c2
     double g00_s, g00_inv, g00_gr;   // p0 extrapolation of f00 for G00
     double idx, idy;      // -1/(2dx), -1/(2dy)
-    // bulk-copy pipelined variant
-    const int* seq;       // [nh]: source harmonics in stream order, s | (m << 16)
-    int nh;
     int* err;             // error word (bit 4: a pipeline wait timed out)
     unsigned long long wait_ns;   // a pipeline wait gives up after this many ns (single-problem kernel)
-    int parts;            // kPart* bits of the RHS evaluated (kPartAll: Actions::Adv); any other
-                          // set runs the global-load kernel (the implicit-E actions)
+    int parts;            // kPart* bits of the RHS evaluated (kPartAll: Actions::Adv; others: the implicit-E actions)
     int withhold;         // fault injection for tests: CTA 0's source producer skips this copy (-1: none)
     const void* coef_ts;  // coupling table in the arithmetic type (batched launches)
-    double* jw;           // [cells][3][8]: per-warp partial sums of Jx, Re Jy, Im Jy (single-problem pipeline)
+    double* jw;           // [cells][3][8]: per-warp partial sums of Jx, Re Jy, Im Jy (one-point kernels)
     // x halo columns of the stage input (null: periodic in x).  Side 0 is the
     // x-1 neighbour of column 0, side 1 the x+1 neighbour of column nx-1;
     // one side (hx_side bytes apart): f00 [ny][np] FP64, at hx_pl the l >= 1
@@ -175,9 +180,13 @@ struct CollideBatch {
 };
 
 // launchers (return cudaError_t)
-// pipelined stage kernel (stage_pipe.cu); cudaErrorNotSupported when the shape does not fit
+// one-point pipelined stage kernel (stage_pipe.cu): the full right-hand side, rows of 16-byte multiples;
+// cudaErrorNotSupported when the shape does not fit
 template <typename TS>
 cudaError_t launch_stage_pipe(const StageArgs<TS>& a, int mc, cudaStream_t s);
+// two-point stage kernel (stage_pair.cu): any row length, any parts; cudaErrorNotSupported when the row does not fit
+template <typename TS>
+cudaError_t launch_stage_pair(const StageArgs<TS>& a, cudaStream_t s);
 cudaError_t launch_stage_fp64(const StageArgs<double>& a, int mc, cudaStream_t s);
 // The work of one stage launch: a list of tiles, either of one problem (the
 // kernel parameter) or of a batch of problems (`probs` holds one StageArgs per

@@ -15,18 +15,63 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// out/B/A are base pointers (out may be null: stage 4 has no next input)
+template <typename T>
+__device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
+
+// operand arrays a launch's kind reads per target: Y0 or Y, or both
+__host__ __device__ inline int stage_arrays(int kind) { return kind == kStageSlope ? 0 : kind == kStageMid ? 2 : 1; }
+// RK update of one element of a target from its slope k
+template <typename T>
+__device__ __forceinline__ void rk_update(const int kind, const double c1, const double c2, const T* B, T* A, T* out,
+                                          const long long i, const T k) {
+    if (kind == kStageSlope) { out[i] = k; return; }
+    const T t = mul_rn(k, (T)c1);
+    T y;
+    if (kind == kStageLast) {
+        y = A[i];
+    } else {
+        const T b = B[i];
+        out[i] = add_rn(b, t);
+        y = kind == kStageFirst ? b : A[i];
+    }
+    A[i] = fma_rn(t, (T)c2, y);
+}
+
+// ---------------------------------------------------------------------------
+// E and B of one cell: lane f of the calling half-warp updates field f
+// (Ampere and Faraday with centred differences; J the cell's current)
+// ---------------------------------------------------------------------------
 template <typename TS>
-__device__ __forceinline__ void rk_update(int mode, int first, double c1, double c2, TS* out, const TS* B, TS* A,
-                                          long long i, TS k) {
-    if (mode == 1) { out[i] = k; return; }
-    const TS t = mul_rn(k, (TS)c1);
-    const TS b = B[i];
-    if (out) out[i] = add_rn(b, t);
-    A[i] = fma_rn(t, (TS)c2, first ? b : A[i]);
+__device__ __forceinline__ void field_update(const StageArgs<TS>& a, const int f, const long long cell, const int y,
+                                             const int x, const double Jx, const double Jyr, const double Jyi) {
+    const TS* F = a.fld_in;
+    const long long C = a.cells;
+    const int nx = a.nx, ny = a.ny;
+    const long long row = (long long)y * nx;
+    // the field differenced in x (in y) for this field's slope, and the sign; -1: none
+    const int fx = f == 1 ? 5 : f == 2 ? 4 : f == 4 ? 2 : f == 5 ? 1 : -1;
+    const int fy = f == 0 ? 5 : f == 2 ? 3 : f == 3 ? 2 : f == 5 ? 0 : -1;
+    TS k = TS(0);
+    if (a.parts & (f < 3 ? kPartAmpere : kPartFaraday)) {
+        k = f == 0 ? (TS)Jx : f == 1 ? (TS)(2.0 * Jyr) : f == 2 ? (TS)(-(2.0 * Jyi)) : TS(0);
+        if (fy >= 0) {
+            const long long ym = (long long)(y == 0 ? ny - 1 : y - 1) * nx + x;
+            const long long yp = (long long)(y == ny - 1 ? 0 : y + 1) * nx + x;
+            const TS d = sub_rn(ldg(F + fy * C + ym), ldg(F + fy * C + yp));
+            k = fma_rn((f == 2 || f == 3) ? -(TS)a.idy : (TS)a.idy, d, k);
+        }
+        if (fx >= 0) {
+            const TS vm = (a.hx && x == 0) ? hx_field(a, 0, fx, y) : ldg(F + fx * C + row + (x == 0 ? nx - 1 : x - 1));
+            const TS vp = (a.hx && x == nx - 1) ? hx_field(a, 1, fx, y) : ldg(F + fx * C + row + (x == nx - 1 ? 0 : x + 1));
+            k = fma_rn((f == 1 || f == 5) ? -(TS)a.idx : (TS)a.idx, sub_rn(vm, vp), k);
+        }
+    }
+    rk_update(a.kind, a.c1, a.c2, a.fld_B, a.fld_A, a.fld_out, f * C + cell, k);
 }
 
 // Couplings of source (s, m) at one momentum point.  fr/fi: value, frm/frp

@@ -8,15 +8,8 @@
 namespace oshun {
 namespace {
 
-// CTAs per SM the kernel is compiled for: two for m0 = 0 (few accumulators,
-// 80 registers a thread, half-size ring slots) and at most 384 threads, so
-// that one CTA's tile starts and ends overlap the other's work
-template <int MC, int MAXT>
-constexpr int tile_min_blocks() { return (MC == 0 && MAXT <= 384) ? 2 : 1; }
-
 template <int MC, typename TS, int MAXT>
-__global__ void __launch_bounds__(MAXT, tile_min_blocks<MC, MAXT>())
-    rk_stage_tile_kernel(const StageArgs<TS> a, const int D) {
+__global__ void __launch_bounds__(MAXT, 1) rk_stage_tile_kernel(const StageArgs<TS> a, const int D) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int np = a.np, nx = a.nx, ny = a.ny;
     const int np_pad = (np + 31) & ~31;
@@ -39,11 +32,11 @@ __global__ void __launch_bounds__(MAXT, tile_min_blocks<MC, MAXT>())
     unsigned char* slots = smem + L.off_slots;
     unsigned char* rows = smem + L.off_rows;          // rows l >= 1: [2 buffers][B, A]
     unsigned char* f0row = smem + L.off_f00;          // the f00 row: [B, A]
-    const bool need_B = a.mode != 1;
-    const bool need_A = a.mode != 1 && !a.first;
+    const bool need_B = a.kind != kStageSlope;
+    const bool need_A = need_B && a.kind != kStageFirst;
     // Y0 enters the update only through the stage output and the first
     // stage's Y = Y0 + ...; the last stage (no output) reads none
-    const bool need_Y0 = need_B && (a.first || a.f00_out != nullptr);
+    const bool need_Y0 = need_B && (a.kind == kStageFirst || a.f00_out != nullptr);
 
     const int tid = threadIdx.x;
     const unsigned long long wlim = a.wait_ns;   // every pipeline wait gives up after this
@@ -318,7 +311,7 @@ __global__ void __launch_bounds__(MAXT, tile_min_blocks<MC, MAXT>())
                 // the f00 buffer: its wait was the tile's first
                 if (!dead && pv) {
                     const double k = (double)acc_re(At, 0);
-                    if (a.mode == 1) {
+                    if (a.kind == kStageSlope) {
                         a.f00_out[o] = k;
                     } else {
                         const double* fb = reinterpret_cast<const double*>(f0row);
@@ -326,7 +319,7 @@ __global__ void __launch_bounds__(MAXT, tile_min_blocks<MC, MAXT>())
                         const double b = fb[roff];
                         if (a.f00_out) a.f00_out[o] = add_rn(b, tt);
                         a.f00_A[o] = fma_rn(
-                            tt, a.c2, a.first ? b : reinterpret_cast<const double*>(f0row + L.f00_arr_bytes)[roff]);
+                            tt, a.c2, a.kind == kStageFirst ? b : reinterpret_cast<const double*>(f0row + L.f00_arr_bytes)[roff]);
                     }
                 }
                 __syncwarp();
@@ -424,12 +417,19 @@ __global__ void __launch_bounds__(MAXT, tile_min_blocks<MC, MAXT>())
     }
 }
 
-// E and B of every cell from the current partial sums of the stage kernel
-// (Ampere and Faraday with centred differences, then the RK update)
+// field blockIdx.y of every cell from the current partial sums of the stage
+// kernel (Ampere and Faraday with centred differences, then the RK update):
+// one thread a field, so that a cell's loads are not one thread's chain
 template <typename TS>
 __global__ void __launch_bounds__(256) stage_fields_kernel(const StageArgs<TS> a, const int nw) {
     const long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (cell < a.cells) fields_cell(a, cell, nw);
+    if (cell >= a.cells) return;
+    const int f = blockIdx.y;
+    const int y = (int)(cell / a.nx), x = (int)(cell - (long long)y * a.nx);
+    const double Jx = f == 0 ? cell_current(a, cell, 0, nw) : 0.0;
+    const double Jyr = f == 1 ? cell_current(a, cell, 1, nw) : 0.0;
+    const double Jyi = f == 2 ? cell_current(a, cell, 2, nw) : 0.0;
+    field_update(a, f, cell, y, x, Jx, Jyr, Jyi);
 }
 
 template <int MC, typename TS, int MAXT>
@@ -440,21 +440,12 @@ cudaError_t launch_tile(const StageArgs<TS>& a, int tx, const PipeLayout& L, cud
     }
     const int np_pad = ((a.np + 31) / 32) * 32;
     const long long tiles = (long long)a.ny * ((a.nx + tx - 1) / tx);
-    // as many CTAs as are resident at once (one per SM, two for the m0 = 0
-    // form when its shared memory allows), each walking tiles blockIdx.x + k gridDim.x
-    int per_sm = 1;
-    if (tile_min_blocks<MC, MAXT>() > 1) {
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, rk_stage_tile_kernel<MC, TS, MAXT>, np_pad * tx + 64, L.total);
-        if (e != cudaSuccess || per_sm < 1) { (void)cudaGetLastError(); per_sm = 1; }
-        if (per_sm > tile_min_blocks<MC, MAXT>()) per_sm = tile_min_blocks<MC, MAXT>();
-    }
-    const long long resident = (long long)sm_count() * per_sm;
-    const long long blocks = tiles < resident ? tiles : resident;
+    // persistent CTAs, one per SM, each walking tiles blockIdx.x + k gridDim.x
+    const long long blocks = tiles < sm_count() ? tiles : sm_count();
     rk_stage_tile_kernel<MC, TS, MAXT><<<dim3((unsigned)blocks), dim3(np_pad * tx + 64), L.total, s>>>(a, L.depth);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    stage_fields_kernel<TS><<<dim3((unsigned)((a.cells + 255) / 256)), dim3(256), 0, s>>>(a, np_pad >> 5);
+    stage_fields_kernel<TS><<<dim3((unsigned)((a.cells + 255) / 256), 6), dim3(256), 0, s>>>(a, np_pad >> 5);
     return cudaGetLastError();
 }
 
@@ -467,12 +458,11 @@ cudaError_t pipe_mc(const StageArgs<TS>& a, cudaStream_t s) {
     // the register cap makes the accumulators spill a little.  Registers are
     // granted per SM sub-partition, so a CTA of 9-12 warps costs 12 warps'
     // worth: 168 registers a thread; 13-16 warps: 128.  Consumer threads:
-    //   m0 <= 1, or FP32 with m0 <= 6           up to 448 (16 warps)
+    //   m0 = 1, or FP32 with m0 <= 6            up to 448 (16 warps)
     //   FP64 with m0 <= 6, FP32 with m0 >= 7    up to 320 (12 warps)
     //   FP64 with m0 >= 7 (spills at 168)       up to 192 (8 warps, 255)
     constexpr bool f32 = sizeof(TS) == 4;
-    // m0 = 0: up to 320 consumer threads, two CTAs per SM (tile_min_blocks)
-    constexpr int budget = MC == 0 ? 320 : (MC <= 1 || (f32 && MC <= 6)) ? 448 : (f32 || MC <= 6) ? 320 : 192;
+    constexpr int budget = (MC <= 1 || (f32 && MC <= 6)) ? 448 : (f32 || MC <= 6) ? 320 : 192;
     int tx = budget >= np_pad ? budget / np_pad : 1;
     if (tx > kMaxTx) tx = kMaxTx;
     if (tx > a.nx) tx = a.nx;
@@ -481,25 +471,16 @@ cudaError_t pipe_mc(const StageArgs<TS>& a, cudaStream_t s) {
     const long long per_sm = cells / sm_count();
     if (tx > per_sm) tx = per_sm > 1 ? (int)per_sm : 1;
     const int ncoef = (a.l0 + 1) * (a.m0 + 1);
-    // the deepest source ring that fits `cap` (4 slots at least), else fewer cells a tile
-    auto plan = [&](size_t cap, PipeLayout& L, int& t) -> bool {
-        t = tx;
-        for (;;) {
-            int depth = kDepth;
-            L = pipe_layout(ncoef, t, a.np, a.ny > 1, (int)sizeof(TS), a.m0, depth);
-            while (L.total > cap && depth > 4)
-                L = pipe_layout(ncoef, t, a.np, a.ny > 1, (int)sizeof(TS), a.m0, --depth);
-            if (L.total <= cap || t == 1) break;
-            --t;
-        }
-        return L.total <= cap;
-    };
-    // m0 = 0: half an SM's shared memory, so that two CTAs share it, when
-    // that still leaves 4 slots; otherwise the whole of it
+    // the deepest source ring that fits (4 slots at least), else fewer cells a tile
     PipeLayout L;
-    int txp = tx;
-    if (!(MC == 0 && plan(kSmemHalf, L, txp)) && !plan(kSmemMax, L, txp)) return cudaErrorNotSupported;
-    tx = txp;
+    for (;; --tx) {
+        int depth = kDepth;
+        L = pipe_layout(ncoef, tx, a.np, a.ny > 1, (int)sizeof(TS), a.m0, depth);
+        while (L.total > kSmemMax && depth > 4)
+            L = pipe_layout(ncoef, tx, a.np, a.ny > 1, (int)sizeof(TS), a.m0, --depth);
+        if (L.total <= kSmemMax) break;
+        if (tx == 1) return cudaErrorNotSupported;
+    }
     const int threads = np_pad * tx + 64;
     if (threads <= 256) return launch_tile<MC, TS, 256>(a, tx, L, s);
     if (threads <= 384) return launch_tile<MC, TS, 384>(a, tx, L, s);
@@ -509,13 +490,11 @@ cudaError_t pipe_mc(const StageArgs<TS>& a, cudaStream_t s) {
 
 }  // namespace
 
-// the pipelined stage for m0 <= MC; cudaErrorNotSupported when the shape
-// does not fit it (the caller then uses the global-load kernel)
+// the one-point pipelined stage for 1 <= m0 <= MC; cudaErrorNotSupported when
+// the shape does not fit it (the caller then uses another kernel)
 template <typename TS>
 cudaError_t launch_stage_pipe(const StageArgs<TS>& a, int mc, cudaStream_t s) {
-    if (a.seq == nullptr) return cudaErrorNotSupported;
     switch (mc) {
-        case 0: return pipe_mc<TS, 0>(a, s);
         case 1: return pipe_mc<TS, 1>(a, s);
         case 2: return pipe_mc<TS, 2>(a, s);
         case 3: return pipe_mc<TS, 3>(a, s);

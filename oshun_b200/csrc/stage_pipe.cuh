@@ -45,77 +45,13 @@
 //   (def-VlasovMax.cpp:979-1035); CLEAN_LOW_PC (def-Actions.cpp:240-253).
 #pragma once
 
-#include <type_traits>
-#include <utility>
-
-#include "stage_common.cuh"
+#include "stage_async.cuh"
 
 namespace oshun {
 namespace {
 
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kDepth = 10;                    // source slots in the ring (batched kernel; default)
 constexpr int kMaxDepth = 12;                 // ring slots the barrier area holds
-constexpr unsigned long long kWaitNs = 1000000000ull;   // a pipeline wait gives up after 1 s
-constexpr int kMaxTx = 8;
-constexpr size_t kSmemMax = 227 * 1024;          // dynamic shared memory of one CTA
-constexpr size_t kSmemHalf = (228 * 1024 - 2 * 1024) / 2;   // each of two CTAs on one SM (1 KB reserved each)
-
-template <typename T>
-__device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
-    uint32_t done;
-    // a non-blocking test of the phase (the caller polls with a time bound);
-    // it timed 0.7 % faster per stage than a try_wait that may suspend the thread
-    asm volatile(
-        "{\n\t.reg .pred P1;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, P1;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-// bounded wait for the phase with this parity; false after limit_ns
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          const unsigned long long limit_ns = kWaitNs) {
-    const uint32_t addr = smem_u32(bar);
-    if (mbar_try(addr, parity)) return true;
-    const unsigned long long t0 = global_ns();
-    for (;;) {
-        if (mbar_try(addr, parity)) return true;
-        if (global_ns() - t0 > limit_ns) return false;
-    }
-}
-// global -> shared bulk copy completing on `bar`; 16-byte aligned, size % 16 == 0
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
-__host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // coupling table entry in the arithmetic type (CoefLM converted)
 template <typename TS>
@@ -182,16 +118,6 @@ struct Th {
     bool is0;               // p == 0: H = f[1] hp0
 };
 
-template <int N, typename F, int... I>
-__device__ __forceinline__ void static_for_impl(F&& f, std::integer_sequence<int, I...>) {
-    (f(std::integral_constant<int, I>{}), ...);
-}
-// f(integral_constant<int, 0>) ... f(integral_constant<int, N-1>)
-template <int N, typename F>
-__device__ __forceinline__ void static_for(F&& f) {
-    static_for_impl<N>(f, std::make_integer_sequence<int, N>{});
-}
-
 // Slope accumulators of one target row.  FP64: Re and Im arrays.  FP32:
 // (Re, Im) pairs, which the paired FP32 FMA of sm_100 (__ffma2_rn) updates
 // in one instruction; the Im half of m = 0 is carried along and never stored.
@@ -233,6 +159,8 @@ __device__ __forceinline__ void acc_zero(AccF<MC>& a) {
     for (int m = 0; m <= MC; ++m) a.V[m] = make_float2(0.f, 0.f);
 }
 
+// (stage_pair.cu spells out the roundings these expressions compile to: a batch with
+// m0 >= 1 somewhere runs its m0 = 0 problems here, and they end as they do alone)
 // couplings of source (s, M), s >= 1, into target rows s-1 (R0, I0), s (R1, I1), s+1 (R2, I2)
 template <int MC, int M, typename TS>
 __device__ __forceinline__ void couple_src3_ri(TS (&R0)[MC + 1], TS (&R1)[MC + 1], TS (&R2)[MC + 1],
@@ -426,53 +354,14 @@ __device__ __forceinline__ void couple_f00(AccF<MC>& A2, const CoefT<float>& c, 
     for (int m = 0; m <= MC; ++m) A2.V[m] = make_float2(R2[m], I2[m]);
 }
 
-// field epilogue: J reduction result + Ampere/Faraday, RK update of 6 fields
-// hside: bit 0 the x-1 neighbour, bit 1 the x+1 neighbour comes from the
-// x halo columns (row y)
+// current component k (Jx, Re Jy, Im Jy) of one cell: the per-warp partial
+// sums of the stage kernel, in order (deterministic)
 template <typename TS>
-__device__ __forceinline__ void field_update(const StageArgs<TS>& a, long long cell, long long cxm, long long cxp,
-                                             long long cym, long long cyp, double Jx, double Jyr, double Jyi,
-                                             int hside = 0, long long y = 0) {
-    const TS* F = a.fld_in;
-    const long long C = a.cells;
-    const TS idx = (TS)a.idx, idy = (TS)a.idy;
-    auto xm = [&](int k) { return (hside & 1) ? hx_field(a, 0, k, y) : ldg(F + k * C + cxm); };
-    auto xp = [&](int k) { return (hside & 2) ? hx_field(a, 1, k, y) : ldg(F + k * C + cxp); };
-    const TS dEx = fma_rn(idy, ldg(F + 5 * C + cym) - ldg(F + 5 * C + cyp), (TS)Jx);
-    const TS dEy = fma_rn(-idx, xm(5) - xp(5), (TS)(2.0 * Jyr));
-    const TS dEz = fma_rn(idx, xm(4) - xp(4),
-                          fma_rn(-idy, ldg(F + 3 * C + cym) - ldg(F + 3 * C + cyp), (TS)(-(2.0 * Jyi))));
-    const TS dBx = mul_rn(-idy, ldg(F + 2 * C + cym) - ldg(F + 2 * C + cyp));
-    const TS dBy = mul_rn(idx, xm(2) - xp(2));
-    const TS dBz = fma_rn(-idx, xm(1) - xp(1), mul_rn(idy, ldg(F + 0 * C + cym) - ldg(F + 0 * C + cyp)));
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 0 * C + cell, dEx);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 1 * C + cell, dEy);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 2 * C + cell, dEz);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 3 * C + cell, dBx);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 4 * C + cell, dBy);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 5 * C + cell, dBz);
-}
-
-// E and B of one cell from the per-warp current partial sums of the stage
-// kernel: the warps of the cell in order (deterministic), then field_update
-template <typename TS>
-__device__ __forceinline__ void fields_cell(const StageArgs<TS>& a, const long long cell, const int nw) {
-    const int nx = a.nx, ny = a.ny;
-    const int y = (int)(cell / nx), xc = (int)(cell - (long long)y * nx);
-    const long long row = (long long)y * nx;
-    const long long rym = (long long)(y == 0 ? ny - 1 : y - 1) * nx;
-    const long long ryp = (long long)(y == ny - 1 ? 0 : y + 1) * nx;
-    const double* jc = a.jw + cell * 24;
-    double Jx = 0.0, Jyr = 0.0, Jyi = 0.0;
-    for (int w = 0; w < nw; ++w) {
-        Jx += jc[w];
-        Jyr += jc[8 + w];
-        Jyi += jc[16 + w];
-    }
-    const long long cxm = row + (xc == 0 ? nx - 1 : xc - 1);
-    const long long cxp = row + (xc == nx - 1 ? 0 : xc + 1);
-    const int hside = a.hx ? ((xc == 0 ? 1 : 0) | (xc == nx - 1 ? 2 : 0)) : 0;
-    field_update(a, cell, cxm, cxp, rym + xc, ryp + xc, Jx, Jyr, Jyi, hside, y);
+__device__ __forceinline__ double cell_current(const StageArgs<TS>& a, const long long cell, const int k, const int nw) {
+    const double* jc = a.jw + cell * 24 + k * 8;
+    double J = 0.0;
+    for (int w = 0; w < nw; ++w) J += jc[w];
+    return J;
 }
 
 // the field step of every problem of a batch: one CTA per problem
@@ -481,7 +370,13 @@ __global__ void __launch_bounds__(128) stage_fields_batch_kernel(const unsigned 
                                                                  const int desc_bytes) {
     const StageArgs<TS>& a = *reinterpret_cast<const StageArgs<TS>*>(probs + (size_t)blockIdx.x * desc_bytes);
     const int nw = (a.np + 31) >> 5;
-    for (long long cell = threadIdx.x; cell < a.cells; cell += blockDim.x) fields_cell(a, cell, nw);
+    for (int cell = threadIdx.x; cell < (int)a.cells; cell += blockDim.x) {
+        const int y = cell / a.nx, x = cell - y * a.nx;
+        const double Jx = cell_current(a, cell, 0, nw), Jyr = cell_current(a, cell, 1, nw),
+                     Jyi = cell_current(a, cell, 2, nw);
+#pragma unroll
+        for (int f = 0; f < 6; ++f) field_update(a, f, cell, y, x, Jx, Jyr, Jyi);
+    }
 }
 
 // RK update of one target row's planes from its slopes and the staged Y0 (Bs)
@@ -493,7 +388,7 @@ __device__ __forceinline__ void store_row(const StageArgs<TS>& a, const int mtop
                                           const int rstride) {
     const long long ps = a.pstride;
     auto k_of = [&](int m, int comp) -> TS { return zero ? TS(0) : (comp ? acc_im(K, m) : acc_re(K, m)); };
-    if (a.mode == 1) {
+    if (a.kind == kStageSlope) {
         static_for<MC + 1>([&](auto mcst) {
             constexpr int m = decltype(mcst)::value;
             constexpr int kk = m == 0 ? 0 : 2 * m - 1;
@@ -504,7 +399,7 @@ __device__ __forceinline__ void store_row(const StageArgs<TS>& a, const int mtop
         return;
     }
     const TS c1 = (TS)a.c1, c2 = (TS)a.c2;
-    const bool first = a.first, has_out = out != nullptr;
+    const bool first = a.kind == kStageFirst, has_out = out != nullptr;
     static_for<MC + 1>([&](auto mcst) {
         constexpr int m = decltype(mcst)::value;
         constexpr int kk = m == 0 ? 0 : 2 * m - 1;
@@ -596,7 +491,7 @@ __global__ void __launch_bounds__(MAXT, batch_min_blocks<MC, MAXT>())
     if (tid >= nc) {
         if ((tid & 31) != 0) return;
         const bool src_warp = tid == nc;
-        if (!src_warp && a1.mode == 1) return;   // the slope-only form reads no Y0/Y rows
+        if (!src_warp && a1.kind == kStageSlope) return;   // the slope-only form reads no Y0/Y rows
         int issued = 0;
         bool ok = true;
         int it = blockIdx.x;
@@ -674,9 +569,9 @@ __global__ void __launch_bounds__(MAXT, batch_min_blocks<MC, MAXT>())
                 }
             } else {
                 // row warp: Y0 (and Y) of each target row, up to RD rows ahead of its epilogue
-                const bool need_A = !a.first;
+                const bool need_A = a.kind != kStageFirst;
                 // Y0 enters only through the stage output and the first stage's Y
-                const bool need_Y0 = a.first || a.f00_out != nullptr;
+                const bool need_Y0 = a.kind != kStageLast;
                 const long long base_cell = row + x0;
                 long long q0 = 0;   // first plane of row t (planes in (l, m) order)
                 for (int t = 0; t <= a.l0; ++t) {
@@ -746,8 +641,7 @@ __global__ void __launch_bounds__(MAXT, batch_min_blocks<MC, MAXT>())
         const int np_pad = (np + 31) & ~31;
         const bool has_y = ny > 1;
         const int mstride = a.m0 + 1;
-        const bool need_B = a.mode != 1;
-        const bool need_A = a.mode != 1 && !a.first;
+        const bool need_B = a.kind != kStageSlope;
         const int tx = tile_cells(np, nx, nc, bw.tx_cap);
         const int seg_cells = tx + 2 + (has_y ? 2 * tx : 0);
         const int tiles_x = (nx + tx - 1) / tx;
@@ -813,14 +707,15 @@ __global__ void __launch_bounds__(MAXT, batch_min_blocks<MC, MAXT>())
                 const unsigned char* base = rows + (size_t)rb * 2 * P.row_arr_bytes;
                 if (t == 0) {
                     const double k = (double)acc_re(At, 0);
-                    if (a.mode == 1) {
+                    if (a.kind == kStageSlope) {
                         a.f00_out[o] = k;
                     } else {
                         const double tt = mul_rn(k, a.c1);
                         const double b = reinterpret_cast<const double*>(base)[roff];
                         if (a.f00_out) a.f00_out[o] = add_rn(b, tt);
-                        a.f00_A[o] = fma_rn(tt, a.c2,
-                                            a.first ? b : reinterpret_cast<const double*>(base + P.row_arr_bytes)[roff]);
+                        a.f00_A[o] = fma_rn(
+                            tt, a.c2,
+                            a.kind == kStageFirst ? b : reinterpret_cast<const double*>(base + P.row_arr_bytes)[roff]);
                     }
                 } else {
                     const bool zero = p < (t >= 2 ? min(t - 1, 80) : 0);

@@ -1,21 +1,14 @@
-// Fused RHS + RK4-stage kernels: Actions::Adv (OSHUN-1/def-Actions.cpp:73-94)
-// evaluated on one stage input and folded straight into the stage update of
-// Runge_Kutta_4::advance_p1 (OSHUN-1/def-RK.cpp:110-145).
+// Fused RHS + RK4-stage kernel on global loads, for momentum rows too long
+// for the pipelined kernel of stage_pipe.cu (nump above 512 with m0 = 0, 640
+// to 896 for a few m0, 384 for FP64 with m0 >= 4, or rings that do not fit in
+// shared memory); the launcher below takes the pipelined kernel elsewhere.
 //
-// Work decomposition.  One thread owns one (cell, p) point of every harmonic.
-// Each thread walks the source harmonics row by row (l = 0..l0, all m of a
-// row unrolled) and scatters every coupling of source (l,m) into register
-// accumulators of the only target rows it can reach, l-1, l and l+1.  After
-// source row l has passed, target row l-1 has all of its terms; it is
-// RK-updated and written at once, so the slope never touches HBM.  Per stage
-// and plane HBM sees one read of the stage input, the reads of Y0 and Y and
-// the writes of the next stage input and Y: 3/5/5/3 words over the four
-// stages.
-//
-// This file holds the global-load variant (any nump <= 1024): momentum
-// neighbours by warp shuffles, rows wider than 256 swept in chunks.  The
-// bulk-copy pipelined variant for nump <= 256 is in stage_pipe.cu; the
-// launcher below takes it whenever the shape fits.
+// One thread owns one (cell, p) point of every harmonic, walks the source
+// harmonics row by row (l = 0..l0, all m of a row unrolled) and scatters
+// every coupling of source (l,m) into register accumulators of the only
+// target rows it can reach, l-1, l and l+1; after source row l has passed,
+// target row l-1 is RK-updated and written at once.  Momentum neighbours come
+// by warp shuffles, rows wider than 256 are swept in chunks.
 //
 // Couplings, per source (l,m), G/H as in MakeGH/G00
 // (OSHUN-1/def-VlasovMax.cpp:496-535), Dp = f[p-1]-f[p+1] with the reference's
@@ -43,40 +36,6 @@ constexpr int kPChunk = 256;
 template <typename T>
 __device__ __forceinline__ T ld(const T* p) { return __ldg(p); }
 
-// ---------------------------------------------------------------------------
-// field epilogue: J reduction result + Ampere/Faraday, RK update of 6 fields
-// ---------------------------------------------------------------------------
-// hside: bit 0 the x-1 neighbour, bit 1 the x+1 neighbour comes from the
-// x halo columns (row y)
-template <typename TS>
-__device__ __forceinline__ void field_update(const StageArgs<TS>& a, long long cell, long long cxm, long long cxp,
-                                             long long cym, long long cyp, double Jx, double Jyr, double Jyi,
-                                             int hside, long long y) {
-    const TS* F = a.fld_in;
-    const long long C = a.cells;
-    const TS idx = (TS)a.idx, idy = (TS)a.idy;
-    auto xm = [&](int k) { return (hside & 1) ? hx_field(a, 0, k, y) : ld(F + k * C + cxm); };
-    auto xp = [&](int k) { return (hside & 2) ? hx_field(a, 1, k, y) : ld(F + k * C + cxp); };
-    TS dEx = 0, dEy = 0, dEz = 0, dBx = 0, dBy = 0, dBz = 0;
-    if (a.parts & kPartAmpere) {
-        // J: Ex += Jx, Ey += Re J11, Ez += -Im J11 with J11 = 2 * (f11 quadrature)
-        dEx = fma_rn(idy, ld(F + 5 * C + cym) - ld(F + 5 * C + cyp), (TS)Jx);
-        dEy = fma_rn(-idx, xm(5) - xp(5), (TS)(2.0 * Jyr));
-        dEz = fma_rn(idx, xm(4) - xp(4), fma_rn(-idy, ld(F + 3 * C + cym) - ld(F + 3 * C + cyp), (TS)(-(2.0 * Jyi))));
-    }
-    if (a.parts & kPartFaraday) {
-        dBx = mul_rn(-idy, ld(F + 2 * C + cym) - ld(F + 2 * C + cyp));
-        dBy = mul_rn(idx, xm(2) - xp(2));
-        dBz = fma_rn(-idx, xm(1) - xp(1), mul_rn(idy, ld(F + 0 * C + cym) - ld(F + 0 * C + cyp)));
-    }
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 0 * C + cell, dEx);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 1 * C + cell, dEy);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 2 * C + cell, dEz);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 3 * C + cell, dBx);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 4 * C + cell, dBy);
-    rk_update(a.mode, a.first, a.c1, a.c2, a.fld_out, a.fld_B, a.fld_A, 5 * C + cell, dBz);
-}
-
 // RK epilogue of target row t at one (cell, p) point
 template <int MC, typename TS>
 __device__ __forceinline__ void row_epilogue(const StageArgs<TS>& a, const int* plane_of, int t, int p, bool pv,
@@ -90,11 +49,11 @@ __device__ __forceinline__ void row_epilogue(const StageArgs<TS>& a, const int* 
         if (p < nzero) { kr = 0; ki = 0; }
         if (!pv) continue;
         if (t == 0) {
-            rk_update<double>(a.mode, a.first, a.c1, a.c2, a.f00_out, a.f00_B, a.f00_A, o, (double)kr);
+            rk_update<double>(a.kind, a.c1, a.c2, a.f00_B, a.f00_A, a.f00_out, o, (double)kr);
         } else {
             const long long q = plane_of[t * mstride + m];
-            rk_update(a.mode, a.first, a.c1, a.c2, a.pl_out, a.pl_B, a.pl_A, q * a.pstride + o, kr);
-            if (m > 0) rk_update(a.mode, a.first, a.c1, a.c2, a.pl_out, a.pl_B, a.pl_A, (q + 1) * a.pstride + o, ki);
+            rk_update(a.kind, a.c1, a.c2, a.pl_B, a.pl_A, a.pl_out, q * a.pstride + o, kr);
+            if (m > 0) rk_update(a.kind, a.c1, a.c2, a.pl_B, a.pl_A, a.pl_out, (q + 1) * a.pstride + o, ki);
         }
     }
 }
@@ -225,12 +184,11 @@ __global__ void __launch_bounds__(256) rk_stage_kernel(const StageArgs<TS> a) {
         sj[2][threadIdx.y][warp] = jyi;
     }
     __syncthreads();
-    if (threadIdx.x != 0 || !cv) return;
+    if (threadIdx.x >= 6 || !cv) return;
     double Jx = 0.0, Jyr = 0.0, Jyi = 0.0;
     const int nw = (min(np, (int)blockDim.x) + 31) >> 5;
     for (int w = 0; w < nw; ++w) { Jx += sj[0][threadIdx.y][w]; Jyr += sj[1][threadIdx.y][w]; Jyi += sj[2][threadIdx.y][w]; }
-    const int hside = a.hx ? ((cx == 0 ? 1 : 0) | (cx == a.nx - 1 ? 2 : 0)) : 0;
-    field_update(a, cell, cxm, cxp, cym, cyp, Jx, Jyr, Jyi, hside, cyy);
+    field_update(a, threadIdx.x, cell, (int)cyy, (int)cx, Jx, Jyr, Jyi);
 }
 
 // ---------------------------------------------------------------------------
@@ -250,13 +208,14 @@ cudaError_t launch_mc(const StageArgs<TS>& a, cudaStream_t s) {
 
 template <typename TS>
 cudaError_t launch_stage(const StageArgs<TS>& a, int mc, cudaStream_t s) {
-    // the pipelined kernel where the shape fits it (the full right-hand side),
-    // else the global-load kernel
-    if (a.parts == kPartAll) {
-        const cudaError_t e = launch_stage_pipe<TS>(a, mc, s);
-        if (e != cudaErrorNotSupported) return e;
-        (void)cudaGetLastError();
-    }
+    // The full right-hand side of m0 >= 1 on rows of 16-byte multiples: the
+    // one-point pipelined kernel.  m0 = 0, other row lengths and partial
+    // right-hand sides: the two-point one.  Rows too long for either: global loads.
+    cudaError_t e = cudaErrorNotSupported;
+    if (a.m0 > 0 && a.parts == kPartAll) e = launch_stage_pipe<TS>(a, mc, s);
+    if (e == cudaErrorNotSupported) e = launch_stage_pair<TS>(a, s);
+    if (e != cudaErrorNotSupported) return e;
+    (void)cudaGetLastError();
     switch (mc) {
         case 0: return launch_mc<TS, 0>(a, s);
         case 1: return launch_mc<TS, 1>(a, s);
