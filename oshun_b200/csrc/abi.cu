@@ -728,6 +728,7 @@ CollideArgs collide_args(oshun_ctx* h, int do_ee, int do_l1, int do_lm, int nsub
     a.np = np; a.l0 = c.l0; a.m0 = c.m0;
     a.mmax_coll = c.if_implicit1D ? 0 : c.m0;
     a.do_ee = do_ee; a.do_l1 = do_l1; a.do_lm = do_lm;
+    a.unit_planes = collide_unit_planes(np, c.l0, c.m0, a.mmax_coll, do_l1, do_lm);
     a.if_tridiagonal = c.if_tridiagonal;
     a.nsub = nsub; a.hsub = hsub; a.Dt = Dt;
     a.ee_implicit = (c.flags & OSHUN_FLAG_IMPLICIT_EE) ? kEeImplicitSweeps : 0;
@@ -1574,9 +1575,8 @@ int oshun_plane_index(oshun_handle h, int l, int m, int* plane) {
 //   4 x batched RK4 stage launch (one persistent kernel each, over the
 //       (problem, tile) list of the whole batch),
 //   device clock advance,
-//   per group of problems with equal ceil(nump/32) and on the same side of
-//       8 resident collision CTAs per SM: one batched collision launch over
-//       their (problem, cell) list,
+//   per group of problems of one collision form: one batched collision
+//       launch over their (problem, cell) list,
 //   device clock commit.
 // The stage tiles (consumer threads per CTA, cells per tile) are chosen by
 // oshun_batch_autotune, which times each candidate on the batch itself.
@@ -1607,11 +1607,8 @@ struct oshun_batch_ctx {
     std::vector<unsigned char> h_a1[2][4];   // kernel parameter of each launch (a problem's descriptor)
     // collision launches
     struct Group {
-        int E = 0;
+        int form = 0;
         size_t smem = 0;
-        int4* d_chunks = nullptr;   // chunked form (CTAs of `warps` cells of one problem), or none
-        long long nchunks = 0;
-        int warps = 0, tab_doubles = 0;
         CollideArgs* d_args[2] = {nullptr, nullptr};   // per parity
         int2* d_items = nullptr;
         long long nitems = 0;
@@ -1636,7 +1633,7 @@ void free_batch(oshun_batch_ctx* b) {
     batch_drop_graphs(b);
     for (oshun_ctx* h : b->P)
         if (h) free_ctx(h);
-    for (auto& g : b->groups) { cudaFree(g.d_args[0]); cudaFree(g.d_args[1]); cudaFree(g.d_items); cudaFree(g.d_chunks); }
+    for (auto& g : b->groups) { cudaFree(g.d_args[0]); cudaFree(g.d_args[1]); cudaFree(g.d_items); }
     cudaFree(b->d_desc); cudaFree(b->d_coef_ts); cudaFree(b->d_items);
     cudaFree(b->d_clocks); cudaFree(b->d_dt); cudaFree(b->d_collide); cudaFree(b->d_status);
     for (int i = 0; i < 2; ++i) {
@@ -1733,12 +1730,12 @@ int batch_enqueue_step(oshun_batch_ctx* b, int c) {
     }
     CK(launch_clock_advance(b->d_clocks, b->d_dt, n, b->stream));
     // fork: each group goes to the least loaded of the three streams, largest
-    // first (load = cells x ceil(nump/32)); join before the clock commit
+    // first (load = cells x row length); join before the clock commit
     CK(cudaEventRecord(b->ev_fork, b->stream));
     for (int i = 0; i < 2; ++i) CK(cudaStreamWaitEvent(b->side[i], b->ev_fork, 0));
     std::vector<int> order(b->groups.size());
     for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
-    auto load_of = [&](int i) { return (double)b->groups[i].nitems * b->groups[i].E; };
+    auto load_of = [&](int i) { return (double)b->groups[i].nitems * b->groups[i].form; };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return load_of(x) > load_of(y); });
     double load[3] = {0.0, 0.0, 0.0};
     cudaStream_t lanes[3] = {b->stream, b->side[0], b->side[1]};
@@ -1747,9 +1744,8 @@ int batch_enqueue_step(oshun_batch_ctx* b, int c) {
         const auto& g = b->groups[gi];
         const int li = (int)(std::min_element(load, load + 3) - load);
         load[li] += load_of(gi);
-        CollideBatch cb{g.d_args[c ^ 1], g.d_items, g.nitems, g.d_chunks, g.nchunks, g.warps, g.tab_doubles,
-                        (int)(g.smem / sizeof(double))};   // the new state is parity c^1
-        e = launch_collide_batch(cb, g.E, b->fp32 ? 1 : 0, g.smem, lanes[li]);
+        CollideBatch cb{g.d_args[c ^ 1], g.d_items, g.nitems};   // the new state is parity c^1
+        e = launch_collide_batch(cb, g.form, b->fp32 ? 1 : 0, g.smem, lanes[li]);
         if (e != cudaSuccess) break;
     }
     for (int i = 0; i < 2; ++i) {
@@ -1914,25 +1910,16 @@ int oshun_batch_create(const oshun_cfg* cfgs, int n, const int* collide, oshun_b
         CKB(cudaMemcpy(b->d_dt, dt.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
         CKB(cudaMemcpy(b->d_collide, b->collide.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
     }
-    // collision groups by ceil(nump / 32) and, within one nump class, by
-    // whether a cell's shared memory allows at least 8 resident one-warp CTAs
-    // per SM (the pivots of every l take 2 l0 nump doubles), so that a few
-    // problems with large l0 do not set the footprint of all the others;
+    // collision groups by the form of the collision kernel (row lengths);
     // descriptors per state parity, (problem, cell) items
-    auto ctas_per_sm = [](size_t smem) {
-        const size_t k = (size_t)228 * 1024 / (smem + 1024);   // 1 KB reserved per CTA
-        return (int)std::min<size_t>(16, std::max<size_t>(1, k));
-    };
-    for (int E = 1; E <= 8; ++E)
-    for (int wide = 1; wide >= 0; --wide) {
+    for (int form = 1; form <= 32; ++form) {
         oshun_batch_ctx::Group g;
-        g.E = E;
+        g.form = form;
         std::vector<CollideArgs> args[2];
         std::vector<int2> items;
         for (int i = 0; i < n; ++i) {
             oshun_ctx* h = b->P[i];
-            if (!b->collide[i] || (h->cfg.nump + 31) / 32 != E) continue;
-            if ((ctas_per_sm(collide_tri_smem_per_cell(h->cfg.nump, h->cfg.l0)) >= 8) != (wide == 1)) continue;
+            if (!b->collide[i] || collide_form(h->cfg.nump) != form) continue;
             const int local = (int)args[0].size();
             for (int c = 0; c < 2; ++c) {
                 const int cur0 = h->cur;
@@ -1947,45 +1934,6 @@ int oshun_batch_create(const oshun_cfg* cfgs, int n, const int* collide, oshun_b
             for (long long cell = 0; cell < h->cells; ++cell) items.push_back(make_int2(local, (int)cell));
         }
         if (items.empty()) continue;
-        // chunked form where it keeps at least as many warps resident: CTAs of
-        // W cells of one problem share the problem's velocity tables in shared
-        // memory (per SM: 228 KB of shared memory with 1 KB reserved per CTA,
-        // 64 K registers granted in 256-register units per warp, 32 CTAs)
-        {
-            int npmax = 0;
-            for (const auto& a : args[0]) npmax = std::max(npmax, a.np);
-            const size_t tab = 12 * (size_t)npmax, celld = g.smem / sizeof(double);
-            auto resident = [](size_t bytes, int W, int regs) {
-                const int by_smem = (int)((size_t)228 * 1024 / (bytes + 1024));
-                const int per_warp = (regs * 32 + 255) / 256 * 256;
-                const int by_regs = 65536 / (per_warp * W);
-                return W * std::min(std::min(by_smem, by_regs), 32);
-            };
-            const int f32 = b->fp32 ? 1 : 0;
-            const int plain = resident(g.smem, 1, collide_batch_regs(E, f32, 0));
-            const int rchunk = collide_batch_regs(E, f32, 1);
-            int bestW = 0, bestWarps = 0;
-            for (int W = 1; W <= 8; ++W) {
-                const size_t bytes = collide_chunk_smem(W, (int)tab, (int)celld);
-                if (bytes > (size_t)227 * 1024) break;
-                const int warps = resident(bytes, W, rchunk);
-                if (warps >= bestWarps) { bestWarps = warps; bestW = W; }
-            }
-            if (bestW > 0 && bestWarps >= plain) {
-                std::vector<int4> chunks;
-                for (size_t k = 0; k < items.size();) {
-                    const int p = items[k].x, c0 = items[k].y;
-                    int cnt = 0;
-                    while (k < items.size() && items[k].x == p && cnt < bestW) { ++k; ++cnt; }
-                    chunks.push_back(make_int4(p, c0, cnt, 0));
-                }
-                g.warps = bestW;
-                g.tab_doubles = (int)tab;
-                g.nchunks = (long long)chunks.size();
-                CKB(cudaMalloc(&g.d_chunks, sizeof(int4) * chunks.size()));
-                CKB(cudaMemcpy(g.d_chunks, chunks.data(), sizeof(int4) * chunks.size(), cudaMemcpyHostToDevice));
-            }
-        }
         b->groups.push_back(g);
         auto& gg = b->groups.back();
         gg.nitems = (long long)items.size();

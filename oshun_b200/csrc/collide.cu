@@ -22,6 +22,9 @@
 //        convergence rule) on one complex right-hand side.
 #include <float.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "oshun_internal.h"
 
 namespace oshun {
@@ -625,43 +628,6 @@ __device__ void ee_substeps(const CollideArgs& a, const Smem& s) {
     }
 }
 
-// The same substeps with the four slopes from one call site of ee_slope:
-// one inlined copy of its scans and logarithms instead of four, for the lane
-// kernels of short rows (the stage updates are the ones above)
-__device__ void ee_substeps_one_site(const CollideArgs& a, const Smem& s) {
-    const StepP sp = step_params(a);
-    const int n = a.np;
-    const int lane = threadIdx.x & 31;
-    for (int sub = 0; sub < sp.nsub; ++sub) {
-        const double h = sp.hsub;
-        for (int k = lane; k < n; k += 32) { s.f0[k] = s.f[k]; s.f1[k] = s.f[k]; }
-        __syncwarp();
-        for (int st = 0; st < 4; ++st) {
-            ee_slope(a, s, st == 3 ? s.f0 : s.f1, s.fh);
-            if (st == 0) {
-                for (int k = lane; k < n; k += 32) {
-                    double t = s.fh[k] * (0.5 * h);
-                    s.f1[k] += t; t *= 1.0 / 3.0; s.f[k] += t;
-                }
-            } else if (st == 1) {
-                for (int k = lane; k < n; k += 32) {
-                    s.f1[k] = s.f0[k];
-                    double t = s.fh[k] * (0.5 * h);
-                    s.f1[k] += t; t *= 2.0 / 3.0; s.f[k] += t;
-                }
-            } else if (st == 2) {
-                for (int k = lane; k < n; k += 32) {
-                    double t = s.fh[k] * h;
-                    s.f0[k] += t; t *= 1.0 / 3.0; s.f[k] += t;
-                }
-            } else {
-                for (int k = lane; k < n; k += 32) s.f[k] += s.fh[k] * (h / 6.0);
-            }
-            __syncwarp();
-        }
-    }
-}
-
 // the backward-Euler e-e step alone, one warp per cell (the collision
 // kernels then run with do_ee = 0)
 __global__ void __launch_bounds__(32) ee_implicit_kernel(const CollideArgs a) {
@@ -829,46 +795,35 @@ __global__ void __launch_bounds__(32) collide_warp_kernel(const CollideArgs a) {
     }
 }
 
-// Tridiagonal collision step for nump <= 32 E, one warp per cell (1-warp
-// CTAs, grid-stride over cells), rows in registers:
-//   1. f00 e-e substeps and reset_coeff as above.
-//   2. per collided l, the Thomas pivots of each lane's run of p (c'_i and
-//      1/(b_i - c'_{i-1} a_i), 1/b_0 at i = 0; TridiagonalSolve,
-//      def-Nmethods.cpp:152-159) from a warp scan of the pivot recurrence
-//      (lane_pivots); then the collided planes of that l in batches of P: lane j holds p in
-//      [jE, jE+E) of each row in registers (the next batch's rows are loaded
-//      while this one is solved).  Both recurrences of TridiagonalSolve --
-//      d'_i = (d_i - a_i d'_{i-1}) / (b_i - c'_{i-1} a_i) forward,
-//      x_i = d'_i - c'_i x_{i+1} backward -- are affine maps of the previous
-//      value.  Each lane composes its run, a warp scan gives the value entering
-//      the run, and the lane applies the recursion inside its run.  The maps'
-//      multipliers depend on l only, so their composition and scan are done
-//      once per l and only the offsets are scanned per plane.
-// Shared memory (doubles): 4 scalars, tri_a, tri_b, tri_c, scat, then the
-// e-e/reset work arrays (the pivots stay in registers, per l).
-__device__ Smem carve_lane(double* base, int np) {
-    Smem s;
-    s.sc = base;
-    s.tri_a = base + 4; s.tri_b = s.tri_a + np; s.tri_c = s.tri_b + np; s.scat = s.tri_c + np;
-    s.df0 = s.scat + np; s.ddf0 = s.df0 + np;
-    s.f = s.ddf0 + np; s.f0 = s.f + np; s.f1 = s.f0 + np; s.fh = s.f1 + np;
-    s.I4 = s.fh + np; s.I2 = s.I4 + np; s.J1 = s.I2 + np;
-    s.chunk = nullptr;
-    return s;
-}
-__host__ __device__ inline size_t lane_smem_doubles(int np, int /*l0*/) {
-    return 4 + 13 * (size_t)np;   // scalars, tri_a/b/c, scat, e-e and reset work arrays
-}
+// Tridiagonal collision step for nump <= 512, one CTA per cell:
+//   1. f00 e-e substeps and the coefficients of reset_coeff with one thread
+//      per momentum point (two from 257 points on): f, the RK4 stages and the
+//      point's velocity tables in registers, the three cumulative integrals as
+//      warp scans joined through the warps' totals, neighbours through shared
+//      memory, three barriers a slope.
+//   2. the collided planes, by groups of G lanes (8 for rows of up to 64
+//      points, 16 up to 128, else 32) so that a lane's run of p is 4 to 8
+//      points long and a warp solves 32/G planes at once: a group takes units
+//      of up to unit_planes planes of one l, forms that l's Thomas pivots for
+//      each lane's run (lane_pivots; TridiagonalSolve, def-Nmethods.cpp:
+//      152-159) and solves its planes one after the other, rows in registers,
+//      the next plane's rows loading meanwhile.  Both recurrences of
+//      TridiagonalSolve -- d'_i = (d_i - a_i d'_{i-1}) / (b_i - c'_{i-1} a_i)
+//      forward, x_i = d'_i - c'_i x_{i+1} backward -- are affine maps of the
+//      previous value.  Each lane composes its run, a scan over the group gives
+//      the value entering the run, and the lane applies the recursion inside
+//      its run.  The maps' multipliers depend on l only, so their composition
+//      and scan are done once per unit and only the offsets are scanned per
+//      plane.
 
 // Thomas pivots of harmonic order l for this lane's run of p, c'_i and
 // 1/(b_i - c'_{i-1} a_i), with b_i = tri_b_i + 1 - ll1 scat_i (tri_b_0 left
 // out for l > 1), as TridiagonalSolve forms them (def-Nmethods.cpp:152-159).
 // c'_i = c_i / (b_i - a_i c'_{i-1}) is a linear-fractional map of c'_{i-1},
 // the 2x2 matrix [[0, c_i], [-a_i, b_i]] acting on (c'_{i-1}, 1): each lane
-// composes its run's matrices, a warp scan of the products (rescaled by
-// powers of two, which leaves the maps unchanged) gives the value entering
-// the run, and the lane applies the recursion inside its run.  No per-l
-// table is kept, so a cell needs 4 + 13 np doubles of shared memory.
+// composes its run's matrices, a scan over the group (rescaled by powers of
+// two, which leaves the maps unchanged) gives the value entering
+// the run, and the lane applies the recursion inside its run.
 struct M22 {
     double a, b, c, d;
 };
@@ -885,41 +840,48 @@ __device__ __forceinline__ M22 m22_rescale(M22 x) {
     }
     return x;
 }
-template <int E>
-__device__ __forceinline__ void lane_pivots(const Smem& s, const int l, const int n, const int i0, double (&cp)[E],
-                                            double (&id)[E]) {
-    const int lane = threadIdx.x & 31;
+// the coefficients of one cell in shared memory (np each)
+struct TriRows {
+    double *a, *b, *c, *scat;
+};
+template <int G, int R>
+__device__ __forceinline__ void lane_pivots(const TriRows& s, const int l, const int n, const int i0, double (&cp)[R],
+                                            double (&id)[R]) {
+    const int gl = threadIdx.x & (G - 1);
     const double ll1 = l * ((-0.5) * (l + 1.0));
-    double b[E];
     M22 m{1.0, 0.0, 0.0, 1.0};
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
+    for (int e = 0; e < R; ++e) {
         const int i = i0 + e;
-        b[e] = 1.0;
+        id[e] = 1.0;   // b_i until the recursion below
         if (i < n) {
-            b[e] = (i == 0 && l > 1 ? 0.0 : s.tri_b[i]) + (1.0 - ll1 * s.scat[i]);
-            m = m22_mul(M22{0.0, s.tri_c[i], -s.tri_a[i], b[e]}, m);
+            const double a = s.a[i], c = s.c[i];
+            const double b = (i == 0 && l > 1 ? 0.0 : s.b[i]) + (1.0 - ll1 * s.scat[i]);
+            id[e] = b;
+            m = M22{c * m.c, c * m.d, fma(-a, m.a, b * m.c), fma(-a, m.b, b * m.d)};
         }
+        if (e % 8 == 7) m = m22_rescale(m);
     }
     m = m22_rescale(m);
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const M22 o{__shfl_up_sync(kFull, m.a, off), __shfl_up_sync(kFull, m.b, off),
-                    __shfl_up_sync(kFull, m.c, off), __shfl_up_sync(kFull, m.d, off)};
-        if (lane >= off) m = m22_rescale(m22_mul(m, o));
+    for (int off = 1; off < G; off <<= 1) {
+        const M22 o{__shfl_up_sync(kFull, m.a, off, G), __shfl_up_sync(kFull, m.b, off, G),
+                    __shfl_up_sync(kFull, m.c, off, G), __shfl_up_sync(kFull, m.d, off, G)};
+        if (gl >= off) m = m22_rescale(m22_mul(m, o));
     }
-    const double xb = __shfl_up_sync(kFull, m.b, 1), xd = __shfl_up_sync(kFull, m.d, 1);
-    double cprev = lane == 0 ? 0.0 : xb / xd;
+    const double xb = __shfl_up_sync(kFull, m.b, 1, G), xd = __shfl_up_sync(kFull, m.d, 1, G);
+    double cprev = gl == 0 ? 0.0 : xb / xd;
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
+    for (int e = 0; e < R; ++e) {
         const int i = i0 + e;
         if (i < n) {
+            const double b = id[e];
             if (i == 0) {
-                id[e] = 1.0 / b[e];
-                cprev = s.tri_c[0] / b[e];
+                id[e] = 1.0 / b;
+                cprev = s.c[0] / b;
             } else {
-                id[e] = 1.0 / (b[e] - cprev * s.tri_a[i]);
-                cprev = s.tri_c[i] * id[e];
+                id[e] = 1.0 / (b - cprev * s.a[i]);
+                cprev = s.c[i] * id[e];
             }
             cp[e] = cprev;
         } else {
@@ -929,235 +891,382 @@ __device__ __forceinline__ void lane_pivots(const Smem& s, const int l, const in
     }
 }
 
-template <typename TP, int E, int P>
-__device__ __forceinline__ void collide_lane_cell(const CollideArgs& a, const long long cell, double* smem) {
+// velocity tables of a thread's PT momentum points k0 .. k0+PT-1
+template <int PT>
+struct PointTab {
+    double U4[PT], U4m[PT], U2[PT], U2m[PT], U1p[PT], U1mp[PT];   // I4, I2 terms of k; the J1 term of k + 1
+    double U3[PT], V5[PT], V7[PT], Qn[PT], Pn[PT], Pm[PT];        // Pm: Pn of k - 1
+};
+template <int PT>
+__device__ __forceinline__ void load_tab(const CollideArgs& a, const int k0, PointTab<PT>& t) {
     const int n = a.np;
-    const int l0 = a.l0;
-    const int lane = threadIdx.x & 31;
-    TP* planes = reinterpret_cast<TP*>(a.planes);
-    const bool solve = a.do_l1 || a.do_lm;
-    const Smem s = carve_lane(smem, n);
-    const int i0 = lane * E;   // first p of this lane's run
+#pragma unroll
+    for (int j = 0; j < PT; ++j) {
+        const int k = k0 + j;
+        const bool in = k < n, up = k + 1 < n;
+        const int kc = in ? k : 0;
+        t.U4[j] = in ? __ldg(a.U4 + kc) : 0.0;     // 0 at k = 0 (the tables start at 1)
+        t.U4m[j] = in ? __ldg(a.U4m1 + kc) : 0.0;
+        t.U2[j] = in ? __ldg(a.U2 + kc) : 0.0;
+        t.U2m[j] = in ? __ldg(a.U2m1 + kc) : 0.0;
+        t.U1p[j] = up ? __ldg(a.U1 + kc + 1) : 0.0;
+        t.U1mp[j] = up ? __ldg(a.U1m1 + kc + 1) : 0.0;
+        t.U3[j] = in ? __ldg(a.U3 + kc) : 1.0;
+        t.V5[j] = k < a.NB ? __ldg(a.V5 + kc) : 0.0;
+        t.V7[j] = k < a.NB ? __ldg(a.V7 + kc) : 0.0;
+        t.Qn[j] = in ? __ldg(a.Qn + kc) : 0.0;
+        t.Pn[j] = up ? __ldg(a.Pn + kc) : 0.0;
+        t.Pm[j] = in && k > 0 ? __ldg(a.Pn + kc - 1) : 0.0;
+    }
+}
+// shared memory of one cell's CTA (doubles): tri_a, tri_b, tri_c, scat [np],
+// f and G with a point of padding on both sides, the warps' totals [3][16]
+__host__ __device__ inline size_t cell_smem_doubles(int np, int pts) { return 4 * (size_t)np + 2 * ((size_t)pts + 2) + 48; }
+struct CellSmem {
+    TriRows tri;
+    double *f, *g, *tot;   // f, g: index -1 .. pts
+};
+__device__ __forceinline__ CellSmem carve_cell(double* base, int np, int pts) {
+    CellSmem s;
+    s.tri.a = base; s.tri.b = base + np; s.tri.c = base + 2 * np; s.tri.scat = base + 3 * np;
+    s.f = base + 4 * np + 1;
+    s.g = s.f + pts + 2;
+    s.tot = s.g + pts + 1;
+    return s;
+}
 
-    // plane batches: l, first plane, count (planes of one l are consecutive)
-    auto batch_first = [&](int& l, int& j) {
-        l = 1; j = 0;
-        while (l <= l0 && !collided(a, l, 0)) ++l;
-    };
-    auto batch_next = [&](int& l, int& j) {
-        const int nq = 1 + 2 * min(min(l, a.m0), a.mmax_coll);
-        j += P;
-        if (j < nq) return;
-        j = 0;
-        do { ++l; } while (l <= l0 && !collided(a, l, 0));
-    };
-    // a batch's rows as stored: the next batch's loads stay in flight during
-    // this batch's solve in the storage type (FP32 planes take half the
-    // registers of their FP64 values) ...
-    auto load_raw = [&](long long cell, int l, int j, TP (&r)[P][E]) {
-        if (l > l0) return;
-        const int nq = 1 + 2 * min(min(l, a.m0), a.mmax_coll);
-        const long long q0 = a.plane_of[l * (a.m0 + 1)] + j;
+// The cumulative integrals I4, I2 (k' <= k) and J1 (k' > k) of f at a thread's
+// points, and the whole I4, I2 (S4, S2).  fm, fp: the neighbours.
+template <int PT>
+__device__ __forceinline__ void cell_scans(const PointTab<PT>& t, const double (&f)[PT], const double (&fm)[PT],
+                                           const double (&fp)[PT], double* tot, double (&I4)[PT], double (&I2)[PT],
+                                           double (&J1)[PT], double& S4, double& S2) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double s4 = 0.0, s2 = 0.0, s1 = 0.0;
 #pragma unroll
-        for (int b = 0; b < P; ++b) {
-            const TP* g = planes + (q0 + b) * a.pstride + cell * n;
+    for (int j = 0; j < PT; ++j) {
+        I4[j] = fma(t.U4[j], f[j], t.U4m[j] * fm[j]);
+        I2[j] = fma(t.U2[j], f[j], t.U2m[j] * fm[j]);
+        J1[j] = fma(t.U1p[j], fp[j], t.U1mp[j] * f[j]);
+        s4 += I4[j]; s2 += I2[j]; s1 += J1[j];
+    }
 #pragma unroll
-            for (int e = 0; e < E; ++e) r[b][e] = (j + b < nq && i0 + e < n) ? g[i0 + e] : TP(0);
-        }
-    };
-    // ... and widened to FP64, the plane's profile added, when the batch is solved
-    auto widen = [&](int l, int j, const TP (&r)[P][E], double (&d)[P][E]) {
-        const int nq = 1 + 2 * min(min(l, a.m0), a.mmax_coll);
-        const long long q0 = a.plane_of[l * (a.m0 + 1)] + j;
+    for (int off = 1; off < 32; off <<= 1) {
+        const double v4 = __shfl_up_sync(kFull, s4, off);
+        const double v2 = __shfl_up_sync(kFull, s2, off);
+        const double v1 = __shfl_down_sync(kFull, s1, off);
+        if (lane >= off) { s4 += v4; s2 += v2; }
+        if (lane + off < 32) s1 += v1;
+    }
+    if (lane == 31) { tot[warp] = s4; tot[16 + warp] = s2; }
+    if (lane == 0) tot[32 + warp] = s1;
+    double r4 = __shfl_up_sync(kFull, s4, 1), r2 = __shfl_up_sync(kFull, s2, 1);
+    double r1 = __shfl_down_sync(kFull, s1, 1);
+    if (lane == 0) { r4 = 0.0; r2 = 0.0; }
+    if (lane == 31) r1 = 0.0;
+    __syncthreads();
+    double b4 = 0.0, b2 = 0.0, b1 = 0.0;
+    S4 = 0.0; S2 = 0.0;
+    for (int w = 0; w < nw; ++w) {
+        if (w == warp) { b4 = S4; b2 = S2; }
+        S4 += tot[w]; S2 += tot[16 + w];
+        if (w > warp) b1 += tot[32 + w];
+    }
+    r4 += b4; r2 += b2; r1 += b1;
 #pragma unroll
-        for (int b = 0; b < P; ++b) {
+    for (int j = 0; j < PT; ++j) {
+        r4 += I4[j]; I4[j] = r4;
+        r2 += I2[j]; I2[j] = r2;
+    }
 #pragma unroll
-            for (int e = 0; e < E; ++e) d[b][e] = (double)r[b][e];
-            const float* rp = (j + b < nq) ? ref_row<TP>(a, q0 + b) : nullptr;
-            if (rp) {
+    for (int j = PT - 1; j >= 0; --j) {
+        r1 += J1[j];
+        J1[j] = r1;
+    }
+}
+// a thread's points to shared memory, then its neighbours back
+template <int PT>
+__device__ __forceinline__ void neighbours(double* buf, const int k0, const double (&v)[PT], double (&lo)[PT],
+                                           double (&hi)[PT]) {
 #pragma unroll
-                for (int e = 0; e < E; ++e)
-                    if (i0 + e < n) d[b][e] += (double)__ldg(rp + i0 + e);
-            }
-        }
-    };
-
-    TP raw[P][E];
-    double cur[P][E];
-    {
-        int bl, bj;
-        batch_first(bl, bj);
-        if (solve) load_raw(cell, bl, bj, raw);   // in flight during the e-e step
-        for (int k = lane; k < n; k += 32) s.f[k] = a.f00[cell * n + k];
-        __syncwarp();
-        if (a.do_ee) {
-            if constexpr (E <= 3) ee_substeps_one_site(a, s);
-            else ee_substeps(a, s);
-            for (int k = lane; k < n; k += 32) a.f00[cell * n + k] = s.f[k];
-        }
-        if (!solve) return;
-        flm_reset(a, s, s.f);
-        // this lane's tri_a (forward multiplier -a_i id_i)
-        double ta[E];
+    for (int j = 0; j < PT; ++j) buf[k0 + j] = v[j];
+    __syncthreads();
 #pragma unroll
-        for (int e = 0; e < E; ++e) ta[e] = (i0 + e < n) ? s.tri_a[i0 + e] : 0.0;
-
-        int cl = -1;   // l of the per-l constants below
-        double id[E], cp[E], Af[5], Ab[5];
-        if (bl <= l0) widen(bl, bj, raw, cur);
-        while (bl <= l0) {
-            const int l = bl, j = bl <= l0 ? bj : 0;
-            const int nq = 1 + 2 * min(min(l, a.m0), a.mmax_coll);
-            int nl = bl, nj = bj;
-            batch_next(nl, nj);
-            if (nl <= l0) load_raw(cell, nl, nj, raw);
-            if (l != cl) {
-                // per-l constants: pivots of this lane's run and the scan multipliers
-                cl = l;
-                lane_pivots<E>(s, l, n, i0, cp, id);
-                double A = 1.0, B = 1.0;
-#pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int i = i0 + e;
-                    if (i < n) A = (i == 0) ? 0.0 : A * (-(ta[e] * id[e]));
-                }
-#pragma unroll
-                for (int e = E - 1; e >= 0; --e) {
-                    const int i = i0 + e;
-                    if (i < n) B = (i == n - 1) ? 0.0 : B * (-cp[e]);
-                }
-#pragma unroll
-                for (int k = 0, off = 1; k < 5; ++k, off <<= 1) {
-                    Af[k] = A;
-                    Ab[k] = B;
-                    const double Ap = __shfl_up_sync(kFull, A, off);
-                    const double Bp = __shfl_down_sync(kFull, B, off);
-                    if (lane >= off) A *= Ap;
-                    if (lane + off < 32) B *= Bp;
-                }
-            }
-            // forward: run offsets, scan, recursion inside the run
-            double Bf[P];
-#pragma unroll
-            for (int b = 0; b < P; ++b) {
-                double B = 0.0;
-#pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int i = i0 + e;
-                    if (i < n) B = (i == 0) ? cur[b][e] * id[e] : (cur[b][e] - B * ta[e]) * id[e];
-                }
-                Bf[b] = B;
-            }
-#pragma unroll
-            for (int k = 0, off = 1; k < 5; ++k, off <<= 1) {
-#pragma unroll
-                for (int b = 0; b < P; ++b) {
-                    const double Bp = __shfl_up_sync(kFull, Bf[b], off);
-                    if (lane >= off) Bf[b] += Af[k] * Bp;
-                }
-            }
-#pragma unroll
-            for (int b = 0; b < P; ++b) {
-                double d = __shfl_up_sync(kFull, Bf[b], 1);
-#pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int i = i0 + e;
-                    if (i < n) {
-                        d = (i == 0) ? cur[b][e] * id[e] : (cur[b][e] - d * ta[e]) * id[e];
-                        cur[b][e] = d;
-                    }
-                }
-            }
-            // backward
-            double Bb[P];
-#pragma unroll
-            for (int b = 0; b < P; ++b) {
-                double B = 0.0;
-#pragma unroll
-                for (int e = E - 1; e >= 0; --e) {
-                    const int i = i0 + e;
-                    if (i < n) B = (i == n - 1) ? cur[b][e] : cur[b][e] - cp[e] * B;
-                }
-                Bb[b] = B;
-            }
-#pragma unroll
-            for (int k = 0, off = 1; k < 5; ++k, off <<= 1) {
-#pragma unroll
-                for (int b = 0; b < P; ++b) {
-                    const double Bp = __shfl_down_sync(kFull, Bb[b], off);
-                    if (lane + off < 32) Bb[b] += Ab[k] * Bp;
-                }
-            }
-            const long long q0 = a.plane_of[l * (a.m0 + 1)] + j;
-#pragma unroll
-            for (int b = 0; b < P; ++b) {
-                double x = __shfl_down_sync(kFull, Bb[b], 1);
-                TP* g = planes + (q0 + b) * a.pstride + cell * n;
-                const float* rp = (j + b < nq) ? ref_row<TP>(a, q0 + b) : nullptr;
-#pragma unroll
-                for (int e = E - 1; e >= 0; --e) {
-                    const int i = i0 + e;
-                    if (i < n) {
-                        x = (i == n - 1) ? cur[b][e] : cur[b][e] - cp[e] * x;
-                        if (j + b < nq) g[i] = (TP)(rp ? x - (double)__ldg(rp + i) : x);
-                    }
-                }
-            }
-            if (nl <= l0) widen(nl, nj, raw, cur);
-            bl = nl; bj = nj;
-        }
-        __syncwarp();
+    for (int j = 0; j < PT; ++j) {
+        lo[j] = j > 0 ? v[j > 0 ? j - 1 : 0] : buf[k0 - 1];
+        hi[j] = j + 1 < PT ? v[j + 1 < PT ? j + 1 : 0] : buf[k0 + PT];
     }
 }
 
-// rows of up to 96 points (E <= 3) leave 12.3 KB of shared memory per cell:
-// the kernel is held to 128 registers so that 16 cells are resident per SM
-template <int E>
-constexpr int lane_min_blocks() { return E <= 3 ? 16 : 1; }
-template <typename TP, int E, int P>
-__global__ void __launch_bounds__(32, lane_min_blocks<E>()) collide_lane_kernel(const CollideArgs a) {
-    extern __shared__ double smem[];
-    for (long long cell = blockIdx.x; cell < a.cells; cell += gridDim.x) collide_lane_cell<TP, E, P>(a, cell, smem);
+// EE_isotropic_conserva::Getslope (def-FokkerPlanck.cpp:192-267): fh = C_ee(fin)
+template <int PT>
+__device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSmem& s, const PointTab<PT>& t,
+                                              const int k0, const double v0s, const double v1s,
+                                              const double (&fin)[PT], double (&fh)[PT]) {
+    const int n = a.np;
+    double fm[PT], fp[PT], I4[PT], I2[PT], J1[PT], S4, S2;
+    neighbours<PT>(s.f, k0, fin, fm, fp);
+    const double fa = s.f[0], fb = s.f[1];
+    cell_scans<PT>(t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
+    // flux G_n; the first NB cells use the parabolic fit near v = 0
+    double G[PT], Gm[PT], Gp[PT];
+#pragma unroll
+    for (int j = 0; j < PT; ++j) {
+        if (k0 + j < a.NB) {
+            const double f00 = (fa - fb * v0s / v1s) / (1.0 - v0s / v1s);
+            const double i2s = f00 * t.U3[j] / 3.0 + (fb - f00) * t.V5[j] / v1s * 0.2;
+            const double i4s = f00 * t.V5[j] * 0.2 + (fb - f00) * t.V7[j] / (v1s * 7.0);
+            G[j] = fin[j] * i4s + (t.U3[j] * fin[j] - 3.0 * i2s) * J1[j];
+        } else {
+            const double i2 = -3.0 * (I2[j] * J1[j]);
+            G[j] = fma(fma(t.U3[j], J1[j], I4[j]), fin[j], i2);
+        }
+    }
+    neighbours<PT>(s.g, k0, G, Gm, Gp);
+    const double norm = a.c_kpre * log_ee(4.0 * M_PI * S2, 4.0 * M_PI * S4, a.density_np);
+#pragma unroll
+    for (int j = 0; j < PT; ++j) {
+        const int k = k0 + j;
+        // D_k = (G_k - G_{k+1}) P_k for k < n-1, D_{n-1} = G_{n-1}
+        const double D = k < n - 1 ? (G[j] - Gp[j]) * t.Pn[j] : G[j];
+        const double v = k == 0 ? ((-G[j]) * (2.0 / v0s) - D) : ((Gm[j] - G[j]) * t.Pm[j] - D);
+        fh[j] = v * t.Qn[j] * norm;
+    }
 }
 
-// batched form: work item = (problem, cell); the problems share E
-template <typename TP, int E, int P>
-__global__ void __launch_bounds__(32) collide_lane_batch_kernel(const CollideBatch b) {
+// the collided planes of the cell over the CTA's groups of G lanes: units in
+// order of falling l, group g takes units g, g + groups, ...
+template <typename TP, int G, int R>
+__device__ __forceinline__ void cell_solves(const CollideArgs& a, const TriRows& s, const long long cell) {
+    constexpr int kSteps = G == 8 ? 3 : (G == 16 ? 4 : 5);
+    const int n = a.np;
+    const int gl = threadIdx.x & (G - 1);
+    const int ng = blockDim.x / G;
+    TP* planes = reinterpret_cast<TP*>(a.planes);
+    const int i0 = gl * R;   // first p of this lane's run
+    const int C = a.unit_planes;
+    auto nplanes_of = [&](int l) { return collided(a, l, 0) ? 1 + 2 * min(min(l, a.m0), a.mmax_coll) : 0; };
+    // this group's unit: k-th of order l; l = 0: none left
+    int l = a.l0, k = threadIdx.x / G;
+    auto settle = [&]() {
+        while (l >= 1) {
+            const int u = (nplanes_of(l) + C - 1) / C;
+            if (k < u) return;
+            k -= u;
+            --l;
+        }
+        l = 0;
+    };
+    // the planes of one l split evenly over its units
+    auto split = [&](int& first, int& count) {
+        const int nq = nplanes_of(l), u = (nq + C - 1) / C;
+        first = (int)((long long)nq * k / u);
+        count = (int)((long long)nq * (k + 1) / u) - first;
+    };
+    double ta[R];
+#pragma unroll
+    for (int e = 0; e < R; ++e) ta[e] = (i0 + e < n) ? s.a[i0 + e] : 0.0;
+    settle();
+    while (__any_sync(kFull, l >= 1)) {
+        int j0 = 0, cnt = 0;
+        if (l >= 1) split(j0, cnt);
+        const int most = __reduce_max_sync(kFull, cnt);
+        const long long q0 = l >= 1 ? (long long)a.plane_of[l * (a.m0 + 1)] + j0 : 0;
+        TP* g = planes + q0 * a.pstride + cell * n + i0;
+        // rows as stored: the next plane's loads stay in flight during this plane's solve
+        TP raw[R];
+        auto load = [&](int b) {
+#pragma unroll
+            for (int e = 0; e < R; ++e) raw[e] = (b < cnt && i0 + e < n) ? g[b * a.pstride + e] : TP(0);
+        };
+        load(0);
+        // per-l constants: pivots of this lane's run and the scan multipliers
+        double id[R], cp[R], Af[kSteps], Ab[kSteps];
+        lane_pivots<G, R>(s, l >= 1 ? l : 1, n, i0, cp, id);
+        {
+            double A = 1.0, B = 1.0;
+#pragma unroll
+            for (int e = 0; e < R; ++e) {
+                const int i = i0 + e;
+                if (i < n) A = (i == 0) ? 0.0 : A * (-(ta[e] * id[e]));
+            }
+#pragma unroll
+            for (int e = R - 1; e >= 0; --e) {
+                const int i = i0 + e;
+                if (i < n) B = (i == n - 1) ? 0.0 : B * (-cp[e]);
+            }
+#pragma unroll
+            for (int t = 0, off = 1; t < kSteps; ++t, off <<= 1) {
+                const double Ap = __shfl_up_sync(kFull, A, off, G);
+                const double Bp = __shfl_down_sync(kFull, B, off, G);
+                Af[t] = gl >= off ? A : 0.0;
+                Ab[t] = gl + off < G ? B : 0.0;
+                if (gl >= off) A *= Ap;
+                if (gl + off < G) B *= Bp;
+            }
+        }
+        for (int b = 0; b < most; ++b) {
+            double cur[R];
+#pragma unroll
+            for (int e = 0; e < R; ++e) cur[e] = (double)raw[e];
+            const float* rp = (b < cnt) ? ref_row<TP>(a, q0 + b) : nullptr;
+            if (rp) {   // the plane's profile (FP32 planes)
+#pragma unroll
+                for (int e = 0; e < R; ++e)
+                    if (i0 + e < n) cur[e] += (double)__ldg(rp + i0 + e);
+            }
+            if (b + 1 < most) load(b + 1);
+            // forward: run offset, scan, recursion inside the run
+            double B = 0.0;
+#pragma unroll
+            for (int e = 0; e < R; ++e) B = (cur[e] - B * ta[e]) * id[e];   // a_0 = 0; beyond the row nothing reads it
+#pragma unroll
+            for (int t = 0, off = 1; t < kSteps; ++t, off <<= 1) B = fma(Af[t], __shfl_up_sync(kFull, B, off, G), B);
+            double d = __shfl_up_sync(kFull, B, 1, G);
+            if (gl == 0) d = 0.0;
+#pragma unroll
+            for (int e = 0; e < R; ++e) {
+                if (i0 + e < n) d = (cur[e] - d * ta[e]) * id[e];
+                cur[e] = i0 + e < n ? d : 0.0;
+            }
+            // backward: x_{n-1} = d'_{n-1}; c'_{n-1} = 0 and the points beyond are zero
+            B = 0.0;
+#pragma unroll
+            for (int e = R - 1; e >= 0; --e) B = cur[e] - cp[e] * B;
+#pragma unroll
+            for (int t = 0, off = 1; t < kSteps; ++t, off <<= 1) B = fma(Ab[t], __shfl_down_sync(kFull, B, off, G), B);
+            double x = __shfl_down_sync(kFull, B, 1, G);
+            if (gl == G - 1) x = 0.0;
+            TP* o = g + b * a.pstride;
+#pragma unroll
+            for (int e = R - 1; e >= 0; --e) {
+                x = cur[e] - cp[e] * x;
+                if (b < cnt && i0 + e < n) o[e] = (TP)(rp ? x - (double)__ldg(rp + i0 + e) : x);
+            }
+        }
+        k += ng;
+        settle();
+    }
+}
+
+template <typename TP, int G, int R, int PT>
+__device__ __forceinline__ void collide_cell(const CollideArgs& a, const long long cell, double* smem) {
+    const int n = a.np;
+    const int pts = PT * (int)blockDim.x;
+    const CellSmem s = carve_cell(smem, n, pts);
+    const int k0 = PT * (int)threadIdx.x;
+    const double* vr = a.vr;
+    const bool solve = a.do_l1 || a.do_lm;
+    PointTab<PT> t;
+    load_tab<PT>(a, k0, t);
+    const double v0s = vr[0] * vr[0], v1s = vr[1] * vr[1];
+    const StepP sp = step_params(a);
+    double f[PT];
+#pragma unroll
+    for (int j = 0; j < PT; ++j) f[j] = k0 + j < n ? a.f00[cell * n + k0 + j] : 0.0;
+    if (threadIdx.x == 0) { s.f[-1] = 0.0; s.f[pts] = 0.0; s.g[-1] = 0.0; s.g[pts] = 0.0; }
+    if (a.do_ee) {
+        // RK4 substeps of Explicit_EC_FP::loop (RungeKutta4_ee::advance, def-FokkerPlanck.cpp:518-553)
+        const double h = sp.hsub;
+        for (int sub = 0; sub < sp.nsub; ++sub) {
+            double f0[PT], f1[PT], fh[PT];
+#pragma unroll
+            for (int j = 0; j < PT; ++j) { f0[j] = f[j]; f1[j] = f[j]; }
+            // one call site of the slope for the four stages
+            for (int st = 0; st < 4; ++st) {
+                cell_ee_slope<PT>(a, s, t, k0, v0s, v1s, f1, fh);
+                const double w = st < 2 ? 0.5 * h : (st == 2 ? h : h / 6.0);
+                const double u = st == 1 ? 2.0 / 3.0 : (st == 3 ? 1.0 : 1.0 / 3.0);
+#pragma unroll
+                for (int j = 0; j < PT; ++j) {
+                    const double d = fh[j] * w;
+                    f1[j] = f0[j] + d;
+                    f[j] = fma(d, u, f[j]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < PT; ++j)
+            if (k0 + j < n) a.f00[cell * n + k0 + j] = f[j];
+    }
+    if (!solve) return;
+    // Implicit_FLM_step::reset_coeff (def-FokkerPlanck.cpp:808-939), tridiagonal part
+    double fm[PT], fp[PT], I2[PT], I0[PT], J1m[PT], S4, S2;
+    neighbours<PT>(s.f, k0, f, fm, fp);
+    cell_scans<PT>(t, f, fm, fp, s.tot, I2, I0, J1m, S4, S2);
+    const double I2_temperature = S4 * (4.0 * M_PI);
+    const double I0_density = S2 * (4.0 * M_PI);
+    const double lnee = log_ee(I0_density, I2_temperature, a.density_np);
+    const double zlnei = zlog_ei(I0_density, I2_temperature, a.density_np, a.Zeta);
+    const double scale = (-1.0) * lnee * a.kpre * sp.Dt;
+#pragma unroll
+    for (int j = 0; j < PT; ++j) {
+        const int k = k0 + j;
+        if (k >= n) continue;
+        const double v = vr[k];
+        double i2 = I2[j] * (4.0 * M_PI);
+        i2 /= v * v;
+        const double i0 = I0[j] * (4.0 * M_PI);
+        const double j1m = J1m[j] * (4.0 * M_PI * v);
+        const double t1 = i0 + (2.0 * j1m - i2) / 3.0;
+        const double t2 = (i2 + j1m) / 3.0;
+        double sc = (k == 0) ? 0.0 : t1 * lnee;
+        sc += zlnei * I0_density;
+        sc /= t.U3[j];
+        sc *= a.kpre * sp.Dt;
+        s.tri.scat[k] = sc;
+        double ta = 0.0, tb = 0.0, tc = 0.0;
+        if (k == 0) {
+            tb = 8.0 * M_PI * f[j] * scale;
+        } else if (k < n - 1) {
+            const double vp = vr[k + 1], vm = vr[k - 1];
+            const double IvDnDm1 = 1.0 / (v * 0.5 * (vp - vm) * (v - vm));
+            const double IvDnDp1 = 1.0 / (v * 0.5 * (vp - vm) * (vp - v));
+            const double Ivsq2Dn = 1.0 / (v * v * (vp - vm));
+            tb = (8.0 * M_PI * f[j] - t2 * (IvDnDm1 + IvDnDp1)) * scale;
+            ta = (t2 * IvDnDm1 - t1 * Ivsq2Dn) * scale;
+            tc = (t2 * IvDnDp1 + t1 * Ivsq2Dn) * scale;
+        }
+        s.tri.a[k] = ta; s.tri.b[k] = tb; s.tri.c[k] = tc;
+    }
+    __syncthreads();
+    cell_solves<TP, G, R>(a, s.tri, cell);
+}
+
+// What it measured (B200, the collision launch, one cell a warp before -> now): 256 cells of 128 points, l0 = 1, ten e-e
+// substeps 0.21 -> 0.115 ms for the three calls of a step; 384 cells of 432 points, l0 = 31 (the staged-chunk kernel
+// before) 0.88 -> 0.2 ms; Weibel (16384 cells of 96 points, 48 planes) equal in FP64, 0.65 -> 0.60 ms in the FP32 split;
+// 512 uneven 1D problems 9.0 -> 7.7 ms a step.  Long e-e runs on few cells wait on the slope's three barriers and its
+// logarithms; large grids on the latency of the solves at 16 warps an SM (128 registers).
+// The forms: K = G R / 8 (the row's points, rounded up to the form's, over 8).
+// One thread a point up to 256 points, two beyond.
+constexpr int form_lanes(int K) { return K <= 8 ? 8 : (K <= 16 ? 16 : 32); }
+constexpr int form_run(int K) { return 8 * K / form_lanes(K); }
+constexpr int form_points(int K) { return K <= 32 ? 1 : 2; }
+constexpr int form_warps(int K) { return (8 * K + 32 * form_points(K) - 1) / (32 * form_points(K)); }
+// resident CTAs per SM: 16 warps of 128 registers up to 256 points
+constexpr int form_blocks(int K) { return K <= 32 ? 16 / form_warps(K) : 1; }
+template <typename TP, int K>
+__global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K)) collide_cell_kernel(const CollideArgs a) {
     extern __shared__ double smem[];
+    for (long long cell = blockIdx.x; cell < a.cells; cell += gridDim.x) {
+        collide_cell<TP, form_lanes(K), form_run(K), form_points(K)>(a, cell, smem);
+        __syncthreads();
+    }
+}
+
+// batched form: work item = (problem, cell); the problems share the form
+template <typename TP, int K>
+__global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K)) collide_cell_batch_kernel(const CollideBatch b) {
+    extern __shared__ double smem[];
+    __shared__ CollideArgs a;
+    static_assert(sizeof(CollideArgs) % 4 == 0, "copied word by word");
     for (long long it = blockIdx.x; it < b.nitems; it += gridDim.x) {
         const int2 w = b.items[it];
-        collide_lane_cell<TP, E, P>(b.probs[w.x], (long long)w.y, smem);
-        __syncwarp();
-    }
-}
-
-// chunked batched form: a CTA of W warps takes W cells of one problem (one
-// cell per warp) and first stages the problem's twelve velocity tables (vr,
-// U4, U4m1, U2, U2m1, U1, U1m1, U3, Qn, Pn, v^5, v^7: contiguous from vr) and
-// its arguments in shared memory, so the e-e slopes and the coefficient
-// build read them there instead of from L2
-constexpr int kArgsDoubles = (int)((sizeof(CollideArgs) + 15) / 16 * 2);
-template <typename TP, int E, int P>
-__global__ void __launch_bounds__(256, 1) collide_lane_chunk_kernel(const CollideBatch b) {
-    extern __shared__ __align__(16) double smem[];
-    CollideArgs* sa = reinterpret_cast<CollideArgs*>(smem);
-    double* tab = smem + kArgsDoubles;
-    double* work = tab + b.tab_doubles;
-    const int warp = threadIdx.x >> 5;
-    for (long long ch = blockIdx.x; ch < b.nchunks; ch += gridDim.x) {
-        const int4 c = b.chunks[ch];
-        const CollideArgs& ga = b.probs[c.x];
-        const int np = ga.np;
-        if (threadIdx.x == 0) *sa = ga;
-        for (int i = threadIdx.x; i < 12 * np; i += blockDim.x) tab[i] = ga.vr[i];
+        const int* src = reinterpret_cast<const int*>(b.probs + w.x);
+        for (int i = threadIdx.x; i < (int)(sizeof(CollideArgs) / 4); i += blockDim.x) reinterpret_cast<int*>(&a)[i] = src[i];
         __syncthreads();
-        if (threadIdx.x == 0) {
-            sa->vr = tab; sa->U4 = tab + np; sa->U4m1 = tab + 2 * np; sa->U2 = tab + 3 * np;
-            sa->U2m1 = tab + 4 * np; sa->U1 = tab + 5 * np; sa->U1m1 = tab + 6 * np; sa->U3 = tab + 7 * np;
-            sa->Qn = tab + 8 * np; sa->Pn = tab + 9 * np; sa->V5 = tab + 10 * np; sa->V7 = tab + 11 * np;
-        }
-        __syncthreads();
-        if (warp < c.z) collide_lane_cell<TP, E, P>(*sa, (long long)c.y + warp, work + (size_t)warp * b.cell_doubles);
+        collide_cell<TP, form_lanes(K), form_run(K), form_points(K)>(a, (long long)w.y, smem);
         __syncthreads();
     }
 }
@@ -1201,65 +1310,83 @@ cudaError_t launch_collide(const CollideArgs& a, cudaStream_t st, size_t smem, i
     return cudaGetLastError();
 }
 
+namespace {
+template <typename F>
+cudaError_t with_form(int K, F&& go) {
+    switch (K) {
+        case 4: return go(std::integral_constant<int, 4>{});
+        case 6: return go(std::integral_constant<int, 6>{});
+        case 8: return go(std::integral_constant<int, 8>{});
+        case 10: return go(std::integral_constant<int, 10>{});
+        case 12: return go(std::integral_constant<int, 12>{});
+        case 14: return go(std::integral_constant<int, 14>{});
+        case 16: return go(std::integral_constant<int, 16>{});
+        case 20: return go(std::integral_constant<int, 20>{});
+        case 24: return go(std::integral_constant<int, 24>{});
+        case 28: return go(std::integral_constant<int, 28>{});
+        case 32: return go(std::integral_constant<int, 32>{});
+        case 40: return go(std::integral_constant<int, 40>{});
+        case 48: return go(std::integral_constant<int, 48>{});
+        case 56: return go(std::integral_constant<int, 56>{});
+        case 64: return go(std::integral_constant<int, 64>{});
+        default: return cudaErrorInvalidValue;
+    }
+}
+size_t cell_smem(int np) {
+    const int K = collide_form(np), pts = 32 * form_warps(K) * form_points(K);
+    return cell_smem_doubles(np, pts) * sizeof(double);
+}
+}  // namespace
+
+int collide_form(int np) {
+    const int k = (np + 7) / 8;
+    if (k <= 4) return 4;
+    if (k <= 16) return (k + 1) / 2 * 2;
+    return k <= 32 ? (k + 3) / 4 * 4 : (k + 7) / 8 * 8;
+}
+// Planes of one l a lane group takes at a time: as many as make the longest
+// group's work shortest, a unit's pivots counted as three planes
+int collide_unit_planes(int np, int l0, int m0, int mmax_coll, int do_l1, int do_lm) {
+    if (np > 512) return 1;
+    const int K = collide_form(np), groups = 32 * form_warps(K) / form_lanes(K);
+    int best = 1, cost = 1 << 30;
+    const int widest = 1 + 2 * std::min(std::min(l0, m0), mmax_coll);
+    for (int C = 1; C <= widest; ++C) {
+        int units = 0;
+        for (int l = 1; l <= l0; ++l)
+            if (l == 1 ? do_l1 : do_lm) units += (1 + 2 * std::min(std::min(l, m0), mmax_coll) + C - 1) / C;
+        const int c = (units + groups - 1) / groups * (C + 3);
+        if (c < cost) { cost = c; best = C; }
+    }
+    return best;
+}
+
 size_t collide_tri_smem_per_cell(int np, int l0) {
-    if (np <= 256) return lane_smem_doubles(np, l0) * sizeof(double);
+    if (np <= 512) return cell_smem(np);
     return ((size_t)kSmemArrays * np + kSmemScalars + 2 * (size_t)l0 * np + np) * sizeof(double);
 }
 
 namespace {
-template <typename TP, int E>
-cudaError_t launch_lane(const CollideArgs& a, cudaStream_t st, int blocks, size_t smem) {
-    // planes per batch: two row sets of P x E doubles stay in registers
-    constexpr int P = E <= 2 ? 4 : (E <= 4 ? 2 : 1);
-    {
-        const cudaError_t e = ensure_dyn_smem((const void*)collide_lane_kernel<TP, E, P>, smem);
-        if (e != cudaSuccess) return e;
-    }
-    collide_lane_kernel<TP, E, P><<<blocks, 32, smem, st>>>(a);
-    return cudaGetLastError();
+template <typename TP>
+cudaError_t launch_cell(const CollideArgs& a, cudaStream_t st, int blocks) {
+    return with_form(collide_form(a.np), [&](auto form) {
+        constexpr int K = decltype(form)::value;
+        collide_cell_kernel<TP, K><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
+        return cudaGetLastError();
+    });
 }
 template <typename TP>
-cudaError_t launch_lane_e(const CollideArgs& a, cudaStream_t st, int blocks, size_t smem) {
-    switch ((a.np + 31) / 32) {
-        case 1: return launch_lane<TP, 1>(a, st, blocks, smem);
-        case 2: return launch_lane<TP, 2>(a, st, blocks, smem);
-        case 3: return launch_lane<TP, 3>(a, st, blocks, smem);
-        case 4: return launch_lane<TP, 4>(a, st, blocks, smem);
-        case 5: return launch_lane<TP, 5>(a, st, blocks, smem);
-        case 6: return launch_lane<TP, 6>(a, st, blocks, smem);
-        case 7: return launch_lane<TP, 7>(a, st, blocks, smem);
-        case 8: return launch_lane<TP, 8>(a, st, blocks, smem);
-        default: return cudaErrorInvalidValue;
-    }
-}
-}  // namespace
-
-namespace {
-template <typename TP, int E>
-cudaError_t launch_lane_batch(const CollideBatch& b, cudaStream_t st, size_t smem) {
-    constexpr int P = E <= 2 ? 4 : (E <= 4 ? 2 : 1);
-    {
-        const cudaError_t e = ensure_dyn_smem((const void*)collide_lane_batch_kernel<TP, E, P>, smem);
-        if (e != cudaSuccess) return e;
-    }
+cudaError_t launch_cell_batch(const CollideBatch& b, int form, cudaStream_t st, size_t smem) {
     const long long blocks = b.nitems < (1ll << 30) ? b.nitems : (1ll << 30);
     if (blocks < 1) return cudaSuccess;
-    collide_lane_batch_kernel<TP, E, P><<<(unsigned)blocks, 32, smem, st>>>(b);
-    return cudaGetLastError();
-}
-template <typename TP>
-cudaError_t launch_lane_batch_e(const CollideBatch& b, int E, cudaStream_t st, size_t smem) {
-    switch (E) {
-        case 1: return launch_lane_batch<TP, 1>(b, st, smem);
-        case 2: return launch_lane_batch<TP, 2>(b, st, smem);
-        case 3: return launch_lane_batch<TP, 3>(b, st, smem);
-        case 4: return launch_lane_batch<TP, 4>(b, st, smem);
-        case 5: return launch_lane_batch<TP, 5>(b, st, smem);
-        case 6: return launch_lane_batch<TP, 6>(b, st, smem);
-        case 7: return launch_lane_batch<TP, 7>(b, st, smem);
-        case 8: return launch_lane_batch<TP, 8>(b, st, smem);
-        default: return cudaErrorInvalidValue;
-    }
+    return with_form(form, [&](auto f) {
+        constexpr int K = decltype(f)::value;
+        if constexpr (K <= 32) {   // a batch's rows have at most 256 points
+            collide_cell_batch_kernel<TP, K><<<(unsigned)blocks, 32 * form_warps(K), smem, st>>>(b);
+            return cudaGetLastError();
+        }
+        return cudaErrorInvalidValue;
+    });
 }
 
 __global__ void clock_advance_batch_kernel(double* clocks, const double* dt, int n) {
@@ -1272,70 +1399,8 @@ __global__ void clock_commit_batch_kernel(double* clocks, const int* collide, in
 }
 }  // namespace
 
-size_t collide_chunk_smem(int warps, int tab_doubles, int cell_doubles) {
-    return sizeof(double) * ((size_t)kArgsDoubles + (size_t)tab_doubles + (size_t)warps * cell_doubles);
-}
-
-namespace {
-template <typename TP, int E>
-cudaError_t launch_lane_chunk(const CollideBatch& b, cudaStream_t st) {
-    constexpr int P = E <= 2 ? 4 : (E <= 4 ? 2 : 1);
-    const size_t smem = collide_chunk_smem(b.warps, b.tab_doubles, b.cell_doubles);
-    {
-        const cudaError_t e = ensure_dyn_smem((const void*)collide_lane_chunk_kernel<TP, E, P>, smem);
-        if (e != cudaSuccess) return e;
-    }
-    const long long blocks = b.nchunks < (1ll << 30) ? b.nchunks : (1ll << 30);
-    if (blocks < 1) return cudaSuccess;
-    collide_lane_chunk_kernel<TP, E, P><<<(unsigned)blocks, 32 * b.warps, smem, st>>>(b);
-    return cudaGetLastError();
-}
-template <typename TP, int E>
-int regs_of(int chunked) {
-    constexpr int P = E <= 2 ? 4 : (E <= 4 ? 2 : 1);
-    cudaFuncAttributes fa{};
-    const cudaError_t e = chunked ? cudaFuncGetAttributes(&fa, collide_lane_chunk_kernel<TP, E, P>)
-                                  : cudaFuncGetAttributes(&fa, collide_lane_batch_kernel<TP, E, P>);
-    return e == cudaSuccess ? fa.numRegs : 255;
-}
-template <typename TP>
-int regs_e(int E, int chunked) {
-    switch (E) {
-        case 1: return regs_of<TP, 1>(chunked);
-        case 2: return regs_of<TP, 2>(chunked);
-        case 3: return regs_of<TP, 3>(chunked);
-        case 4: return regs_of<TP, 4>(chunked);
-        case 5: return regs_of<TP, 5>(chunked);
-        case 6: return regs_of<TP, 6>(chunked);
-        case 7: return regs_of<TP, 7>(chunked);
-        case 8: return regs_of<TP, 8>(chunked);
-        default: return 255;
-    }
-}
-template <typename TP>
-cudaError_t launch_lane_chunk_e(const CollideBatch& b, int E, cudaStream_t st) {
-    switch (E) {
-        case 1: return launch_lane_chunk<TP, 1>(b, st);
-        case 2: return launch_lane_chunk<TP, 2>(b, st);
-        case 3: return launch_lane_chunk<TP, 3>(b, st);
-        case 4: return launch_lane_chunk<TP, 4>(b, st);
-        case 5: return launch_lane_chunk<TP, 5>(b, st);
-        case 6: return launch_lane_chunk<TP, 6>(b, st);
-        case 7: return launch_lane_chunk<TP, 7>(b, st);
-        case 8: return launch_lane_chunk<TP, 8>(b, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-}  // namespace
-
-int collide_batch_regs(int E, int planes_fp32, int chunked) {
-    return planes_fp32 ? regs_e<float>(E, chunked) : regs_e<double>(E, chunked);
-}
-
-cudaError_t launch_collide_batch(const CollideBatch& b, int E, int planes_fp32, size_t smem, cudaStream_t st) {
-    if (b.nchunks > 0) return planes_fp32 ? launch_lane_chunk_e<float>(b, E, st) : launch_lane_chunk_e<double>(b, E, st);
-    if (planes_fp32) return launch_lane_batch_e<float>(b, E, st, smem);
-    return launch_lane_batch_e<double>(b, E, st, smem);
+cudaError_t launch_collide_batch(const CollideBatch& b, int form, int planes_fp32, size_t smem, cudaStream_t st) {
+    return planes_fp32 ? launch_cell_batch<float>(b, form, st, smem) : launch_cell_batch<double>(b, form, st, smem);
 }
 cudaError_t launch_clock_advance(double* clocks, const double* dt, int n, cudaStream_t st) {
     clock_advance_batch_kernel<<<(n + 127) / 128, 128, 0, st>>>(clocks, dt, n);
@@ -1347,11 +1412,8 @@ cudaError_t launch_clock_commit(double* clocks, const int* collide, int n, cudaS
 }
 
 cudaError_t launch_collide_tri(const CollideArgs& a, cudaStream_t st, int /*cells_per_cta*/, int blocks) {
+    if (a.np <= 512) return a.planes_fp32 ? launch_cell<float>(a, st, blocks) : launch_cell<double>(a, st, blocks);
     const size_t smem = collide_tri_smem_per_cell(a.np, a.l0);
-    if (a.np <= 256) {
-        if (a.planes_fp32) return launch_lane_e<float>(a, st, blocks, smem);
-        return launch_lane_e<double>(a, st, blocks, smem);
-    }
     if (a.planes_fp32) {
         const cudaError_t e = ensure_dyn_smem((const void*)collide_warp_kernel<float>, smem);
         if (e != cudaSuccess) return e;

@@ -138,6 +138,7 @@ struct CollideArgs {
     double c_kpre, kpre;  // 4pi/3 re kp, re kp
     // velocity grid tables [np]
     const double *vr, *U4, *U4m1, *U2, *U2m1, *U1, *U1m1, *U3, *Qn, *Pn, *V5, *V7;
+    int unit_planes;      // planes of one l a lane group solves at a time (collide_unit_planes)
     int chunk;            // planes staged per pass (tridiagonal path)
     double* dense_ws;     // dense path: np*np doubles per block
     int* status;          // [0] flags, [1] non-dominant count
@@ -170,13 +171,6 @@ struct CollideBatch {
     const CollideArgs* probs;
     const int2* items;
     long long nitems;
-    // chunked form: CTAs of `warps` warps, one chunk (problem, first cell,
-    // cells) per CTA, the problem's velocity tables staged in shared memory
-    const int4* chunks;
-    long long nchunks;
-    int warps;
-    int tab_doubles;    // 12 x the group's largest nump
-    int cell_doubles;   // work space of one cell
 };
 
 // launchers (return cudaError_t)
@@ -228,12 +222,11 @@ cudaError_t launch_collide_adj(const adj::CollTables& T, int l0, int nx, const d
                                const int* plane_of = nullptr, int m0 = 0, int mmax = 0);
 cudaError_t launch_rk_combine(double* out, const double* v0, double a0, const double* v1, double a1, const double* v2,
                               double a2, long long n, cudaStream_t st);
-// tridiagonal collision step of a batch whose problems share E = ceil(np/32) <= 8
-cudaError_t launch_collide_batch(const CollideBatch& b, int E, int planes_fp32, size_t smem, cudaStream_t s);
-// shared memory of one chunked batched-collision CTA
-size_t collide_chunk_smem(int warps, int tab_doubles, int cell_doubles);
-// registers per thread of the batched collision kernel for this E (chunked or one cell per CTA)
-int collide_batch_regs(int E, int planes_fp32, int chunked);
+// the tridiagonal collision kernel's form for rows of np <= 512 points
+int collide_form(int np);
+int collide_unit_planes(int np, int l0, int m0, int mmax_coll, int do_l1, int do_lm);
+// tridiagonal collision step of a batch whose problems share the form
+cudaError_t launch_collide_batch(const CollideBatch& b, int form, int planes_fp32, size_t smem, cudaStream_t s);
 // device clocks {t, t_ee, t_eb} of n problems: t += dt; after a collision step t_ee = t_eb = t
 cudaError_t launch_clock_advance(double* clocks, const double* dt, int n, cudaStream_t s);
 cudaError_t launch_clock_commit(double* clocks, const int* collide, int n, cudaStream_t s);
