@@ -2385,7 +2385,7 @@ int oshun_adjoint_vjp(oshun_adjoint a, const double* y, const double* lam_next, 
         }
         const int mmax = h->cfg.if_implicit1D ? 0 : h->cfg.m0;
         CK(launch_collide_adj(adj_tables(h), h->cfg.l0, (int)h->cells, a->y1, a->lam1, 1, 1, nsub, hsub, Dt, a->ws,
-                              wsz, h->stream, a->general ? h->d_plane_of : nullptr, h->cfg.m0, mmax));
+                              wsz, h->stream, h->d_plane_of, h->cfg.m0, mmax));
     }
     // RK4 transpose
     const adj::Grid1 g = adj_grid(a);

@@ -9,17 +9,13 @@
 //   collide_adj_kernel the collision step's transpose (reverse sweep through
 //                      the e-e RK4 substeps, the transposed Thomas solves and
 //                      the dependence of the tridiagonal coefficients on f00),
-//                      one warp per cell (adjoint_warp.cuh: lane-parallel
-//                      maps, warp scans for the cumulative integrals and
-//                      their transposes, Thomas on lane 0), the cell's work
-//                      space in shared memory where it fits, else in global
-//                      memory;
+//                      one CTA per cell (adjoint_cell.cuh);
 //   rk_combine_kernel  the linear combinations of the RK4 transpose.
 // State vectors use the plane layout: f00 plane, the l >= 1 planes, the 6
 // field planes (for m0 = 0 and numy = 1: f[l][x][p] then E_x[x], ...).
 #include "adjoint2d.cuh"
+#include "adjoint_cell.cuh"
 #include "adjoint_math.h"
-#include "adjoint_warp.cuh"
 #include "oshun_internal.h"
 
 namespace oshun {
@@ -122,18 +118,17 @@ __global__ void to_fp64_kernel(const float* __restrict__ src, double* __restrict
         dst[i] = (double)src[i];
 }
 
-__global__ void __launch_bounds__(32) collide_adj_kernel(const CollTables T, const int l0, const double* __restrict__ y,
-                                                         double* __restrict__ lam, const int ee, const int eb,
-                                                         const int nsub, const double hsub, const double Dt,
-                                                         double* __restrict__ ws, const long long wsz,
-                                                         const int smem_ws, const long long pstride,
-                                                         const adjw::CellPlanes P) {
-    extern __shared__ double sws[];
+// K: the form of collide_cell.cuh (nump <= 256: one thread a point)
+template <int K>
+__global__ void __launch_bounds__(32 * form_warps(K), 1)
+    collide_adj_kernel(const CollTables T, const adjc::StepT st, const double* __restrict__ y, double* __restrict__ lam,
+                       double* __restrict__ ws, const long long wsz, const int smem_ws) {
+    extern __shared__ double smem[];
     const long long x = blockIdx.x;
     const int np = T.np;
-    double* w = smem_ws ? sws : ws + x * wsz;
-    adjw::collide_cell_T(T, l0, y + x * np, y + pstride + x * np, pstride, ee, eb, nsub, hsub, Dt, lam + x * np,
-                         lam + pstride + x * np, pstride, w, P);
+    double* starts = smem_ws ? smem + adjc::cell_doubles(np, blockDim.x) : ws + x * wsz;
+    adjc::collide_cell_T<form_lanes(K), form_run(K)>(T, st, y + x * np, y + st.pstride + x * np, lam + x * np,
+                                                     lam + st.pstride + x * np, smem, starts);
 }
 
 // out = a0 * v0 + a1 * v1 (+ a2 * v2)
@@ -175,20 +170,25 @@ cudaError_t launch_convert(const float* src, double* dst, long long n, cudaStrea
 cudaError_t launch_collide_adj(const CollTables& T, int l0, int nx, const double* y, double* lam, int ee, int eb,
                                int nsub, double hsub, double Dt, double* ws, long long wsz, cudaStream_t st,
                                const int* plane_of, int m0, int mmax) {
-    // wsz: the serial form's work space per cell (adj::coll_ws), at least the warp form's
-    const long long need = adjw::coll_ws(T.np, nsub);
-    if (need > wsz) return cudaErrorInvalidValue;
-    const long long pstride = (long long)nx * T.np;   // nx: the cells of the grid
-    const adjw::CellPlanes P{plane_of, m0, mmax};
-    const size_t smem = sizeof(double) * (size_t)need;
-    if (smem <= 200 * 1024) {
-        const cudaError_t e = ensure_dyn_smem((const void*)collide_adj_kernel, smem);
-        if (e != cudaSuccess) return e;
-        collide_adj_kernel<<<nx, 32, smem, st>>>(T, l0, y, lam, ee, eb, nsub, hsub, Dt, ws, wsz, 1, pstride, P);
-    } else {
-        collide_adj_kernel<<<nx, 32, 0, st>>>(T, l0, y, lam, ee, eb, nsub, hsub, Dt, ws, wsz, 0, pstride, P);
-    }
-    return cudaGetLastError();
+    // ws: the substep starts of the cells where a CTA's shared memory does not hold them
+    if (T.np > 256 || (long long)nsub * T.np > wsz) return cudaErrorInvalidValue;
+    const int K = collide_form(T.np);
+    const adjc::StepT s{l0, m0, mmax, collide_unit_planes(T.np, l0, m0, mmax, 1, 1), ee, eb, nsub, hsub, Dt, plane_of,
+                        (long long)nx * T.np};   // nx: the cells of the grid
+    return with_form(K, [&](auto form) {
+        constexpr int F = decltype(form)::value;
+        if constexpr (F <= 32) {
+            const size_t base = sizeof(double) * adjc::cell_doubles(T.np, 32 * form_warps(F));
+            const size_t starts = sizeof(double) * (size_t)nsub * T.np;
+            const int in_smem = base + starts <= 100 * 1024;
+            const size_t smem = base + (in_smem ? starts : 0);
+            const cudaError_t e = ensure_dyn_smem((const void*)collide_adj_kernel<F>, smem);
+            if (e != cudaSuccess) return e;
+            collide_adj_kernel<F><<<nx, 32 * form_warps(F), smem, st>>>(T, s, y, lam, ws, wsz, in_smem);
+            return cudaGetLastError();
+        }
+        return cudaErrorInvalidValue;
+    });
 }
 
 cudaError_t launch_stage_vjp2(const adj2::Grid2& g, const double* s, const double* c, double* out, cudaStream_t st) {

@@ -25,12 +25,12 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "collide_cell.cuh"
 #include "oshun_internal.h"
 
 namespace oshun {
 namespace {
 
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kCollideThreads = 128;
 
 // The three cumulative integrals of one f on one warp, interleaved:
@@ -816,188 +816,6 @@ __global__ void __launch_bounds__(32) collide_warp_kernel(const CollideArgs a) {
 //      and scan are done once per unit and only the offsets are scanned per
 //      plane.
 
-// Thomas pivots of harmonic order l for this lane's run of p, c'_i and
-// 1/(b_i - c'_{i-1} a_i), with b_i = tri_b_i + 1 - ll1 scat_i (tri_b_0 left
-// out for l > 1), as TridiagonalSolve forms them (def-Nmethods.cpp:152-159).
-// c'_i = c_i / (b_i - a_i c'_{i-1}) is a linear-fractional map of c'_{i-1},
-// the 2x2 matrix [[0, c_i], [-a_i, b_i]] acting on (c'_{i-1}, 1): each lane
-// composes its run's matrices, a scan over the group (rescaled by powers of
-// two, which leaves the maps unchanged) gives the value entering
-// the run, and the lane applies the recursion inside its run.
-struct M22 {
-    double a, b, c, d;
-};
-__device__ __forceinline__ M22 m22_mul(const M22& x, const M22& y) {
-    return M22{fma(x.a, y.a, x.b * y.c), fma(x.a, y.b, x.b * y.d), fma(x.c, y.a, x.d * y.c),
-               fma(x.c, y.b, x.d * y.d)};
-}
-__device__ __forceinline__ M22 m22_rescale(M22 x) {
-    const double mx = fmax(fmax(fabs(x.a), fabs(x.b)), fmax(fabs(x.c), fabs(x.d)));
-    const int ex = (int)((__double_as_longlong(mx) >> 52) & 0x7ff);
-    if (mx > 0.0 && ex > 0 && ex < 0x7ff) {
-        const double sc = __longlong_as_double((long long)(2046 - ex) << 52);   // 2^(1023 - ex)
-        x.a *= sc; x.b *= sc; x.c *= sc; x.d *= sc;
-    }
-    return x;
-}
-// the coefficients of one cell in shared memory (np each)
-struct TriRows {
-    double *a, *b, *c, *scat;
-};
-template <int G, int R>
-__device__ __forceinline__ void lane_pivots(const TriRows& s, const int l, const int n, const int i0, double (&cp)[R],
-                                            double (&id)[R]) {
-    const int gl = threadIdx.x & (G - 1);
-    const double ll1 = l * ((-0.5) * (l + 1.0));
-    M22 m{1.0, 0.0, 0.0, 1.0};
-#pragma unroll
-    for (int e = 0; e < R; ++e) {
-        const int i = i0 + e;
-        id[e] = 1.0;   // b_i until the recursion below
-        if (i < n) {
-            const double a = s.a[i], c = s.c[i];
-            const double b = (i == 0 && l > 1 ? 0.0 : s.b[i]) + (1.0 - ll1 * s.scat[i]);
-            id[e] = b;
-            m = M22{c * m.c, c * m.d, fma(-a, m.a, b * m.c), fma(-a, m.b, b * m.d)};
-        }
-        if (e % 8 == 7) m = m22_rescale(m);
-    }
-    m = m22_rescale(m);
-#pragma unroll
-    for (int off = 1; off < G; off <<= 1) {
-        const M22 o{__shfl_up_sync(kFull, m.a, off, G), __shfl_up_sync(kFull, m.b, off, G),
-                    __shfl_up_sync(kFull, m.c, off, G), __shfl_up_sync(kFull, m.d, off, G)};
-        if (gl >= off) m = m22_rescale(m22_mul(m, o));
-    }
-    const double xb = __shfl_up_sync(kFull, m.b, 1, G), xd = __shfl_up_sync(kFull, m.d, 1, G);
-    double cprev = gl == 0 ? 0.0 : xb / xd;
-#pragma unroll
-    for (int e = 0; e < R; ++e) {
-        const int i = i0 + e;
-        if (i < n) {
-            const double b = id[e];
-            if (i == 0) {
-                id[e] = 1.0 / b;
-                cprev = s.c[0] / b;
-            } else {
-                id[e] = 1.0 / (b - cprev * s.a[i]);
-                cprev = s.c[i] * id[e];
-            }
-            cp[e] = cprev;
-        } else {
-            id[e] = 0.0;
-            cp[e] = 0.0;
-        }
-    }
-}
-
-// velocity tables of a thread's PT momentum points k0 .. k0+PT-1
-template <int PT>
-struct PointTab {
-    double U4[PT], U4m[PT], U2[PT], U2m[PT], U1p[PT], U1mp[PT];   // I4, I2 terms of k; the J1 term of k + 1
-    double U3[PT], V5[PT], V7[PT], Qn[PT], Pn[PT], Pm[PT];        // Pm: Pn of k - 1
-};
-template <int PT>
-__device__ __forceinline__ void load_tab(const CollideArgs& a, const int k0, PointTab<PT>& t) {
-    const int n = a.np;
-#pragma unroll
-    for (int j = 0; j < PT; ++j) {
-        const int k = k0 + j;
-        const bool in = k < n, up = k + 1 < n;
-        const int kc = in ? k : 0;
-        t.U4[j] = in ? __ldg(a.U4 + kc) : 0.0;     // 0 at k = 0 (the tables start at 1)
-        t.U4m[j] = in ? __ldg(a.U4m1 + kc) : 0.0;
-        t.U2[j] = in ? __ldg(a.U2 + kc) : 0.0;
-        t.U2m[j] = in ? __ldg(a.U2m1 + kc) : 0.0;
-        t.U1p[j] = up ? __ldg(a.U1 + kc + 1) : 0.0;
-        t.U1mp[j] = up ? __ldg(a.U1m1 + kc + 1) : 0.0;
-        t.U3[j] = in ? __ldg(a.U3 + kc) : 1.0;
-        t.V5[j] = k < a.NB ? __ldg(a.V5 + kc) : 0.0;
-        t.V7[j] = k < a.NB ? __ldg(a.V7 + kc) : 0.0;
-        t.Qn[j] = in ? __ldg(a.Qn + kc) : 0.0;
-        t.Pn[j] = up ? __ldg(a.Pn + kc) : 0.0;
-        t.Pm[j] = in && k > 0 ? __ldg(a.Pn + kc - 1) : 0.0;
-    }
-}
-// shared memory of one cell's CTA (doubles): tri_a, tri_b, tri_c, scat [np],
-// f and G with a point of padding on both sides, the warps' totals [3][16]
-__host__ __device__ inline size_t cell_smem_doubles(int np, int pts) { return 4 * (size_t)np + 2 * ((size_t)pts + 2) + 48; }
-struct CellSmem {
-    TriRows tri;
-    double *f, *g, *tot;   // f, g: index -1 .. pts
-};
-__device__ __forceinline__ CellSmem carve_cell(double* base, int np, int pts) {
-    CellSmem s;
-    s.tri.a = base; s.tri.b = base + np; s.tri.c = base + 2 * np; s.tri.scat = base + 3 * np;
-    s.f = base + 4 * np + 1;
-    s.g = s.f + pts + 2;
-    s.tot = s.g + pts + 1;
-    return s;
-}
-
-// The cumulative integrals I4, I2 (k' <= k) and J1 (k' > k) of f at a thread's
-// points, and the whole I4, I2 (S4, S2).  fm, fp: the neighbours.
-template <int PT>
-__device__ __forceinline__ void cell_scans(const PointTab<PT>& t, const double (&f)[PT], const double (&fm)[PT],
-                                           const double (&fp)[PT], double* tot, double (&I4)[PT], double (&I2)[PT],
-                                           double (&J1)[PT], double& S4, double& S2) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    double s4 = 0.0, s2 = 0.0, s1 = 0.0;
-#pragma unroll
-    for (int j = 0; j < PT; ++j) {
-        I4[j] = fma(t.U4[j], f[j], t.U4m[j] * fm[j]);
-        I2[j] = fma(t.U2[j], f[j], t.U2m[j] * fm[j]);
-        J1[j] = fma(t.U1p[j], fp[j], t.U1mp[j] * f[j]);
-        s4 += I4[j]; s2 += I2[j]; s1 += J1[j];
-    }
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const double v4 = __shfl_up_sync(kFull, s4, off);
-        const double v2 = __shfl_up_sync(kFull, s2, off);
-        const double v1 = __shfl_down_sync(kFull, s1, off);
-        if (lane >= off) { s4 += v4; s2 += v2; }
-        if (lane + off < 32) s1 += v1;
-    }
-    if (lane == 31) { tot[warp] = s4; tot[16 + warp] = s2; }
-    if (lane == 0) tot[32 + warp] = s1;
-    double r4 = __shfl_up_sync(kFull, s4, 1), r2 = __shfl_up_sync(kFull, s2, 1);
-    double r1 = __shfl_down_sync(kFull, s1, 1);
-    if (lane == 0) { r4 = 0.0; r2 = 0.0; }
-    if (lane == 31) r1 = 0.0;
-    __syncthreads();
-    double b4 = 0.0, b2 = 0.0, b1 = 0.0;
-    S4 = 0.0; S2 = 0.0;
-    for (int w = 0; w < nw; ++w) {
-        if (w == warp) { b4 = S4; b2 = S2; }
-        S4 += tot[w]; S2 += tot[16 + w];
-        if (w > warp) b1 += tot[32 + w];
-    }
-    r4 += b4; r2 += b2; r1 += b1;
-#pragma unroll
-    for (int j = 0; j < PT; ++j) {
-        r4 += I4[j]; I4[j] = r4;
-        r2 += I2[j]; I2[j] = r2;
-    }
-#pragma unroll
-    for (int j = PT - 1; j >= 0; --j) {
-        r1 += J1[j];
-        J1[j] = r1;
-    }
-}
-// a thread's points to shared memory, then its neighbours back
-template <int PT>
-__device__ __forceinline__ void neighbours(double* buf, const int k0, const double (&v)[PT], double (&lo)[PT],
-                                           double (&hi)[PT]) {
-#pragma unroll
-    for (int j = 0; j < PT; ++j) buf[k0 + j] = v[j];
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < PT; ++j) {
-        lo[j] = j > 0 ? v[j > 0 ? j - 1 : 0] : buf[k0 - 1];
-        hi[j] = j + 1 < PT ? v[j + 1 < PT ? j + 1 : 0] : buf[k0 + PT];
-    }
-}
-
 // EE_isotropic_conserva::Getslope (def-FokkerPlanck.cpp:192-267): fh = C_ee(fin)
 template <int PT>
 __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSmem& s, const PointTab<PT>& t,
@@ -1238,14 +1056,6 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
 // before) 0.88 -> 0.2 ms; Weibel (16384 cells of 96 points, 48 planes) equal in FP64, 0.65 -> 0.60 ms in the FP32 split;
 // 512 uneven 1D problems 9.0 -> 7.7 ms a step.  Long e-e runs on few cells wait on the slope's three barriers and its
 // logarithms; large grids on the latency of the solves at 16 warps an SM (128 registers).
-// The forms: K = G R / 8 (the row's points, rounded up to the form's, over 8).
-// One thread a point up to 256 points, two beyond.
-constexpr int form_lanes(int K) { return K <= 8 ? 8 : (K <= 16 ? 16 : 32); }
-constexpr int form_run(int K) { return 8 * K / form_lanes(K); }
-constexpr int form_points(int K) { return K <= 32 ? 1 : 2; }
-constexpr int form_warps(int K) { return (8 * K + 32 * form_points(K) - 1) / (32 * form_points(K)); }
-// resident CTAs per SM: 16 warps of 128 registers up to 256 points
-constexpr int form_blocks(int K) { return K <= 32 ? 16 / form_warps(K) : 1; }
 template <typename TP, int K>
 __global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K)) collide_cell_kernel(const CollideArgs a) {
     extern __shared__ double smem[];
@@ -1311,27 +1121,6 @@ cudaError_t launch_collide(const CollideArgs& a, cudaStream_t st, size_t smem, i
 }
 
 namespace {
-template <typename F>
-cudaError_t with_form(int K, F&& go) {
-    switch (K) {
-        case 4: return go(std::integral_constant<int, 4>{});
-        case 6: return go(std::integral_constant<int, 6>{});
-        case 8: return go(std::integral_constant<int, 8>{});
-        case 10: return go(std::integral_constant<int, 10>{});
-        case 12: return go(std::integral_constant<int, 12>{});
-        case 14: return go(std::integral_constant<int, 14>{});
-        case 16: return go(std::integral_constant<int, 16>{});
-        case 20: return go(std::integral_constant<int, 20>{});
-        case 24: return go(std::integral_constant<int, 24>{});
-        case 28: return go(std::integral_constant<int, 28>{});
-        case 32: return go(std::integral_constant<int, 32>{});
-        case 40: return go(std::integral_constant<int, 40>{});
-        case 48: return go(std::integral_constant<int, 48>{});
-        case 56: return go(std::integral_constant<int, 56>{});
-        case 64: return go(std::integral_constant<int, 64>{});
-        default: return cudaErrorInvalidValue;
-    }
-}
 size_t cell_smem(int np) {
     const int K = collide_form(np), pts = 32 * form_warps(K) * form_points(K);
     return cell_smem_doubles(np, pts) * sizeof(double);
