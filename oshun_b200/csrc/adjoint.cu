@@ -118,9 +118,11 @@ __global__ void to_fp64_kernel(const float* __restrict__ src, double* __restrict
         dst[i] = (double)src[i];
 }
 
-// K: the form of collide_cell.cuh (nump <= 256: one thread a point)
+// K: the form of collide_cell.cuh (nump <= 256: one thread a point).  16 warps
+// an SM: the e-e sweeps, most of a cell's time, hold far fewer registers than
+// the solves, which spill a little for it.
 template <int K>
-__global__ void __launch_bounds__(32 * form_warps(K), 1)
+__global__ void __launch_bounds__(32 * form_warps(K), 16 / form_warps(K))
     collide_adj_kernel(const CollTables T, const adjc::StepT st, const double* __restrict__ y, double* __restrict__ lam,
                        double* __restrict__ ws, const long long wsz, const int smem_ws) {
     extern __shared__ double smem[];

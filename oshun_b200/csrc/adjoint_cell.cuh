@@ -119,7 +119,7 @@ struct Slope {
     double I4, I2, J1, raw, lnee, dn, dT, fa, fb;
 };
 __device__ __forceinline__ double ee_slope(const CollTables& T, const Mem& s, const Tab& t, const int k,
-                                           const double v0s, const double v1s, const double f, Slope& o) {
+                                           const double f, Slope& o) {
     const int n = T.np;
     double fin[1] = {f}, fm[1], fp[1], I4[1], I2[1], J1[1], S4, S2;
     neighbours<1>(s.f, k, fin, fm, fp);
@@ -128,23 +128,23 @@ __device__ __forceinline__ double ee_slope(const CollTables& T, const Mem& s, co
     cell_scans<1>(t.t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
     double G[1], Gm[1], Gp[1];
     if (k < T.NB) {
-        const double f00 = (o.fa - o.fb * v0s / v1s) / (1.0 - v0s / v1s);
-        const double i2s = f00 * t.t.U3[0] / 3.0 + (o.fb - f00) * t.t.V5[0] / v1s * 0.2;
-        const double i4s = f00 * t.t.V5[0] * 0.2 + (o.fb - f00) * t.t.V7[0] / (v1s * 7.0);
+        const double f00 = (o.fa - o.fb * t.t.r) * t.t.inv1r, df = o.fb - f00;
+        const double i2s = f00 * t.t.A2[0] + df * t.t.B2[0];
+        const double i4s = f00 * t.t.A4[0] + df * t.t.B4[0];
         G[0] = f * i4s + (t.t.U3[0] * f - 3.0 * i2s) * J1[0];
     } else {
         G[0] = (I4[0] + t.t.U3[0] * J1[0]) * f - 3.0 * I2[0] * J1[0];
     }
-    neighbours<1>(s.g, k, G, Gm, Gp);
     o.lnee = adj::log_ee_d(4.0 * adj::kPi * S2, 4.0 * adj::kPi * S4, T.density_np, &o.dn, &o.dT);
+    neighbours<1>(s.g, k, G, Gm, Gp);
     const double D = k < n - 1 ? (G[0] - Gp[0]) * t.t.Pn[0] : G[0];
-    o.raw = (k == 0 ? ((-G[0]) * (2.0 / v0s) - D) : ((Gm[0] - G[0]) * t.t.Pm[0] - D)) * t.t.Qn[0];
+    o.raw = (k == 0 ? ((-G[0]) * t.t.two_v0s - D) : ((Gm[0] - G[0]) * t.t.Pm[0] - D)) * t.t.Qn[0];
     o.I4 = I4[0]; o.I2 = I2[0]; o.J1 = J1[0];
     return o.raw * (T.c_kpre * o.lnee);
 }
 // transpose of the slope's derivative at f (adj::ee_slope_T): mu -> the cotangent of f
 __device__ __forceinline__ double ee_slope_T(const CollTables& T, const Mem& s, const Tab& t, const int k,
-                                             const double v0s, const double v1s, const double f, const Slope& o,
+                                             const double f, const Slope& o,
                                              const double mu) {
     const int n = T.np;
     const double norm = T.c_kpre * o.lnee;
@@ -156,17 +156,17 @@ __device__ __forceinline__ double ee_slope_T(const CollTables& T, const Mem& s, 
         const double lD = wp[0] - w[0], lDm = w[0] - wm[0];
         double lg = k < n - 1 ? lD * t.t.Pn[0] : lD;
         if (k >= 1) lg -= lDm * t.t.Pm[0];
-        else lg -= w[0] * (2.0 / v0s);
+        else lg -= w[0] * t.t.two_v0s;
         if (k < T.NB) {
-            const double r = v0s / v1s, f00 = (o.fa - o.fb * r) / (1.0 - r);
-            const double v3 = t.t.U3[0], v5 = t.t.V5[0], v7 = t.t.V7[0];
-            const double i2s = f00 * v3 / 3.0 + (o.fb - f00) * v5 / v1s * 0.2;
-            const double i4s = f00 * v5 * 0.2 + (o.fb - f00) * v7 / (v1s * 7.0);
+            const double f00 = (o.fa - o.fb * t.t.r) * t.t.inv1r, df = o.fb - f00;
+            const double v3 = t.t.U3[0], A2 = t.t.A2[0], B2 = t.t.B2[0], A4 = t.t.A4[0], B4 = t.t.B4[0];
+            const double i2s = f00 * A2 + df * B2;
+            const double i4s = f00 * A4 + df * B4;
             lf = lg * (i4s + v3 * o.J1);
             const double l_i4s = lg * f, l_i2s = -3.0 * lg * o.J1;
             l1 = lg * (v3 * f - 3.0 * i2s);
-            sum[1] = l_i2s * (v3 / 3.0 - v5 / v1s * 0.2) + l_i4s * (v5 * 0.2 - v7 / (v1s * 7.0));
-            sum[2] = l_i2s * (v5 / v1s * 0.2) + l_i4s * (v7 / (v1s * 7.0));
+            sum[1] = l_i2s * (A2 - B2) + l_i4s * (A4 - B4);
+            sum[2] = l_i2s * B2 + l_i4s * B4;
         } else {
             l4 = lg * f;
             l1 = lg * (t.t.U3[0] * f - 3.0 * o.I2);
@@ -176,9 +176,8 @@ __device__ __forceinline__ double ee_slope_T(const CollTables& T, const Mem& s, 
     }
     double r4, r2, r1;
     suffix_scans<3>(s.tot, l4, l2, l1, r4, r2, r1, sum);
-    const double r = v0s / v1s;
-    if (k == 0) lf += sum[1] / (1.0 - r);
-    if (k == 1) lf += sum[2] - sum[1] * r / (1.0 - r);
+    if (k == 0) lf += sum[1] * t.t.inv1r;
+    if (k == 1) lf += sum[2] - sum[1] * t.t.r * t.t.inv1r;
     const double l_lnee = sum[0] * T.c_kpre;
     return lf + scans_T(t, k, n, l4, l2, l1, r4, r2, r1, l_lnee * o.dT * 4.0 * adj::kPi, l_lnee * o.dn * 4.0 * adj::kPi);
 }
@@ -358,7 +357,6 @@ __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT&
     const int k = threadIdx.x, pts = blockDim.x;
     const bool in = k < n;
     const Mem s = carve(smem, n, pts);
-    const double v0s = T.vr[0] * T.vr[0], v1s = T.vr[1] * T.vr[1];
     Tab t;
     load(T, k, t);
     if (k == 0) { s.f[-1] = 0.0; s.f[pts] = 0.0; s.g[-1] = 0.0; s.g[pts] = 0.0; }
@@ -371,7 +369,7 @@ __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT&
             double fs = f, acc = 0.0;
             for (int st = 0; st < 4; ++st) {
                 Slope o;
-                const double d = ee_slope(T, s, t, k, v0s, v1s, fs, o);
+                const double d = ee_slope(T, s, t, k, fs, o);
                 acc = fma(st == 0 || st == 3 ? h / 6.0 : h / 3.0, d, acc);
                 fs = fma(st == 2 ? h : 0.5 * h, d, f);
             }
@@ -450,7 +448,7 @@ __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT&
             S[0] = fs;
 #pragma unroll
             for (int st = 0; st < 4; ++st) {
-                const double d = ee_slope(T, s, t, k, v0s, v1s, S[st], o[st]);
+                const double d = ee_slope(T, s, t, k, S[st], o[st]);
                 if (st < 3) S[st < 3 ? st + 1 : 0] = fma(st == 2 ? h : 0.5 * h, d, fs);
             }
             const double out = lam;
@@ -458,7 +456,7 @@ __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT&
 #pragma unroll
             for (int st = 3; st >= 0; --st) {
                 const double c = (st == 0 || st == 3 ? h / 6.0 : h / 3.0) * out + (st == 3 ? 0.0 : st == 2 ? h : 0.5 * h) * a;
-                a = ee_slope_T(T, s, t, k, v0s, v1s, S[st], o[st], c);
+                a = ee_slope_T(T, s, t, k, S[st], o[st], c);
                 lam += a;
             }
         }

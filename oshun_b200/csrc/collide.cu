@@ -819,8 +819,7 @@ __global__ void __launch_bounds__(32) collide_warp_kernel(const CollideArgs a) {
 // EE_isotropic_conserva::Getslope (def-FokkerPlanck.cpp:192-267): fh = C_ee(fin)
 template <int PT>
 __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSmem& s, const PointTab<PT>& t,
-                                              const int k0, const double v0s, const double v1s,
-                                              const double (&fin)[PT], double (&fh)[PT]) {
+                                              const int k0, const double (&fin)[PT], double (&fh)[PT]) {
     const int n = a.np;
     double fm[PT], fp[PT], I4[PT], I2[PT], J1[PT], S4, S2;
     neighbours<PT>(s.f, k0, fin, fm, fp);
@@ -831,23 +830,23 @@ __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSm
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
         if (k0 + j < a.NB) {
-            const double f00 = (fa - fb * v0s / v1s) / (1.0 - v0s / v1s);
-            const double i2s = f00 * t.U3[j] / 3.0 + (fb - f00) * t.V5[j] / v1s * 0.2;
-            const double i4s = f00 * t.V5[j] * 0.2 + (fb - f00) * t.V7[j] / (v1s * 7.0);
+            const double f00 = (fa - fb * t.r) * t.inv1r, df = fb - f00;
+            const double i2s = fma(df, t.B2[j], f00 * t.A2[j]);
+            const double i4s = fma(df, t.B4[j], f00 * t.A4[j]);
             G[j] = fin[j] * i4s + (t.U3[j] * fin[j] - 3.0 * i2s) * J1[j];
         } else {
             const double i2 = -3.0 * (I2[j] * J1[j]);
             G[j] = fma(fma(t.U3[j], J1[j], I4[j]), fin[j], i2);
         }
     }
-    neighbours<PT>(s.g, k0, G, Gm, Gp);
     const double norm = a.c_kpre * log_ee(4.0 * M_PI * S2, 4.0 * M_PI * S4, a.density_np);
+    neighbours<PT>(s.g, k0, G, Gm, Gp);
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
         const int k = k0 + j;
         // D_k = (G_k - G_{k+1}) P_k for k < n-1, D_{n-1} = G_{n-1}
         const double D = k < n - 1 ? (G[j] - Gp[j]) * t.Pn[j] : G[j];
-        const double v = k == 0 ? ((-G[j]) * (2.0 / v0s) - D) : ((Gm[j] - G[j]) * t.Pm[j] - D);
+        const double v = k == 0 ? ((-G[j]) * t.two_v0s - D) : ((Gm[j] - G[j]) * t.Pm[j] - D);
         fh[j] = v * t.Qn[j] * norm;
     }
 }
@@ -977,7 +976,6 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
     const bool solve = a.do_l1 || a.do_lm;
     PointTab<PT> t;
     load_tab<PT>(a, k0, t);
-    const double v0s = vr[0] * vr[0], v1s = vr[1] * vr[1];
     const StepP sp = step_params(a);
     double f[PT];
 #pragma unroll
@@ -992,7 +990,7 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
             for (int j = 0; j < PT; ++j) { f0[j] = f[j]; f1[j] = f[j]; }
             // one call site of the slope for the four stages
             for (int st = 0; st < 4; ++st) {
-                cell_ee_slope<PT>(a, s, t, k0, v0s, v1s, f1, fh);
+                cell_ee_slope<PT>(a, s, t, k0, f1, fh);
                 const double w = st < 2 ? 0.5 * h : (st == 2 ? h : h / 6.0);
                 const double u = st == 1 ? 2.0 / 3.0 : (st == 3 ? 1.0 : 1.0 / 3.0);
 #pragma unroll

@@ -121,7 +121,10 @@ __device__ __forceinline__ void lane_pivots(const TriRows& s, const int l, const
 template <int PT>
 struct PointTab {
     double U4[PT], U4m[PT], U2[PT], U2m[PT], U1p[PT], U1mp[PT];   // I4, I2 terms of k; the J1 term of k + 1
-    double U3[PT], V5[PT], V7[PT], Qn[PT], Pn[PT], Pm[PT];        // Pm: Pn of k - 1
+    double U3[PT], Qn[PT], Pn[PT], Pm[PT];                        // Pm: Pn of k - 1
+    // the parabolic fit of the first NB points: i2 = f00 A2 + (f1 - f00) B2, i4 likewise
+    double A2[PT], B2[PT], A4[PT], B4[PT];
+    double r, inv1r, two_v0s;   // v0^2/v1^2, 1/(1 - r), 2/v0^2
 };
 // A: CollideArgs or adj::CollTables
 template <int PT, class A>
@@ -139,11 +142,27 @@ __device__ __forceinline__ void load_tab(const A& a, const int k0, PointTab<PT>&
         t.U1p[j] = up ? __ldg(a.U1 + kc + 1) : 0.0;
         t.U1mp[j] = up ? __ldg(a.U1m1 + kc + 1) : 0.0;
         t.U3[j] = in ? __ldg(a.U3 + kc) : 1.0;
-        t.V5[j] = k < a.NB ? __ldg(a.V5 + kc) : 0.0;
-        t.V7[j] = k < a.NB ? __ldg(a.V7 + kc) : 0.0;
         t.Qn[j] = in ? __ldg(a.Qn + kc) : 0.0;
         t.Pn[j] = up ? __ldg(a.Pn + kc) : 0.0;
         t.Pm[j] = in && k > 0 ? __ldg(a.Pn + kc - 1) : 0.0;
+    }
+    // the divisions of every slope, once a cell
+    const double v0 = __ldg(a.vr), v1 = __ldg(a.vr + 1);
+    const double v0s = v0 * v0, v1s = v1 * v1;
+    t.r = v0s / v1s;
+    t.inv1r = 1.0 / (1.0 - t.r);
+    t.two_v0s = 2.0 / v0s;
+#pragma unroll
+    for (int j = 0; j < PT; ++j) {
+        const int k = k0 + j;
+        t.A2[j] = t.B2[j] = t.A4[j] = t.B4[j] = 0.0;
+        if (k < a.NB && k < n) {
+            const double v5 = __ldg(a.V5 + k);
+            t.A2[j] = t.U3[j] / 3.0;
+            t.B2[j] = v5 / v1s * 0.2;
+            t.A4[j] = v5 * 0.2;
+            t.B4[j] = __ldg(a.V7 + k) / (v1s * 7.0);
+        }
     }
 }
 // shared memory of one cell's CTA (doubles): tri_a, tri_b, tri_c, scat [np],
