@@ -2213,6 +2213,35 @@ int adj_copy_out(oshun_ctx* h, int set, double* y) {
     return OSHUN_OK;
 }
 
+// ---- the step on state vectors in place of the handle's sets (FP64) --------
+
+// A stage reads whole 16-byte pieces of its inputs: vectors the caller owns
+// are used where they start on such a boundary, else through the handle's sets.
+bool vec_aligned(const double* y) { return (reinterpret_cast<uintptr_t>(y) & 15) == 0; }
+bool vec_disjoint(const double* x, const double* y, long long n) { return x + n <= y || y + n <= x; }
+
+int launch_stage_vec(oshun_ctx* h, int k, const double* in, const double* B, double* A, double* out) {
+    const StageSets q = rk4_sets(k, 0, 0, 0, 0);
+    StageArgs<double> a = h->stage_args<double>(0, q.kind);
+    const long long ps = h->pstride, pf = (1 + (long long)h->nplanes) * h->pstride;
+    a.f00_in = in; a.pl_in = in + ps; a.fld_in = in + pf;
+    a.f00_B = B; a.pl_B = B + ps; a.fld_B = B + pf;
+    a.f00_A = A; a.pl_A = A + ps; a.fld_A = A + pf;
+    if (out) { a.f00_out = out; a.pl_out = out + ps; a.fld_out = out + pf; }
+    a.c1 = h->cfg.dt * q.c1; a.c2 = q.c2;
+    const cudaError_t e = launch_stage_fp64(a, h->mc, h->stream);
+    if (e != cudaSuccess) { set_error(std::string("rk stage launch: ") + cudaGetErrorString(e)); return OSHUN_ERR_CUDA; }
+    return OSHUN_OK;
+}
+// RK4 from y into A; s2, s3, s4 receive the stage inputs (s4 may be s2)
+int rk4_vec(oshun_ctx* h, const double* y, double* A, double* s2, double* s3, double* s4) {
+    int rc = launch_stage_vec(h, 1, y, y, A, s2);
+    if (!rc) rc = launch_stage_vec(h, 2, s2, y, A, s3);
+    if (!rc) rc = launch_stage_vec(h, 3, s3, y, A, s4);
+    if (!rc) rc = launch_stage_vec(h, 4, s4, y, A, nullptr);
+    return rc;
+}
+
 void free_adj(oshun_adj_ctx* a) {
     if (a->h) free_ctx(a->h);
     cudaFree(a->s2); cudaFree(a->s3); cudaFree(a->s4); cudaFree(a->y1);
@@ -2335,8 +2364,25 @@ int oshun_adjoint_forward(oshun_adjoint a, const double* y, double* y_next, int 
                           double t_eb) {
     if (!a || !y || !y_next) return OSHUN_ERR_ARG;
     oshun_ctx* h = a->h;
-    int rc = adj_copy_in(h, h->cur, y);
-    if (rc) return rc;
+    int rc;
+    if (!h->fp32 && vec_aligned(y) && vec_aligned(y_next) && vec_disjoint(y, y_next, a->n)) {
+        // the stages read y and build y_next in place: no copies through the handle's sets
+        h->t_ee = t_ee; h->t_eb = t_eb;
+        if ((rc = rk4_vec(h, y, y_next, a->s2, a->s3, a->s2))) return rc;
+        h->t = t + h->cfg.dt;
+        if (collisions) {
+            int nsub; double hsub, Dt;
+            collide_params(h, h->t, &nsub, &hsub, &Dt);
+            CollideArgs c = collide_args(h, 1, 1, 1, nsub, hsub, Dt);
+            c.f00 = y_next;
+            c.planes = y_next + h->pstride;
+            if ((rc = launch_collide_args(h, c))) return rc;
+            h->t_ee = h->t_eb = h->t;
+        }
+        if (!a->async) CK(cudaStreamSynchronize(h->stream));
+        return OSHUN_OK;
+    }
+    if ((rc = adj_copy_in(h, h->cur, y))) return rc;
     h->t = t; h->t_ee = t_ee; h->t_eb = t_eb;
     if (a->async) {
         // queued on the caller's stream: the clock set by a kernel, no wait
@@ -2359,15 +2405,19 @@ int oshun_adjoint_vjp(oshun_adjoint a, const double* y, const double* lam_next, 
     const int B = h->cur, A = h->cur ^ 1, Sa = 2, Sb = 3;
     int rc;
     // stage inputs of the step (the production stage kernels)
-    if ((rc = adj_copy_in(h, B, y))) return rc;
-    if ((rc = launch_stage(h, rk4_sets(1, B, A, Sa, Sb)))) return rc;
-    if ((rc = adj_copy_out(h, Sa, a->s2))) return rc;
-    if ((rc = launch_stage(h, rk4_sets(2, B, A, Sa, Sb)))) return rc;
-    if ((rc = adj_copy_out(h, Sb, a->s3))) return rc;
-    if ((rc = launch_stage(h, rk4_sets(3, B, A, Sa, Sb)))) return rc;
-    if ((rc = adj_copy_out(h, Sa, a->s4))) return rc;
-    if ((rc = launch_stage(h, rk4_sets(4, B, A, Sa, Sb)))) return rc;
-    if ((rc = adj_copy_out(h, A, a->y1))) return rc;
+    if (!h->fp32 && vec_aligned(y)) {
+        if ((rc = rk4_vec(h, y, a->y1, a->s2, a->s3, a->s4))) return rc;
+    } else {
+        if ((rc = adj_copy_in(h, B, y))) return rc;
+        if ((rc = launch_stage(h, rk4_sets(1, B, A, Sa, Sb)))) return rc;
+        if ((rc = adj_copy_out(h, Sa, a->s2))) return rc;
+        if ((rc = launch_stage(h, rk4_sets(2, B, A, Sa, Sb)))) return rc;
+        if ((rc = adj_copy_out(h, Sb, a->s3))) return rc;
+        if ((rc = launch_stage(h, rk4_sets(3, B, A, Sa, Sb)))) return rc;
+        if ((rc = adj_copy_out(h, Sa, a->s4))) return rc;
+        if ((rc = launch_stage(h, rk4_sets(4, B, A, Sa, Sb)))) return rc;
+        if ((rc = adj_copy_out(h, A, a->y1))) return rc;
+    }
     CK(cudaMemcpyAsync(a->lam1, lam_next, sizeof(double) * a->n, cudaMemcpyDeviceToDevice, h->stream));
     // collision step transpose at y1
     if (collisions) {
@@ -2391,18 +2441,18 @@ int oshun_adjoint_vjp(oshun_adjoint a, const double* y, const double* lam_next, 
     const adj::Grid1 g = adj_grid(a);
     const adj2::Grid2 g2 = adj_grid2(h);
     const long long n = a->n;
-    CK(cudaMemcpyAsync(a->acc, a->lam1, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
     const double* S[4] = {y, a->s2, a->s3, a->s4};
     const double w_out[4] = {dt / 6.0, dt / 3.0, dt / 3.0, dt / 6.0};
     const double w_in[4] = {0.0, 0.5 * dt, 0.5 * dt, dt};   // weight of k_{i-1} in s_i
     for (int st = 3; st >= 0; --st) {
-        if (st == 3) CK(launch_rk_combine(a->c, a->lam1, w_out[3], a->lam1, 0.0, nullptr, 0.0, n, h->stream));
-        else CK(launch_rk_combine(a->c, a->lam1, w_out[st], a->a, w_in[st + 1], nullptr, 0.0, n, h->stream));
+        // c = w_out lam1 + w_in a, and the sum of the a's so far on lam1
+        if (st == 3) CK(launch_rk_combine(a->c, a->lam1, w_out[3], nullptr, 0.0, nullptr, nullptr, n, h->stream));
+        else CK(launch_rk_combine(a->c, a->lam1, w_out[st], a->a, w_in[st + 1], a->acc, st == 2 ? a->lam1 : a->acc, n,
+                                  h->stream));
         if (a->general) CK(launch_stage_vjp2(g2, S[st], a->c, a->a, h->stream));
         else CK(launch_stage_vjp(g, S[st], a->c, a->a, h->stream, h->fp32));
-        CK(launch_rk_combine(a->acc, a->acc, 1.0, a->a, 1.0, nullptr, 0.0, n, h->stream));
     }
-    CK(cudaMemcpyAsync(lam, a->acc, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
+    CK(launch_rk_combine(lam, a->acc, 1.0, a->a, 1.0, nullptr, nullptr, n, h->stream));
     if (!a->async) CK(cudaStreamSynchronize(h->stream));
     return OSHUN_OK;
 }

@@ -133,13 +133,13 @@ __global__ void __launch_bounds__(32 * form_warps(K), 16 / form_warps(K))
                                                      lam + st.pstride + x * np, smem, starts);
 }
 
-// out = a0 * v0 + a1 * v1 (+ a2 * v2)
-__global__ void rk_combine_kernel(double* out, const double* v0, double a0, const double* v1, double a1,
-                                  const double* v2, double a2, long long n) {
+// out = a0 v0 + a1 v1 and, where acc is given, acc = base + v1
+__global__ void rk_combine_kernel(double* out, const double* v0, double a0, const double* v1, double a1, double* acc,
+                                  const double* base, long long n) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double r = a0 * v0[i] + a1 * v1[i];
-        if (v2) r += a2 * v2[i];
-        out[i] = r;
+        const double v = v1 ? v1[i] : 0.0;
+        out[i] = v1 ? a0 * v0[i] + a1 * v : a0 * v0[i];
+        if (acc) acc[i] = base[i] + v;
     }
 }
 
@@ -200,11 +200,11 @@ cudaError_t launch_stage_vjp2(const adj2::Grid2& g, const double* s, const doubl
     return cudaGetLastError();
 }
 
-cudaError_t launch_rk_combine(double* out, const double* v0, double a0, const double* v1, double a1, const double* v2,
-                              double a2, long long n, cudaStream_t st) {
+cudaError_t launch_rk_combine(double* out, const double* v0, double a0, const double* v1, double a1, double* acc,
+                              const double* base, long long n, cudaStream_t st) {
     long long b = (n + 255) / 256;
     if (b > 148 * 8) b = 148 * 8;
-    rk_combine_kernel<<<(unsigned)b, 256, 0, st>>>(out, v0, a0, v1, a1, v2, a2, n);
+    rk_combine_kernel<<<(unsigned)b, 256, 0, st>>>(out, v0, a0, v1, a1, acc, base, n);
     return cudaGetLastError();
 }
 

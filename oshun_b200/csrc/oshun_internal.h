@@ -220,8 +220,9 @@ cudaError_t launch_convert(const float* src, double* dst, long long n, cudaStrea
 cudaError_t launch_collide_adj(const adj::CollTables& T, int l0, int nx, const double* y, double* lam, int ee, int eb,
                                int nsub, double hsub, double Dt, double* ws, long long wsz, cudaStream_t st,
                                const int* plane_of, int m0, int mmax);
-cudaError_t launch_rk_combine(double* out, const double* v0, double a0, const double* v1, double a1, const double* v2,
-                              double a2, long long n, cudaStream_t st);
+// out = a0 v0 + a1 v1 (v1 may be null) and, where acc is given, acc = base + v1
+cudaError_t launch_rk_combine(double* out, const double* v0, double a0, const double* v1, double a1, double* acc,
+                              const double* base, long long n, cudaStream_t st);
 // the tridiagonal collision kernel's form for rows of np <= 512 points
 int collide_form(int np);
 int collide_unit_planes(int np, int l0, int m0, int mmax_coll, int do_l1, int do_lm);
