@@ -54,33 +54,12 @@ __global__ void stage_vjp_kernel(const Grid1 g, const double* __restrict__ s, co
     }
 }
 
-// F'(s)^T c for any grid (adjoint2d.cuh): one CTA per cell, one thread per
-// momentum point gathers the cotangent of every source harmonic at its
-// point; the cell's field cotangents are summed over the CTA in a fixed
-// order, then the transposes of the current and of Ampere/Faraday added
-__global__ void stage_vjp2_kernel(const adj2::Grid2 g, const double* __restrict__ s, const double* __restrict__ c,
-                                  double* __restrict__ out) {
-    const long long cell = blockIdx.x;
-    const int k = threadIdx.x;
+// the cell's field cotangents: the points' shares summed over the CTA in a fixed
+// order, then the transposes of Ampere/Faraday
+__device__ __forceinline__ void field_cotangents(const adj2::Grid2& g, const double* __restrict__ c,
+                                                 double* __restrict__ out, const long long cell, const double (&cF)[6]) {
     __shared__ double red[6][8];
-    double cF[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (k < g.np) {
-        const double cdEx = adj2::fld(g, c, 0, cell), cdEy = adj2::fld(g, c, 1, cell), cdEz = adj2::fld(g, c, 2, cell);
-        for (int l = 0; l <= g.l0; ++l)
-            for (int M = 0; M <= (l < g.m0 ? l : g.m0); ++M) {
-                adj2::Cx v = adj2::vjp_source(g, s, c, l, M, cell, k, cF);
-                // the current: dEx = sum wj Re f10, dEy = 2 sum wj Re f11, dEz = -2 sum wj Im f11
-                if (l == 1 && M == 0) v.r += g.wj[k] * cdEx;
-                if (l == 1 && M == 1) { v.r += 2.0 * g.wj[k] * cdEy; v.i += -2.0 * g.wj[k] * cdEz; }
-                if (l == 0) {
-                    out[cell * g.np + k] = v.r;
-                } else {
-                    const long long q = g.plane_of[l * (g.m0 + 1) + M];
-                    out[(1 + q) * g.pstride + cell * g.np + k] = v.r;
-                    if (M > 0) out[(2 + q) * g.pstride + cell * g.np + k] = v.i;
-                }
-            }
-    }
+    const int k = threadIdx.x;
     const int lane = k & 31, warp = k >> 5;
 #pragma unroll
     for (int f = 0; f < 6; ++f) {
@@ -106,6 +85,219 @@ __global__ void stage_vjp2_kernel(const adj2::Grid2 g, const double* __restrict_
         double* of = out + (1 + (long long)g.nplanes) * g.pstride;
         for (int f = 0; f < 6; ++f) of[(long long)f * g.cells + cell] = F[f];
     }
+}
+
+// F'(s)^T c for any grid (adjoint2d.cuh): one CTA per cell, one thread per
+// momentum point k.  The transposed momentum stencils of a target's cotangent
+// c need c(k) and D = c(k+1) - c(k-1) alone, the advection v (c(x+1) - c(x-1))
+// and the same in y; a thread forms these four for the target rows s-1, s, s+1
+// once (a window of three rows in shared memory, its own column: no barrier)
+// and source (s, M) combines the up to nine targets that it feeds.  Gathering
+// every target's three momentum points and four neighbours per source from
+// global memory instead took 94 us a stage (32 x 32 cells, l0 = 4, m0 = 2, np =
+// 64), most of it address arithmetic and load latency.
+__global__ void __launch_bounds__(256) stage_vjp2_kernel(const adj2::Grid2 g, const double* __restrict__ s,
+                                                         const double* __restrict__ c, double* __restrict__ out) {
+    using adj2::Cx;
+    extern __shared__ double win[];   // [3 rows][m0+1][8][threads]
+    const long long cell = blockIdx.x;
+    const int k = threadIdx.x, np = g.np, stride = blockDim.x;
+    double cF[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (k < np) {
+        const int m1 = g.m0 + 1;
+        const adj2::Nbr nb = adj2::nbr(g, cell);
+        const bool has_y = g.ny > 1;
+        const double v = g.vr[k], ip = g.invp[k], wj = g.wj[k];
+        const double Ex = adj2::fld(g, s, 0, cell), Ey = adj2::fld(g, s, 1, cell), Ez = adj2::fld(g, s, 2, cell);
+        const double Bx = adj2::fld(g, s, 3, cell), By = adj2::fld(g, s, 4, cell), Bz = adj2::fld(g, s, 5, cell);
+        const double cdEx = adj2::fld(g, c, 0, cell), cdEy = adj2::fld(g, c, 1, cell), cdEz = adj2::fld(g, c, 2, cell);
+        const long long o = cell * np + k;
+        auto slot = [&](int t, int m) { return win + (size_t)((t % 3) * m1 + m) * 8 * stride + k; };
+        // base of harmonic (t, m) in a vector
+        auto plane = [&](const double* u, int t, int m) {
+            return t == 0 ? u : u + (1 + (long long)g.plane_of[t * m1 + m]) * g.pstride;
+        };
+        auto load_row = [&](int t) {
+            const int nclean = t >= 2 ? min(t - 1, 80) : 0;   // CLEAN_LOW_PC: no cotangent below
+            for (int m = 0; m <= min(t, g.m0); ++m) {
+                const double* b = plane(c, t, m);
+                double* w = slot(t, m);
+#pragma unroll
+                for (int comp = 0; comp < 2; ++comp) {
+                    double cc = 0.0, D = 0.0, X = 0.0, Y = 0.0;
+                    if (comp == 0 || m > 0) {
+                        const double* q = b + comp * g.pstride;
+                        if (k >= nclean) {
+                            cc = q[o];
+                            X = v * (q[nb.xp * np + k] - q[nb.xm * np + k]);
+                            if (has_y) Y = v * (q[nb.yp * np + k] - q[nb.ym * np + k]);
+                        }
+                        // p = 0 has no G and its own H (below); the last point differences onto itself
+                        const double up = k + 1 < np ? (k + 1 >= nclean ? q[o + 1] : 0.0) : -cc;
+                        D = up - (k >= 2 && k - 1 >= nclean ? q[o - 1] : 0.0);
+                    }
+                    w[comp * stride] = cc;
+                    w[(2 + comp) * stride] = D;
+                    w[(4 + comp) * stride] = X;
+                    w[(6 + comp) * stride] = Y;
+                }
+            }
+        };
+        load_row(0);
+        for (int sl = 0; sl <= g.l0; ++sl) {
+            if (sl < g.l0) load_row(sl + 1);
+            for (int M = 0; M <= min(sl, g.m0); ++M) {
+                const CoefLM& cf = g.coef[sl * m1 + M];
+                const double ipx = ip * cf.invpax;
+                // the source's value and stencils at k
+                Cx f, G{0.0, 0.0}, H{0.0, 0.0};
+                {
+                    const double* b = plane(s, sl, M);
+                    double r[2][3];
+#pragma unroll
+                    for (int comp = 0; comp < 2; ++comp)
+                        if (comp == 0 || M > 0) {
+                            const double* q = b + comp * g.pstride + o;
+                            r[comp][1] = q[0];
+                            r[comp][0] = k > 0 ? q[-1] : 0.0;
+                            r[comp][2] = k + 1 < np ? q[1] : q[0];
+                        } else {
+                            r[comp][0] = r[comp][1] = r[comp][2] = 0.0;
+                        }
+                    f = {r[0][1], r[1][1]};
+                    auto st = [&](const double* x, double& Gc, double& Hc) {
+                        const double d = x[0] - x[2];
+                        if (sl == 0) {
+                            Gc = k == 0 ? (x[2] - (x[1] - x[2] * g.g00_s) * g.g00_inv) * g.g00_gr : d;
+                        } else {
+                            Hc = k == 0 ? cf.hp0 * x[2] : ipx * x[1] + d;
+                            Gc = k == 0 ? 0.0 : cf.gfac * d + Hc;
+                        }
+                    };
+                    st(r[0], G.r, H.r);
+                    if (M > 0) st(r[1], G.i, H.i);
+                }
+                Cx acc{0.0, 0.0};
+                auto cot = [&](const double* w) -> Cx { return {w[0], w[stride]}; };
+                // conj(a) u
+                auto add = [&](double ar, double ai, Cx u) {
+                    acc.r += ar * u.r + ai * u.i;
+                    acc.i += ar * u.i - ai * u.r;
+                };
+                // a target through G (or H) and a difference term; a = (ar + i ai) the field factor
+                auto term = [&](int t, int m, bool isH, double ar, double ai, double dif, bool ydir) -> Cx {
+                    const double* w = slot(t, m);
+                    const Cx cc = cot(w);
+                    Cx u{w[2 * stride], w[3 * stride]};
+                    if (sl > 0) {
+                        const double gf = isH ? 1.0 : 1.0 + cf.gfac, pi = k > 0 ? ipx : 0.0;
+                        u.r = gf * u.r + pi * cc.r;
+                        u.i = gf * u.i + pi * cc.i;
+                    }
+                    // what point 0 of the target takes from points 0 and 1
+                    if (k <= 1 && t < 2) {   // (CLEAN_LOW_PC leaves point 0 of higher rows none)
+                        const double e0 = sl == 0 ? (k == 0 ? -g.g00_gr * g.g00_inv : g.g00_gr * (1.0 + g.g00_inv * g.g00_s))
+                                                  : (isH && k == 1 ? cf.hp0 : 0.0);
+                        if (e0 != 0.0) {
+                            const double* q = plane(c, t, m) + cell * np;
+                            u.r += e0 * q[0];
+                            if (m > 0) u.i += e0 * q[g.pstride];
+                        }
+                    }
+                    add(ar, ai, u);
+                    const double* dw = w + (ydir ? 6 : 4) * stride;
+                    acc.r += dif * dw[0];
+                    acc.i += dif * dw[stride];
+                    return cc;
+                };
+                const bool up = sl + 1 <= g.l0, dn = sl >= 1;
+                auto in = [&](int t, int m) { return m <= min(t, g.m0); };
+                if (up) {
+                    const Cx t = term(sl + 1, M, false, cf.ex_g * Ex, 0.0, cf.ax_p, false);
+                    cF[0] += cf.ex_g * (t.r * G.r + t.i * G.i);
+                }
+                if (dn && in(sl - 1, M)) {
+                    const Cx t = term(sl - 1, M, true, cf.ex_h * Ex, 0.0, cf.ax_m, false);
+                    cF[0] += cf.ex_h * (t.r * H.r + t.i * H.i);
+                }
+                if (M + 1 <= g.m0) {
+                    if (up) {
+                        const Cx t = term(sl + 1, M + 1, false, cf.em_g * Ey, -cf.em_g * Ez, has_y ? cf.ay_pp : 0.0, true);
+                        cF[1] += cf.em_g * (t.r * G.r + t.i * G.i);
+                        cF[2] += cf.em_g * (t.r * G.i - t.i * G.r);
+                    }
+                    if (dn && in(sl - 1, M + 1)) {
+                        const Cx t = term(sl - 1, M + 1, true, cf.em_h * Ey, -cf.em_h * Ez, has_y ? cf.ay_mp : 0.0, true);
+                        cF[1] += cf.em_h * (t.r * H.r + t.i * H.i);
+                        cF[2] += cf.em_h * (t.r * H.i - t.i * H.r);
+                    }
+                    if (dn && in(sl, M + 1)) {
+                        const Cx t = cot(slot(sl, M + 1));
+                        add(0.5 * Bz, 0.5 * By, t);
+                        cF[5] += 0.5 * (t.r * f.r + t.i * f.i);
+                        cF[4] += 0.5 * (t.i * f.r - t.r * f.i);
+                    }
+                }
+                if (M >= 1) {
+                    if (in(sl - 1, M - 1)) {
+                        const Cx t = term(sl - 1, M - 1, true, cf.ep_h * Ey, cf.ep_h * Ez, has_y ? cf.ay_mm : 0.0, true);
+                        cF[1] += cf.ep_h * (t.r * H.r + t.i * H.i);
+                        cF[2] += cf.ep_h * (t.i * H.r - t.r * H.i);
+                    }
+                    if (up) {
+                        const Cx t = term(sl + 1, M - 1, false, cf.ep_g * Ey, cf.ep_g * Ez, has_y ? cf.ay_pm : 0.0, true);
+                        cF[1] += cf.ep_g * (t.r * G.r + t.i * G.i);
+                        cF[2] += cf.ep_g * (t.i * G.r - t.r * G.i);
+                    }
+                    {
+                        const Cx t = cot(slot(sl, M - 1));
+                        add(cf.b_m * Bz, -cf.b_m * By, t);
+                        cF[5] += cf.b_m * (t.r * f.r + t.i * f.i);
+                        cF[4] += cf.b_m * (t.r * f.i - t.i * f.r);
+                    }
+                    {
+                        const Cx t = cot(slot(sl, M));
+                        add(0.0, -(double)M * Bx, t);
+                        cF[3] += (double)M * (t.r * f.i - t.i * f.r);
+                    }
+                }
+                // the current: dEx = sum wj Re f10, dEy = 2 sum wj Re f11, dEz = -2 sum wj Im f11
+                if (sl == 1 && M == 0) acc.r += wj * cdEx;
+                if (sl == 1 && M == 1) { acc.r += 2.0 * wj * cdEy; acc.i += -2.0 * wj * cdEz; }
+                double* q = (sl == 0 ? out : out + (1 + (long long)g.plane_of[sl * m1 + M]) * g.pstride) + o;
+                q[0] = acc.r;
+                if (M > 0) q[g.pstride] = acc.i;
+            }
+        }
+    }
+    field_cotangents(g, c, out, cell, cF);
+}
+
+// The same gathered point by point from global memory (adj2::vjp_source): for
+// rows whose window of targets does not fit in shared memory.
+__global__ void stage_vjp2_gather_kernel(const adj2::Grid2 g, const double* __restrict__ s, const double* __restrict__ c,
+                                  double* __restrict__ out) {
+    const long long cell = blockIdx.x;
+    const int k = threadIdx.x;
+    double cF[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (k < g.np) {
+        const double cdEx = adj2::fld(g, c, 0, cell), cdEy = adj2::fld(g, c, 1, cell), cdEz = adj2::fld(g, c, 2, cell);
+        for (int l = 0; l <= g.l0; ++l)
+            for (int M = 0; M <= (l < g.m0 ? l : g.m0); ++M) {
+                adj2::Cx v = adj2::vjp_source(g, s, c, l, M, cell, k, cF);
+                // the current: dEx = sum wj Re f10, dEy = 2 sum wj Re f11, dEz = -2 sum wj Im f11
+                if (l == 1 && M == 0) v.r += g.wj[k] * cdEx;
+                if (l == 1 && M == 1) { v.r += 2.0 * g.wj[k] * cdEy; v.i += -2.0 * g.wj[k] * cdEz; }
+                if (l == 0) {
+                    out[cell * g.np + k] = v.r;
+                } else {
+                    const long long q = g.plane_of[l * (g.m0 + 1) + M];
+                    out[(1 + q) * g.pstride + cell * g.np + k] = v.r;
+                    if (M > 0) out[(2 + q) * g.pstride + cell * g.np + k] = v.i;
+                }
+            }
+    }
+    field_cotangents(g, c, out, cell, cF);
 }
 
 // FP64 state vector <-> the FP32 planes and fields of an FP32-split handle
@@ -196,7 +388,14 @@ cudaError_t launch_collide_adj(const CollTables& T, int l0, int nx, const double
 cudaError_t launch_stage_vjp2(const adj2::Grid2& g, const double* s, const double* c, double* out, cudaStream_t st) {
     const int threads = ((g.np + 31) / 32) * 32;
     if (threads > 256) return cudaErrorInvalidValue;
-    stage_vjp2_kernel<<<(unsigned)g.cells, threads, 0, st>>>(g, s, c, out);
+    const size_t smem = sizeof(double) * 3 * 8 * (size_t)(g.m0 + 1) * threads;
+    if (smem <= 200 * 1024) {
+        const cudaError_t e = ensure_dyn_smem((const void*)stage_vjp2_kernel, smem);
+        if (e != cudaSuccess) return e;
+        stage_vjp2_kernel<<<(unsigned)g.cells, threads, smem, st>>>(g, s, c, out);
+    } else {
+        stage_vjp2_gather_kernel<<<(unsigned)g.cells, threads, 0, st>>>(g, s, c, out);
+    }
     return cudaGetLastError();
 }
 
