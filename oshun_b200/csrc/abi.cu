@@ -1603,6 +1603,7 @@ struct oshun_batch_ctx {
     int2* d_items = nullptr;
     int nitems = 0;
     size_t slot_bytes = 0, row_arr_bytes = 0;
+    uint32_t pair_src = 0, pair_tgt = 0;
     int row_depth = 2;
     std::vector<unsigned char> h_a1[2][4];   // kernel parameter of each launch (a problem's descriptor)
     // collision launches
@@ -1660,7 +1661,7 @@ int batch_build_items(oshun_batch_ctx* b) {
     const int esz = b->fp32 ? 4 : 8;
     struct It { double cost; int p, tile; };
     std::vector<It> items;
-    size_t slot = 0, rowb = 0;
+    size_t slot = 0, rowb = 0, pair_src = 0, pair_tgt = 0;
     for (int i = 0; i < (int)b->P.size(); ++i) {
         const oshun_cfg& c = b->P[i]->cfg;
         if (((c.nump + 31) / 32) * 32 > b->nc) {
@@ -1672,6 +1673,11 @@ int batch_build_items(oshun_batch_ctx* b) {
         stage_batch_sizes(c.nump, c.numx, c.numy, c.l0, c.m0, b->nc, b->tx_cap, esz, &tx, &sb, &rb);
         slot = std::max(slot, sb);
         rowb = std::max(rowb, rb);
+        if (b->mc == 0) {
+            stage_pair_batch_sizes(c.nump, c.numx, c.numy, tx, esz, &sb, &rb);
+            pair_src = std::max(pair_src, sb);
+            pair_tgt = std::max(pair_tgt, rb);
+        }
         const int tiles = c.numy * ((c.numx + tx - 1) / tx);
         const double cost = (double)b->P[i]->nh * (double)(((c.nump + 31) / 32) * 32) * tx;
         for (int t = 0; t < tiles; ++t) items.push_back({cost, i, t});
@@ -1695,6 +1701,8 @@ int batch_build_items(oshun_batch_ctx* b) {
     b->nitems = (int)h.size();
     b->slot_bytes = slot;
     b->row_arr_bytes = rowb;
+    b->pair_src = (uint32_t)pair_src;
+    b->pair_tgt = (uint32_t)pair_tgt;
     return OSHUN_OK;
 }
 
@@ -1711,6 +1719,8 @@ BatchWork batch_work(const oshun_batch_ctx* b, int c, int k) {
     bw.row_arr_bytes = (int)b->row_arr_bytes;
     bw.row_depth = b->row_depth;
     bw.nprobs = (int)b->P.size();
+    bw.pair_src = b->pair_src;
+    bw.pair_tgt = b->pair_tgt;
     return bw;
 }
 
@@ -1838,7 +1848,9 @@ int oshun_batch_create(const oshun_cfg* cfgs, int n, const int* collide, oshun_b
     }
     b->mc = pick_mc(m0max);
     b->desc_bytes = (int)((std::max(sizeof(StageArgs<float>), sizeof(StageArgs<double>)) + 15) / 16 * 16);
-    const int cbytes = stage_batch_coef_bytes(esz);
+    const bool pair = b->mc == 0;   // the two-point kernel has its own table entries
+    const int cbytes = pair ? stage_pair_coef(CoefLM{}, esz, std::vector<unsigned char>(128).data())
+                            : stage_batch_coef_bytes(esz);
     b->hdr_bytes = b->desc_bytes;
 
     // coupling tables in the arithmetic type
@@ -1855,7 +1867,13 @@ int oshun_batch_create(const oshun_cfg* cfgs, int n, const int* collide, oshun_b
             const int nco = (b->P[i]->cfg.l0 + 1) * (b->P[i]->cfg.m0 + 1);
             std::vector<double> dc((size_t)nco * 16);
             CKB(cudaMemcpy(dc.data(), b->P[i]->d_coef, sizeof(double) * dc.size(), cudaMemcpyDeviceToHost));
-            for (size_t k = 0; k < dc.size(); ++k) {
+            for (int k = 0; pair && k < nco; ++k) {
+                CoefLM c;
+                static_assert(sizeof(c) == 16 * sizeof(double), "CoefLM layout");
+                std::memcpy(&c, &dc[(size_t)16 * k], sizeof(c));
+                stage_pair_coef(c, esz, &hc[coff[i] + (size_t)cbytes * k]);
+            }
+            for (size_t k = 0; !pair && k < dc.size(); ++k) {
                 if (b->fp32) { const float v = (float)dc[k]; std::memcpy(&hc[coff[i] + 4 * k], &v, 4); }
                 else std::memcpy(&hc[coff[i] + 8 * k], &dc[k], 8);
             }

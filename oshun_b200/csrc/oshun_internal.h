@@ -197,7 +197,13 @@ struct BatchWork {
     int slot_bytes, row_arr_bytes;   // largest slot / staged-row array of the batch
     int row_depth;                // staged-row ring depth (2..8)
     int nprobs;                   // problems of the batch
+    uint32_t pair_src, pair_tgt;  // m0 = 0: largest source slot / operand array of the two-point kernel
 };
+// a batch whose problems all have m0 = 0 (stage_pair.cu); nc: momentum points of a tile, E and B updated in the launch
+template <typename TS>
+cudaError_t launch_stage_pair_batch(const StageArgs<TS>& a1, const BatchWork& bw, int nc, cudaStream_t s);
+void stage_pair_batch_sizes(int np, int nx, int ny, int tx, int elem_bytes, size_t* src_bytes, size_t* tgt_bytes);
+int stage_pair_coef(const CoefLM& c, int elem_bytes, unsigned char* dst);   // one table entry; its bytes
 // batched stage kernel (stage_batch.cu); nc consumer threads per CTA
 template <typename TS>
 cudaError_t launch_stage_batch(const StageArgs<TS>& a1, const BatchWork& bw, int mc, int nc, cudaStream_t s);

@@ -16,6 +16,15 @@ constexpr int kMaxTx = 8;
 constexpr size_t kSmemMax = 227 * 1024;          // dynamic shared memory of one CTA
 constexpr size_t kSmemHalf = (228 * 1024 - 2 * 1024) / 2;   // each of two CTAs on one SM (1 KB reserved each)
 
+// cells of a batch's tile: nc points of momentum rows rounded up to 32, tx_cap cells at most
+__host__ __device__ inline int batch_cells(int np, int nx, int nc, int tx_cap) {
+    const int np_pad = (np + 31) & ~31;
+    int tx = nc / np_pad;
+    if (tx > tx_cap) tx = tx_cap;
+    if (tx > nx) tx = nx;
+    return tx < 1 ? 1 : tx;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

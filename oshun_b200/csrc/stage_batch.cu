@@ -38,7 +38,7 @@ size_t stage_batch_smem(const BatchWork& bw, int elem_bytes) {
 
 void stage_batch_sizes(int np, int nx, int ny, int l0, int m0, int nc, int tx_cap, int elem_bytes, int* tx,
                        size_t* slot_bytes, size_t* row_arr_bytes) {
-    *tx = tile_cells(np, nx, nc, tx_cap);
+    *tx = batch_cells(np, nx, nc, tx_cap);
     const PipeLayout L = pipe_layout((l0 + 1) * (m0 + 1), *tx, np, ny > 1, elem_bytes, m0);
     *slot_bytes = L.slot_bytes;
     *row_arr_bytes = L.row_arr_bytes;
@@ -53,7 +53,7 @@ template <typename TS>
 cudaError_t launch_stage_batch(const StageArgs<TS>& a1, const BatchWork& bw, int mc, int nc, cudaStream_t s) {
     if (nc < 32 || nc > 320 || nc % 32) return cudaErrorInvalidValue;
     switch (mc) {
-        case 0: return batch_mc<TS, 0>(a1, bw, nc, s);
+        case 0: return launch_stage_pair_batch<TS>(a1, bw, nc, s);
         case 1: return batch_mc<TS, 1>(a1, bw, nc, s);
         case 2: return batch_mc<TS, 2>(a1, bw, nc, s);
         case 3: return batch_mc<TS, 3>(a1, bw, nc, s);

@@ -56,6 +56,8 @@
 //   advection (def-VlasovMax.cpp:834-951): x -> (l+-1,m), y -> (l+-1,m+-1);
 //   current (def-VlasovMax.cpp:680-745) from f10, f11; Ampere/Faraday
 //   (def-VlasovMax.cpp:979-1035); CLEAN_LOW_PC (def-Actions.cpp:240-253).
+#include <cstring>
+
 #include "stage_async.cuh"
 
 namespace oshun {
@@ -184,7 +186,8 @@ template <typename TS>
 struct alignas(16) CoefS {
     typename Arith<TS>::S v[16];
 };
-static_assert(sizeof(CoefS<double>) == 128 && sizeof(CoefS<float>) == 128, "CoefS layout");
+constexpr uint32_t kCoefBytes = 128;
+static_assert(sizeof(CoefS<double>) == kCoefBytes && sizeof(CoefS<float>) == kCoefBytes, "CoefS layout");
 // entry i of a source's coefficients (b_m doubled: it multiplies half fields)
 __host__ __device__ inline double coef_entry(const CoefLM& c, int i) {
     switch (i) {
@@ -551,11 +554,14 @@ __device__ __forceinline__ void copy_span(void* dst, const void* src, size_t byt
                   span_bytes<true>(src, bytes), bar);
 }
 
-// the sources of one tile
-template <typename TS, bool SHIFT>
+// the sources of one tile.  BATCH: its problem's descriptor comes along with
+// f00 (to desc_dst), and every source's coefficients at the end of its slot.
+template <typename TS, bool SHIFT, bool BATCH = false>
 __device__ __forceinline__ bool produce_sources(const StageArgs<TS>& a, const Geo& g, const Plan& P, const int tile,
                                                 unsigned char* smem, RingPos& r, int& issued,
-                                                const unsigned long long wlim, const int withhold) {
+                                                const unsigned long long wlim, const int withhold,
+                                                const unsigned char* desc = nullptr, const uint32_t desc_bytes = 0,
+                                                unsigned char* desc_dst = nullptr) {
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);
     uint64_t* empty = full + kMaxDepth;
     const int np = g.np, nx = g.nx, tx = g.tx;
@@ -605,7 +611,14 @@ __device__ __forceinline__ bool produce_sources(const StageArgs<TS>& a, const Ge
             }
             if (s == 0)   // the tile's fields: per field the aligned span holding its txv values
                 for (int f = 0; f < 6; ++f) bytes += span_bytes<true>(a.fld_in + f * a.cells + row + x0, txv * sizeof(TS));
+            if constexpr (BATCH) bytes += kCoefBytes + (s == 0 ? desc_bytes : 0u);
             mbar_expect_tx(bar, bytes);
+            if constexpr (BATCH) {
+                if (s == 0) bulk_g2s(desc_dst, desc, desc_bytes, bar);
+                bulk_g2s(dst + P.src_stride - kCoefBytes,
+                         reinterpret_cast<const unsigned char*>(a.coef_ts) + (size_t)(s * (a.m0 + 1) + m) * kCoefBytes,
+                         kCoefBytes, bar);
+            }
             for (int comp = 0; comp < ncomp; ++comp) {
                 unsigned char* cb = dst + comp * comp_bytes<SHIFT>(g, esz);
                 if (x_contig) {
@@ -702,8 +715,10 @@ struct Consumer {
 // barrier offset from a slot's full to its empty barrier
 constexpr uint32_t kEmptyOff = kMaxDepth * 8;
 
-// MC: the problem's m0; PT: momentum points of a thread
-template <int MC, typename TS, int PT, bool SHIFT>
+// MC: the problem's m0; PT: momentum points of a thread; BATCH: the source
+// slots end with the source's coefficients (coef and plane_of are not read;
+// m0 = 0, whose plane of row l is l - 1)
+template <int MC, typename TS, int PT, bool SHIFT, bool BATCH = false>
 __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS<TS>* __restrict__ coef,
                                              const int* __restrict__ plane_of, const Geo& g, const Plan& P,
                                              const int tile, unsigned char* smem, Consumer& cs, int* err,
@@ -775,6 +790,10 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
     auto release = [&]() {
         warp_arrive(cs.src.bar + kEmptyOff, lane);
         cs.src.next(P.src_stride, P.off_tgt, P.off_src, bar0);
+    };
+
+    auto slot_coef = [&]() {
+        return reinterpret_cast<const CoefS<TS>*>(smem + cs.src.off + P.src_stride - kCoefBytes);
     };
 
     acquire();
@@ -883,7 +902,7 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
     {
         Nb n0 = nb;
         if constexpr (sizeof(TS) == 4) place(n0, 8);
-        couple_f00<MC, TS, V>(A1, coef, operands<SHIFT>(reinterpret_cast<const double*>(smem + cs.src.off), n0, 0), n0, th,
+        couple_f00<MC, TS, V>(A1, BATCH ? slot_coef() : coef, operands<SHIFT>(reinterpret_cast<const double*>(smem + cs.src.off), n0, 0), n0, th,
                               a.g00_s, a.g00_inv, a.g00_gr);
     }
     release();
@@ -893,7 +912,7 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
     // the row.
     const int l0 = a.l0;
     for (int s = 1; s <= l0; ++s) {
-        const CoefS<TS>* crow = coef + s * mstride;
+        const CoefS<TS>* crow = BATCH ? nullptr : coef + s * mstride;
         Acc<V, MC> A2;
         // the sources of the row, one inside the other: a row that ends early
         // leaves them all at once, and no accumulator passes a join per source
@@ -902,9 +921,9 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
             acquire();
             const TS* sb = reinterpret_cast<const TS*>(smem + cs.src.off);
             const TS* ref = nullptr;
-            const int qs = (sizeof(TS) == 4 || SHIFT) ? plane_of[s * mstride + m] : 0;
+            const int qs = BATCH ? s - 1 : (sizeof(TS) == 4 || SHIFT) ? plane_of[s * mstride + m] : 0;
             if constexpr (sizeof(TS) == 4) ref = (a.pl_ref && __ldg(a.pl_keep + qs)) ? a.pl_ref + (long long)qs * np : nullptr;
-            couple_src<MC, m, SHIFT, TS, V>(A0, A1, A2, crow + m, sb, seg, nb, th, ref, np, qs);
+            couple_src<MC, m, SHIFT, TS, V>(A0, A1, A2, BATCH ? slot_coef() : crow + m, sb, seg, nb, th, ref, np, qs);
             if constexpr (m <= 1) {
                 if (s == 1) {
                     // the current of f = ref + stored deviation
@@ -988,12 +1007,7 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
 }
 
 // cells of a tile: as many as the consumers' 32-point segments hold
-inline int tile_cells(int np, int nx, int segments) {
-    int tx = segments / ((np + 31) >> 5);
-    if (tx > kMaxTx) tx = kMaxTx;
-    if (tx > nx) tx = nx;
-    return tx < 1 ? 1 : tx;
-}
+inline int tile_cells(int np, int nx, int segments) { return batch_cells(np, nx, 32 * segments, kMaxTx); }
 
 // Warps of a CTA.  Registers are granted per SM sub-partition, so a CTA costs
 // multiples of 4 warps: 8 warps leave 255 registers a thread, 12 warps 168, 16
@@ -1124,7 +1138,128 @@ cudaError_t pair_mc(const StageArgs<TS>& a, cudaStream_t s) {
     return pair_form<MC, TS, true>(a, s);
 }
 
+// ---------------------------------------------------------------------------
+// a batch of problems with m0 = 0: persistent CTAs walk the (problem, tile)
+// list.  Every problem's rows are 16-byte multiples (oshun_batch_create).
+//
+// An item is one tile of a few harmonics, so what counts is how many items an
+// SM has under way: three small CTAs (80 registers a thread) instead of two,
+// two points a thread, nothing read from global memory between the ring's
+// copies (the descriptor comes with f00, a source's coefficients with its
+// slot), E and B updated in the launch.  512 uneven problems, FP32, two steps:
+// 15.2 -> 11.6 ms against the one-point kernel (its consumers took 12.9
+// thousand cycles an item, 1.9 of them waiting for copies).
+// ---------------------------------------------------------------------------
+// Descriptors kept in shared memory: the producer is at most kMaxDepth slots,
+// two or more of them a tile, ahead of a warp that still reads its tile's.
+constexpr int kDescs = 8;
+static_assert(kMaxDepth / 2 + 1 < kDescs, "descriptor ring");
+constexpr int kBatchWarps = 5;   // consumer warps: 320 points, two a thread
+
+template <typename TS>
+__global__ void __launch_bounds__((kBatchWarps + 2) * 32, 3)
+    rk_stage_pair_batch_kernel(const __grid_constant__ BatchWork bw, const __grid_constant__ Plan P, const int nc, int* err) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x;
+    const int nct = (int)blockDim.x - 64;              // consumer threads
+    const int ncw = nct >> 5;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+    auto desc_at = [&](int iter) { return smem + P.off_coef + (size_t)(iter % kDescs) * bw.desc_bytes; };
+
+    for (int i = tid; i < kJBuf * P.hw; i += blockDim.x) reinterpret_cast<int*>(smem + P.off_cnt)[i] = 0;
+    if (tid == 0) {
+        for (int k = 0; k < kMaxDepth; ++k) {
+            mbar_init(bars + k, 1);
+            mbar_init(bars + kMaxDepth + k, ncw);
+            mbar_init(bars + 2 * kMaxDepth + k, 1);
+            mbar_init(bars + 3 * kMaxDepth + k, ncw);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    auto geo = [&](const StageArgs<TS>& a) { return make_geo(a.np, a.nx, a.ny, batch_cells(a.np, a.nx, nc, bw.tx_cap)); };
+
+    if (tid >= nct) {
+        if ((tid & 31) != 0) return;
+        const bool sources = tid == nct;
+        RingPos r;
+        int issued = 0, iter = 0;
+        bool ok = true;
+        auto desc = [&](int it) { return bw.probs + (size_t)bw.items[it].x * bw.desc_bytes; };
+        for (int it = blockIdx.x; it < bw.nitems && ok; it += gridDim.x, ++iter) {
+            StageArgs<TS> a = *reinterpret_cast<const StageArgs<TS>*>(desc(it));
+            a.hx = nullptr;   // batched problems have no halo columns
+            a.m0 = 0;
+            const Geo g = geo(a);
+            const int tile = bw.items[it].y;
+            ok = sources ? produce_sources<TS, false, true>(a, g, P, tile, smem, r, issued, kWaitNs, -1, desc(it),
+                                                            (uint32_t)bw.desc_bytes, desc_at(iter))
+                         : produce_targets<TS, false>(a, g, P, tile, smem, r, issued, kWaitNs);
+        }
+        if (!ok) {
+            atomicOr(err, 16);
+            drain(bars + (sources ? 0 : 2 * kMaxDepth), r, issued, sources ? P.D : P.RD, kWaitNs);
+        }
+        return;
+    }
+
+    Consumer cs;
+    cs.start(P, smem);
+    for (int it = blockIdx.x; it < bw.nitems; it += gridDim.x) {
+        const int tile = bw.items[it].y;
+        mbar_wait_or_exit(cs.src.bar, cs.src.phase, err, kWaitNs);   // the descriptor comes with f00
+        const StageArgs<TS>& a = *reinterpret_cast<const StageArgs<TS>*>(desc_at(cs.tile_iter));
+        consume_tile<0, TS, 2, false, true>(a, nullptr, nullptr, geo(a), P, tile, smem, cs, err, kWaitNs);
+    }
+}
+
 }  // namespace
+
+void stage_pair_batch_sizes(int np, int nx, int ny, int tx, int elem_bytes, size_t* src_bytes, size_t* tgt_bytes) {
+    const Geo g = make_geo(np, nx, ny, tx);
+    *src_bytes = align_up(src_slot_bytes<false>(g, elem_bytes, 0), 128) + kCoefBytes;
+    *tgt_bytes = tgt_array_bytes<false>(g, elem_bytes, 0);
+}
+
+// entry of a batch's coupling table: the factors of one source as the kernel reads them
+int stage_pair_coef(const CoefLM& c, int elem_bytes, unsigned char* dst) {
+    for (int i = 0; i < 16; ++i) {
+        const double v = coef_entry(c, i);
+        const float f[2] = {(float)v, (float)v};
+        if (elem_bytes == 4) std::memcpy(dst + 8 * i, f, 8);
+        else std::memcpy(dst + 8 * i, &v, 8);
+    }
+    return (int)kCoefBytes;
+}
+
+// nc: momentum points (rows rounded up to 32) of a tile
+template <typename TS>
+cudaError_t launch_stage_pair_batch(const StageArgs<TS>& a1, const BatchWork& bw, int nc, cudaStream_t s) {
+    if (nc < 32 || nc > 64 * kBatchWarps || nc % 32) return cudaErrorInvalidValue;
+    if (bw.nitems < 1) return cudaSuccess;
+    const int hw = (nc / 32 + 1) / 2 * 2, threads = hw * 16 + 64;
+    const auto kernel = rk_stage_pair_batch_kernel<TS>;
+    // as many CTAs an SM as its registers hold, each with at least five source
+    // slots (about a tile of few harmonics): what one CTA waits for, the others hide
+    const int desc_units = (int)((kDescs * (size_t)bw.desc_bytes + kCoefBytes - 1) / kCoefBytes);
+    Plan P;
+    int n = 1;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0);
+    if (e != cudaSuccess || n < 1) { (void)cudaGetLastError(); n = 1; }
+    for (;; --n) {
+        const size_t cap = n > 1 ? (size_t)(228 * 1024) / n - 1024 : kSmemMax;
+        if (deepest_plan(cap, bw.pair_src, bw.pair_tgt, stage_arrays(a1.kind), hw, desc_units, P) && (n == 1 || P.D >= 5)) break;
+        if (n == 1) return cudaErrorNotSupported;
+    }
+    e = ensure_dyn_smem((const void*)kernel, P.total);
+    if (e != cudaSuccess) return e;
+    const long long resident = (long long)sm_count() * n;
+    const long long blocks = bw.nitems < resident ? bw.nitems : resident;
+    kernel<<<dim3((unsigned)blocks), dim3(threads), P.total, s>>>(bw, P, nc, a1.err);
+    return cudaGetLastError();
+}
+template cudaError_t launch_stage_pair_batch<double>(const StageArgs<double>&, const BatchWork&, int, cudaStream_t);
+template cudaError_t launch_stage_pair_batch<float>(const StageArgs<float>&, const BatchWork&, int, cudaStream_t);
 
 // cudaErrorNotSupported when a momentum row does not fit the CTA or its rings
 template <typename TS>

@@ -415,14 +415,6 @@ __device__ __forceinline__ void store_row(const StageArgs<TS>& a, const int mtop
     });
 }
 
-__host__ __device__ inline int tile_cells(int np, int nx, int nc, int tx_cap) {
-    const int np_pad = (np + 31) & ~31;
-    int tx = nc / np_pad;
-    if (tx > tx_cap) tx = tx_cap;
-    if (tx > nx) tx = nx;
-    return tx < 1 ? 1 : tx;
-}
-
 // shared-memory plan of one launch (host and device agree)
 struct SmemPlan {
     size_t off_cur, off_coef, off_plane, off_slots, slot_stride, hdr, off_rows, row_arr_bytes, total;
@@ -504,7 +496,7 @@ __global__ void __launch_bounds__(MAXT, batch_min_blocks<MC, MAXT>())
             const int np = a.np, nx = a.nx, ny = a.ny;
             const bool has_y = ny > 1;
             const int mstride = a.m0 + 1;
-            const int tx = tile_cells(np, nx, nc, bw.tx_cap);
+            const int tx = batch_cells(np, nx, nc, bw.tx_cap);
             const int tiles_x = (nx + tx - 1) / tx;
             const int y = tile / tiles_x;
             const int x0 = (tile - y * tiles_x) * tx;
@@ -642,7 +634,7 @@ __global__ void __launch_bounds__(MAXT, batch_min_blocks<MC, MAXT>())
         const bool has_y = ny > 1;
         const int mstride = a.m0 + 1;
         const bool need_B = a.kind != kStageSlope;
-        const int tx = tile_cells(np, nx, nc, bw.tx_cap);
+        const int tx = batch_cells(np, nx, nc, bw.tx_cap);
         const int seg_cells = tx + 2 + (has_y ? 2 * tx : 0);
         const int tiles_x = (nx + tx - 1) / tx;
         const int y = tile / tiles_x;
