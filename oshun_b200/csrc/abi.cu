@@ -284,6 +284,7 @@ struct oshun_ctx {
     int nh = 0, nplanes = 0, mc = 0;
     long long cells = 0, pstride = 0;
     bool fp32 = false;
+    bool global_rows = false;   // an adjoint's handle (StageArgs.global_rows)
     size_t ts = 8;
     int dev = 0;
 
@@ -457,6 +458,7 @@ StageArgs<TS> oshun_ctx::stage_args(int in_set, int kind) const {
     a.idx = idx; a.idy = idy;
     a.err = d_status;
     a.jw = d_jw;
+    a.global_rows = global_rows && fp32 && (cfg.nump * sizeof(TS)) % 16 != 0;
     a.parts = kPartAll;
     a.wait_ns = inject_active ? inject_wait_ns : 1000000000ull;
     a.withhold = inject_active ? inject_withhold : -1;
@@ -2233,9 +2235,13 @@ int adj_copy_out(oshun_ctx* h, int set, double* y) {
 
 // ---- the step on state vectors in place of the handle's sets (FP64) --------
 
-// A stage reads whole 16-byte pieces of its inputs: vectors the caller owns
-// are used where they start on such a boundary, else through the handle's sets.
-bool vec_aligned(const double* y) { return (reinterpret_cast<uintptr_t>(y) & 15) == 0; }
+// A stage reads whole 16-byte pieces of its inputs and takes f00 and the l >= 1
+// planes to start on such a boundary: vectors the caller owns are used where
+// both do (a plane of an odd number of points leaves the second off it), else
+// through the handle's sets.
+bool vec_aligned(const oshun_ctx* h, const double* y) {
+    return ((reinterpret_cast<uintptr_t>(y) | (sizeof(double) * (uintptr_t)h->pstride)) & 15) == 0;
+}
 bool vec_disjoint(const double* x, const double* y, long long n) { return x + n <= y || y + n <= x; }
 
 int launch_stage_vec(oshun_ctx* h, int k, const double* in, const double* B, double* A, double* out) {
@@ -2328,6 +2334,7 @@ int oshun_adjoint_create(const oshun_cfg* cfg, oshun_adjoint* out) {
     oshun_ctx* h = a->h;
     // FP32 bulk: the handle's planes hold f itself (the trajectory comes in as FP64 vectors)
     h->use_profile = false;
+    h->global_rows = true;
     a->n = (1 + (long long)h->nplanes) * h->pstride + 6 * h->cells;
     auto fail = [&](int code) { free_adj(a); return code; };
     double** bufs[] = {&a->s2, &a->s3, &a->s4, &a->y1, &a->lam1, &a->c, &a->a, &a->acc};
@@ -2383,7 +2390,7 @@ int oshun_adjoint_forward(oshun_adjoint a, const double* y, double* y_next, int 
     if (!a || !y || !y_next) return OSHUN_ERR_ARG;
     oshun_ctx* h = a->h;
     int rc;
-    if (!h->fp32 && vec_aligned(y) && vec_aligned(y_next) && vec_disjoint(y, y_next, a->n)) {
+    if (!h->fp32 && vec_aligned(h, y) && vec_aligned(h, y_next) && vec_disjoint(y, y_next, a->n)) {
         // the stages read y and build y_next in place: no copies through the handle's sets
         h->t_ee = t_ee; h->t_eb = t_eb;
         if ((rc = rk4_vec(h, y, y_next, a->s2, a->s3, a->s2))) return rc;
@@ -2423,7 +2430,7 @@ int oshun_adjoint_vjp(oshun_adjoint a, const double* y, const double* lam_next, 
     const int B = h->cur, A = h->cur ^ 1, Sa = 2, Sb = 3;
     int rc;
     // stage inputs of the step (the production stage kernels)
-    if (!h->fp32 && vec_aligned(y)) {
+    if (!h->fp32 && vec_aligned(h, y)) {
         if ((rc = rk4_vec(h, y, a->y1, a->s2, a->s3, a->s4))) return rc;
     } else {
         if ((rc = adj_copy_in(h, B, y))) return rc;

@@ -91,6 +91,10 @@ struct StageArgs {
     unsigned long long wait_ns;   // a pipeline wait gives up after this many ns (single-problem kernel)
     int parts;            // kPart* bits of the RHS evaluated (kPartAll: Actions::Adv; others: the implicit-E actions)
     int withhold;         // fault injection for tests: CTA 0's source producer skips this copy (-1: none)
+    // an FP32 gradient on rows that are no multiple of 16 bytes: the global-load
+    // kernel.  Its results are FP64 vectors, which follow the FP32 roundings to
+    // 1e-7; this keeps the order of roundings that they are known by.
+    int global_rows;
     const void* coef_ts;  // coupling table in the arithmetic type (batched launches)
     double* jw;           // [cells][3][8]: per-warp partial sums of Jx, Re Jy, Im Jy (one-point kernels)
     // x halo columns of the stage input (null: periodic in x).  Side 0 is the

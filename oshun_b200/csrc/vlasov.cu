@@ -210,10 +210,11 @@ template <typename TS>
 cudaError_t launch_stage(const StageArgs<TS>& a, int mc, cudaStream_t s) {
     // The full right-hand side of m0 >= 1 on rows of 16-byte multiples: the
     // one-point pipelined kernel.  m0 = 0, other row lengths and partial
-    // right-hand sides: the two-point one.  Rows too long for either: global loads.
+    // right-hand sides: the two-point one.  Rows too long for either, and FP32
+    // gradients on rows of other lengths: global loads.
     cudaError_t e = cudaErrorNotSupported;
     if (a.m0 > 0 && a.parts == kPartAll) e = launch_stage_pipe<TS>(a, mc, s);
-    if (e == cudaErrorNotSupported) e = launch_stage_pair<TS>(a, s);
+    if (e == cudaErrorNotSupported && !a.global_rows) e = launch_stage_pair<TS>(a, s);
     if (e != cudaErrorNotSupported) return e;
     (void)cudaGetLastError();
     switch (mc) {
