@@ -825,6 +825,12 @@ __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSm
     neighbours<PT>(s.f, k0, fin, fm, fp);
     const double fa = s.f[0], fb = s.f[1];
     cell_scans<PT>(t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
+    // the logarithm of the whole cell on the last warp (the first has the fit below): every warp
+    // of its own would spend as many FP64 instructions on it as on all the rest of the slope
+    if (threadIdx.x + 32 >= blockDim.x) {
+        const double norm = a.c_kpre * log_ee(4.0 * M_PI * S2, 4.0 * M_PI * S4, a.density_np);
+        if ((threadIdx.x & 31) == 0) s.one[0] = norm;
+    }
     // flux G_n; the first NB cells use the parabolic fit near v = 0
     double G[PT], Gm[PT], Gp[PT];
 #pragma unroll
@@ -839,8 +845,8 @@ __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSm
             G[j] = fma(fma(t.U3[j], J1[j], I4[j]), fin[j], i2);
         }
     }
-    const double norm = a.c_kpre * log_ee(4.0 * M_PI * S2, 4.0 * M_PI * S4, a.density_np);
     neighbours<PT>(s.g, k0, G, Gm, Gp);
+    const double norm = s.one[0];
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
         const int k = k0 + j;
@@ -1012,8 +1018,16 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
     cell_scans<PT>(t, f, fm, fp, s.tot, I2, I0, J1m, S4, S2);
     const double I2_temperature = S4 * (4.0 * M_PI);
     const double I0_density = S2 * (4.0 * M_PI);
-    const double lnee = log_ee(I0_density, I2_temperature, a.density_np);
-    const double zlnei = zlog_ei(I0_density, I2_temperature, a.density_np, a.Zeta);
+    if (threadIdx.x + 32 >= blockDim.x) {
+        const double l = log_ee(I0_density, I2_temperature, a.density_np);
+        if ((threadIdx.x & 31) == 0) s.one[0] = l;
+    }
+    if (threadIdx.x < 32) {
+        const double l = zlog_ei(I0_density, I2_temperature, a.density_np, a.Zeta);
+        if (threadIdx.x == 0) s.one[1] = l;
+    }
+    __syncthreads();
+    const double lnee = s.one[0], zlnei = s.one[1];
     const double scale = (-1.0) * lnee * a.kpre * sp.Dt;
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
@@ -1050,12 +1064,13 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
 }
 
 // What it measured (B200, the collision launch, one cell a warp before -> now): 256 cells of 128 points, l0 = 1, ten e-e
-// substeps 0.21 -> 0.115 ms for the three calls of a step; 384 cells of 432 points, l0 = 31 (the staged-chunk kernel
+// substeps 0.21 -> 0.10 ms for the three calls of a step; 384 cells of 432 points, l0 = 31 (the staged-chunk kernel
 // before) 0.88 -> 0.2 ms; Weibel (16384 cells of 96 points, 48 planes) equal in FP64, 0.65 -> 0.60 ms in the FP32 split;
-// 512 uneven 1D problems 9.0 -> 7.7 ms a step.  Long e-e runs on few cells wait on the slope's three barriers and its
-// logarithms; large grids on the latency of the solves at 16 warps an SM (128 registers).
-template <typename TP, int K>
-__global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K)) collide_cell_kernel(const CollideArgs a) {
+// 20833 cells of 96 points 0.50 -> 0.44 ms with l0 = 8, but 0.26 -> 0.30 ms with l0 = 1, whose e-e part a warp a cell does
+// with fewer scans; 512 uneven 1D problems 9.0 -> 7.2 ms a step.  Long e-e runs on few cells wait on the slope's three
+// barriers and its logarithm; many cells on FP64 latency.
+template <typename TP, int K, bool MANY>
+__global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K, MANY)) collide_cell_kernel(const CollideArgs a) {
     extern __shared__ double smem[];
     for (long long cell = blockIdx.x; cell < a.cells; cell += gridDim.x) {
         collide_cell<TP, form_lanes(K), form_run(K), form_points(K)>(a, cell, smem);
@@ -1065,7 +1080,7 @@ __global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K)) collide_ce
 
 // batched form: work item = (problem, cell); the problems share the form
 template <typename TP, int K>
-__global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K)) collide_cell_batch_kernel(const CollideBatch b) {
+__global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K, true)) collide_cell_batch_kernel(const CollideBatch b) {
     extern __shared__ double smem[];
     __shared__ CollideArgs a;
     static_assert(sizeof(CollideArgs) % 4 == 0, "copied word by word");
@@ -1158,7 +1173,13 @@ template <typename TP>
 cudaError_t launch_cell(const CollideArgs& a, cudaStream_t st, int blocks) {
     return with_form(collide_form(a.np), [&](auto form) {
         constexpr int K = decltype(form)::value;
-        collide_cell_kernel<TP, K><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
+        if constexpr (form_blocks(K, true) > form_blocks(K, false)) {
+            if (a.cells > (long long)form_blocks(K, false) * sm_count()) {
+                collide_cell_kernel<TP, K, true><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
+                return cudaGetLastError();
+            }
+        }
+        collide_cell_kernel<TP, K, false><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
         return cudaGetLastError();
     });
 }

@@ -19,8 +19,16 @@ constexpr int form_lanes(int K) { return K <= 8 ? 8 : (K <= 16 ? 16 : 32); }
 constexpr int form_run(int K) { return 8 * K / form_lanes(K); }
 constexpr int form_points(int K) { return K <= 32 ? 1 : 2; }
 constexpr int form_warps(int K) { return (8 * K + 32 * form_points(K) - 1) / (32 * form_points(K)); }
-// resident CTAs per SM: 16 warps of 128 registers up to 256 points
-constexpr int form_blocks(int K) { return K <= 32 ? 16 / form_warps(K) : 1; }
+// resident CTAs per SM up to 256 points, of 128 registers a thread; more of 80
+// registers for launches of many cells (`many`), where a lane's run is shorter
+// than 8 points.  Many cells are bound by FP64 latency, which more warps hide:
+// 20833 cells of 96 points 0.35 -> 0.30 ms (l0 = 1), 12500 of 160 0.345 ->
+// 0.285 ms.  On few cells the slopes pay for their spills (256 cells of 96
+// points, ten e-e substeps: 118 us against 135), and with runs of 8 points
+// they do on any number (256 cells of 128 points: 119 against 140).
+constexpr int form_blocks(int K, bool many) {
+    return K <= 32 ? (many && form_run(K) < 8 ? 24 : 16) / form_warps(K) : 1;
+}
 template <typename F>
 cudaError_t with_form(int K, F&& go) {
     switch (K) {
@@ -166,11 +174,13 @@ __device__ __forceinline__ void load_tab(const A& a, const int k0, PointTab<PT>&
     }
 }
 // shared memory of one cell's CTA (doubles): tri_a, tri_b, tri_c, scat [np],
-// f and G with a point of padding on both sides, the warps' totals [3][16]
-__host__ __device__ inline size_t cell_smem_doubles(int np, int pts) { return 4 * (size_t)np + 2 * ((size_t)pts + 2) + 48; }
+// f and G with a point of padding on both sides, the warps' totals [3][16], two
+// values that one warp computes for all
+__host__ __device__ inline size_t cell_smem_doubles(int np, int pts) { return 4 * (size_t)np + 2 * ((size_t)pts + 2) + 50; }
 struct CellSmem {
     TriRows tri;
     double *f, *g, *tot;   // f, g: index -1 .. pts
+    double* one;
 };
 __device__ __forceinline__ CellSmem carve_cell(double* base, int np, int pts) {
     CellSmem s;
@@ -178,6 +188,7 @@ __device__ __forceinline__ CellSmem carve_cell(double* base, int np, int pts) {
     s.f = base + 4 * np + 1;
     s.g = s.f + pts + 2;
     s.tot = s.g + pts + 1;
+    s.one = s.tot + 48;
     return s;
 }
 
