@@ -279,7 +279,7 @@ int oshun_restart_read(oshun_handle h, const char* prefix, int rank, int re_step
  * one small step of its own dt per step (oshun_step's sequence) with one
  * captured CUDA graph per step: four persistent stage launches over the
  * (problem, tile) list of the whole batch and one collision launch per group
- * of problems with equal ceil(nump/32).  collide[i] = 0 (or collide = NULL
+ * of problems whose rows take the same threads.  collide[i] = 0 (or collide = NULL
  * for all on) skips problem i's collision calls; collisional problems need
  * if_tridiagonal = 1. */
 typedef struct oshun_batch_ctx* oshun_batch;

@@ -10,6 +10,8 @@
 //                      the e-e RK4 substeps, the transposed Thomas solves and
 //                      the dependence of the tridiagonal coefficients on f00),
 //                      one CTA per cell (adjoint_cell.cuh);
+//   stage_vjp2_kernel  F'(s)^T c of any grid (adjoint2d.cuh), and its
+//                      form without the shared-memory window;
 //   rk_combine_kernel  the linear combinations of the RK4 transpose.
 // State vectors use the plane layout: f00 plane, the l >= 1 planes, the 6
 // field planes (for m0 = 0 and numy = 1: f[l][x][p] then E_x[x], ...).

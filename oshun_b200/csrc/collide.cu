@@ -1,11 +1,14 @@
-// Fokker-Planck collision step, one CTA per configuration-space cell
-// (grid-stride over cells), all arithmetic in FP64:
+// Fokker-Planck collision step, one CTA per configuration-space cell, all
+// arithmetic in FP64.  Three kernels: collide_cell_kernel (tridiagonal, rows to
+// 512 points), collide_warp_kernel (tridiagonal, longer rows: one warp a cell)
+// and collide_kernel (staged chunks, dense matrices).
 //
 //   1. f00 e-e, Explicit_EC_FP::loop (OSHUN-1/def-FokkerPlanck.cpp:590-625):
 //      nsub RK4 substeps (RungeKutta4_ee::advance, :518-553) of Bell's
 //      number/energy conserving operator (EE_isotropic_conserva::Getslope,
-//      :192-267).  Warp 0 runs it; the cumulative integrals I4, I2 (forward)
-//      and J1 (backward) are warp scans over lane-owned runs of the p axis.
+//      :192-267).  collide_cell_kernel: one thread a momentum point, CTA
+//      scans; the others: warp 0, the cumulative integrals I4, I2 (forward)
+//      and J1 (backward) as warp scans over lane-owned runs of the p axis.
 //   2. Coefficients of the implicit f_lm step from the new f00,
 //      Implicit_FLM_step::reset_coeff (:808-939): I2, I0, J_{-1} scans,
 //      Coulomb logarithms, scattering term, the tridiagonal Alpha_Tri,
@@ -13,8 +16,9 @@
 //      computes them in both f1_loop and flm_loop with the same f00).
 //   3. (I - Dt C_l) f_lm^{n+1} = f_lm^n for every collided plane,
 //      Implicit_FLM_step::advance (:943-1035):
-//      tridiagonal: the cell's planes are staged through shared memory in
-//        chunks and each thread runs the reference's Thomas recursion
+//      tridiagonal: lane groups with rows in registers and the recursions as
+//        scans, or (collide_kernel) the cell's planes staged through shared
+//        memory in chunks, a thread running the reference's Thomas recursion
 //        (TridiagonalSolve, OSHUN-1/def-Nmethods.cpp:142-167) on one plane;
 //      dense: per l the np x np matrix is assembled in a per-CTA global
 //        workspace and each warp runs the reference's Gauss-Seidel
