@@ -97,7 +97,7 @@ __device__ __forceinline__ void field_cotangents(const adj2::Grid2& g, const dou
 // and source (s, M) combines the up to nine targets that it feeds.  Gathering
 // every target's three momentum points and four neighbours per source from
 // global memory instead took 94 us a stage (32 x 32 cells, l0 = 4, m0 = 2, np =
-// 64), most of it address arithmetic and load latency.
+// 64), most of it address arithmetic and load latency; the window takes 70.
 __global__ void __launch_bounds__(256) stage_vjp2_kernel(const adj2::Grid2 g, const double* __restrict__ s,
                                                          const double* __restrict__ c, double* __restrict__ out) {
     using adj2::Cx;

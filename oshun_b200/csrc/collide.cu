@@ -1177,8 +1177,9 @@ template <typename TP>
 cudaError_t launch_cell(const CollideArgs& a, cudaStream_t st, int blocks) {
     return with_form(collide_form(a.np), [&](auto form) {
         constexpr int K = decltype(form)::value;
+        // more cells than a wave, few planes: see form_blocks
         if constexpr (form_blocks(K, true) > form_blocks(K, false)) {
-            if (a.cells > (long long)form_blocks(K, false) * sm_count()) {
+            if (a.cells > (long long)form_blocks(K, false) * sm_count() && a.nplanes <= kManyPlanes) {
                 collide_cell_kernel<TP, K, true><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
                 return cudaGetLastError();
             }

@@ -25,7 +25,11 @@ constexpr int form_warps(int K) { return (8 * K + 32 * form_points(K) - 1) / (32
 // 20833 cells of 96 points 0.35 -> 0.30 ms (l0 = 1), 12500 of 160 0.345 ->
 // 0.285 ms.  On few cells the slopes pay for their spills (256 cells of 96
 // points, ten e-e substeps: 118 us against 135), and with runs of 8 points
-// they do on any number (256 cells of 128 points: 119 against 140).
+// they do on any number (256 cells of 128 points: 119 against 140).  With many
+// planes the solves do: a step of 16384 cells of 96 points with 48 planes took
+// 3.60 ms against 3.56, one of 4096 cells of 184 points with 29 planes 1.43
+// against 1.45.
+constexpr int kManyPlanes = 32;
 constexpr int form_blocks(int K, bool many) {
     return K <= 32 ? (many && form_run(K) < 8 ? 24 : 16) / form_warps(K) : 1;
 }
