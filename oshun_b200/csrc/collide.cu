@@ -97,7 +97,8 @@ __device__ double log_ee(double ne, double Te, double density_np) {
         ne *= density_np;
         Te = log(Te);
         ne = log(ne);
-        const double v = 23.5 - 0.5 * ne + 1.25 * Te - sqrt(0.00001 + 0.0625 * (Te - 2.0) * (Te - 2.0));
+        const double d = sub_rn(Te, 2.0);
+        const double v = sub_rn(fma_rn(1.25, Te, fma_rn(-0.5, ne, 23.5)), sqrt(fma_rn(mul_rn(0.0625, d), d, 0.00001)));
         if (v > 2.0) return v;
     }
     return 2.0;
@@ -109,7 +110,7 @@ __device__ double zlog_ei(double ne, double Te, double density_np, double Zeta) 
         ne *= density_np;
         Te = log(Te);
         ne = log(ne);
-        const double v = 24.0 - 0.5 * ne + Te;
+        const double v = add_rn(fma_rn(-0.5, ne, 24.0), Te);
         if (v > 2.0) return v * Zeta;
     }
     return 2.0 * Zeta;
@@ -840,13 +841,13 @@ __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSm
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
         if (k0 + j < a.NB) {
-            const double f00 = (fa - fb * t.r) * t.inv1r, df = fb - f00;
-            const double i2s = fma(df, t.B2[j], f00 * t.A2[j]);
-            const double i4s = fma(df, t.B4[j], f00 * t.A4[j]);
-            G[j] = fin[j] * i4s + (t.U3[j] * fin[j] - 3.0 * i2s) * J1[j];
+            const double f00 = mul_rn(fma_rn(-fb, t.r, fa), t.inv1r), df = sub_rn(fb, f00);
+            const double i2s = fma_rn(df, t.B2[j], mul_rn(f00, t.A2[j]));
+            const double i4s = fma_rn(df, t.B4[j], mul_rn(f00, t.A4[j]));
+            G[j] = fma_rn(fin[j], i4s, mul_rn(fma_rn(t.U3[j], fin[j], mul_rn(-3.0, i2s)), J1[j]));
         } else {
-            const double i2 = -3.0 * (I2[j] * J1[j]);
-            G[j] = fma(fma(t.U3[j], J1[j], I4[j]), fin[j], i2);
+            const double i2 = mul_rn(-3.0, mul_rn(I2[j], J1[j]));
+            G[j] = fma_rn(fma_rn(t.U3[j], J1[j], I4[j]), fin[j], i2);
         }
     }
     neighbours<PT>(s.g, k0, G, Gm, Gp);
@@ -855,9 +856,9 @@ __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSm
     for (int j = 0; j < PT; ++j) {
         const int k = k0 + j;
         // D_k = (G_k - G_{k+1}) P_k for k < n-1, D_{n-1} = G_{n-1}
-        const double D = k < n - 1 ? (G[j] - Gp[j]) * t.Pn[j] : G[j];
-        const double v = k == 0 ? ((-G[j]) * t.two_v0s - D) : ((Gm[j] - G[j]) * t.Pm[j] - D);
-        fh[j] = v * t.Qn[j] * norm;
+        const double D = k < n - 1 ? mul_rn(sub_rn(G[j], Gp[j]), t.Pn[j]) : G[j];
+        const double v = k == 0 ? fma_rn(-G[j], t.two_v0s, -D) : fma_rn(sub_rn(Gm[j], G[j]), t.Pm[j], -D);
+        fh[j] = mul_rn(mul_rn(v, t.Qn[j]), norm);
     }
 }
 
@@ -946,29 +947,29 @@ __device__ __forceinline__ void cell_solves(const CollideArgs& a, const TriRows&
             // forward: run offset, scan, recursion inside the run
             double B = 0.0;
 #pragma unroll
-            for (int e = 0; e < R; ++e) B = (cur[e] - B * ta[e]) * id[e];   // a_0 = 0; beyond the row nothing reads it
+            for (int e = 0; e < R; ++e) B = mul_rn(fma_rn(-B, ta[e], cur[e]), id[e]);   // a_0 = 0; beyond the row nothing reads it
 #pragma unroll
-            for (int t = 0, off = 1; t < kSteps; ++t, off <<= 1) B = fma(Af[t], __shfl_up_sync(kFull, B, off, G), B);
+            for (int t = 0, off = 1; t < kSteps; ++t, off <<= 1) B = fma_rn(Af[t], __shfl_up_sync(kFull, B, off, G), B);
             double d = __shfl_up_sync(kFull, B, 1, G);
             if (gl == 0) d = 0.0;
 #pragma unroll
             for (int e = 0; e < R; ++e) {
-                if (i0 + e < n) d = (cur[e] - d * ta[e]) * id[e];
+                if (i0 + e < n) d = mul_rn(fma_rn(-d, ta[e], cur[e]), id[e]);
                 cur[e] = i0 + e < n ? d : 0.0;
             }
             // backward: x_{n-1} = d'_{n-1}; c'_{n-1} = 0 and the points beyond are zero
             B = 0.0;
 #pragma unroll
-            for (int e = R - 1; e >= 0; --e) B = cur[e] - cp[e] * B;
+            for (int e = R - 1; e >= 0; --e) B = fma_rn(-cp[e], B, cur[e]);
 #pragma unroll
-            for (int t = 0, off = 1; t < kSteps; ++t, off <<= 1) B = fma(Ab[t], __shfl_down_sync(kFull, B, off, G), B);
+            for (int t = 0, off = 1; t < kSteps; ++t, off <<= 1) B = fma_rn(Ab[t], __shfl_down_sync(kFull, B, off, G), B);
             double x = __shfl_down_sync(kFull, B, 1, G);
             if (gl == G - 1) x = 0.0;
             TP* o = g + b * a.pstride;
 #pragma unroll
             for (int e = R - 1; e >= 0; --e) {
-                x = cur[e] - cp[e] * x;
-                if (b < cnt && i0 + e < n) o[e] = (TP)(rp ? x - (double)__ldg(rp + i0 + e) : x);
+                x = fma_rn(-cp[e], x, cur[e]);
+                if (b < cnt && i0 + e < n) o[e] = (TP)(rp ? sub_rn(x, (double)__ldg(rp + i0 + e)) : x);
             }
         }
         k += ng;
@@ -1005,9 +1006,9 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
                 const double u = st == 1 ? 2.0 / 3.0 : (st == 3 ? 1.0 : 1.0 / 3.0);
 #pragma unroll
                 for (int j = 0; j < PT; ++j) {
-                    const double d = fh[j] * w;
-                    f1[j] = f0[j] + d;
-                    f[j] = fma(d, u, f[j]);
+                    const double d = mul_rn(fh[j], w);
+                    f1[j] = add_rn(f0[j], d);
+                    f[j] = fma_rn(d, u, f[j]);
                 }
             }
         }
@@ -1042,10 +1043,9 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
         i2 /= v * v;
         const double i0 = I0[j] * (4.0 * M_PI);
         const double j1m = J1m[j] * (4.0 * M_PI * v);
-        const double t1 = i0 + (2.0 * j1m - i2) / 3.0;
-        const double t2 = (i2 + j1m) / 3.0;
-        double sc = (k == 0) ? 0.0 : t1 * lnee;
-        sc += zlnei * I0_density;
+        const double t1 = add_rn(i0, fma_rn(2.0, j1m, -i2) / 3.0);
+        const double t2 = add_rn(i2, j1m) / 3.0;
+        double sc = fma_rn(zlnei, I0_density, (k == 0) ? 0.0 : mul_rn(t1, lnee));
         sc /= t.U3[j];
         sc *= a.kpre * sp.Dt;
         s.tri.scat[k] = sc;
@@ -1057,9 +1057,10 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
             const double IvDnDm1 = 1.0 / (v * 0.5 * (vp - vm) * (v - vm));
             const double IvDnDp1 = 1.0 / (v * 0.5 * (vp - vm) * (vp - v));
             const double Ivsq2Dn = 1.0 / (v * v * (vp - vm));
-            tb = (8.0 * M_PI * f[j] - t2 * (IvDnDm1 + IvDnDp1)) * scale;
-            ta = (t2 * IvDnDm1 - t1 * Ivsq2Dn) * scale;
-            tc = (t2 * IvDnDp1 + t1 * Ivsq2Dn) * scale;
+            const double t1s = mul_rn(t1, Ivsq2Dn);
+            tb = mul_rn(fma_rn(-t2, add_rn(IvDnDm1, IvDnDp1), mul_rn(8.0 * M_PI, f[j])), scale);
+            ta = mul_rn(fma_rn(t2, IvDnDm1, -t1s), scale);
+            tc = mul_rn(fma_rn(t2, IvDnDp1, t1s), scale);
         }
         s.tri.a[k] = ta; s.tri.b[k] = tb; s.tri.c[k] = tc;
     }

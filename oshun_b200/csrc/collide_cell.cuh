@@ -1,12 +1,15 @@
 // Pieces of the CTA-per-cell collision kernels (collide.cu, adjoint.cu): one
 // thread per momentum point (two from 257 points on) for the pointwise work
 // and the cumulative integrals, groups of G lanes holding runs of R points for
-// the tridiagonal solves.
+// the tridiagonal solves.  Sums of products that end in a state are written with
+// explicit roundings (rounding.cuh): the instances of few and of many cells and
+// of a batch give the same bits.
 #pragma once
 
 #include <type_traits>
 
 #include "oshun_internal.h"
+#include "rounding.cuh"
 
 namespace oshun {
 namespace {
@@ -94,7 +97,7 @@ __device__ __forceinline__ void lane_pivots(const TriRows& s, const int l, const
         id[e] = 1.0;   // b_i until the recursion below
         if (i < n) {
             const double a = s.a[i], c = s.c[i];
-            const double b = (i == 0 && l > 1 ? 0.0 : s.b[i]) + (1.0 - ll1 * s.scat[i]);
+            const double b = add_rn(i == 0 && l > 1 ? 0.0 : s.b[i], fma_rn(-ll1, s.scat[i], 1.0));
             id[e] = b;
             m = M22{c * m.c, c * m.d, fma(-a, m.a, b * m.c), fma(-a, m.b, b * m.d)};
         }
@@ -118,7 +121,7 @@ __device__ __forceinline__ void lane_pivots(const TriRows& s, const int l, const
                 id[e] = 1.0 / b;
                 cprev = s.c[0] / b;
             } else {
-                id[e] = 1.0 / (b - cprev * s.a[i]);
+                id[e] = 1.0 / fma_rn(-cprev, s.a[i], b);
                 cprev = s.c[i] * id[e];
             }
             cp[e] = cprev;

@@ -4,21 +4,9 @@
 #pragma once
 
 #include "oshun_internal.h"
+#include "rounding.cuh"
 
 namespace oshun {
-
-// Roundings spelled out: the RK updates and the field updates run in several
-// kernels (single-problem, batched, global-load), and a product the compiler
-// fused into an add in one and not in another would make their results
-// differ in the last bit
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 template <typename T>
 __device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
