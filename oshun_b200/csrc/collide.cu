@@ -1,7 +1,8 @@
-// Fokker-Planck collision step, one CTA per configuration-space cell, all
-// arithmetic in FP64.  Three kernels: collide_cell_kernel (tridiagonal, rows to
-// 512 points), collide_warp_kernel (tridiagonal, longer rows: one warp a cell)
-// and collide_kernel (staged chunks, dense matrices).
+// Fokker-Planck collision step, all arithmetic in FP64, one CTA or one warp per
+// configuration-space cell: collide_cell_kernel (tridiagonal, rows to 512
+// points; many cells: collide_ee_kernel and collide_solve_kernel),
+// collide_warp_kernel (tridiagonal, longer rows) and collide_kernel (staged
+// chunks, dense matrices).
 //
 //   1. f00 e-e, Explicit_EC_FP::loop (OSHUN-1/def-FokkerPlanck.cpp:590-625):
 //      nsub RK4 substeps (RungeKutta4_ee::advance, :518-553) of Bell's
@@ -800,14 +801,15 @@ __global__ void __launch_bounds__(32) collide_warp_kernel(const CollideArgs a) {
     }
 }
 
-// Tridiagonal collision step for nump <= 512, one CTA per cell:
+// Tridiagonal collision step for nump <= 512, one CTA per cell (of many cells,
+// launch_cell: the e-e substeps so and the rest on a warp a cell):
 //   1. f00 e-e substeps and the coefficients of reset_coeff with one thread
 //      per momentum point (two from 257 points on): f, the RK4 stages and the
 //      point's velocity tables in registers, the three cumulative integrals as
 //      warp scans joined through the warps' totals, neighbours through shared
 //      memory, three barriers a slope.
 //   2. the collided planes, by groups of G lanes (8 for rows of up to 64
-//      points, 16 up to 128, else 32) so that a lane's run of p is 4 to 8
+//      points, 16 up to 112, else 32) so that a lane's run of p is 4 to 8
 //      points long and a warp solves 32/G planes at once: a group takes units
 //      of up to unit_planes planes of one l, forms that l's Thomas pivots for
 //      each lane's run (lane_pivots; TridiagonalSolve, def-Nmethods.cpp:
@@ -891,6 +893,12 @@ __device__ __forceinline__ void cell_solves(const CollideArgs& a, const TriRows&
         first = (int)((long long)nq * k / u);
         count = (int)((long long)nq * (k + 1) / u) - first;
     };
+    // a lane's run in the widest pieces that divide it, where the rows start on such a boundary and are whole numbers
+    // of them: 8-byte accesses 64 bytes apart (128 points) take a tag look-up for every second lane (5000 cells of 128
+    // points in runs of 8, 48 planes, the planes' call alone: 0.266 -> 0.217 ms)
+    constexpr int VW = R * sizeof(TP) % 16 == 0 ? 16 / (int)sizeof(TP) : (R % 2 == 0 ? 2 : 1);
+    struct alignas(VW * sizeof(TP)) Pack { TP v[VW]; };
+    const bool vec = n % VW == 0 && ((reinterpret_cast<uintptr_t>(planes) | (uintptr_t)(a.pstride * sizeof(TP))) & (sizeof(Pack) - 1)) == 0;
     double ta[R];
 #pragma unroll
     for (int e = 0; e < R; ++e) ta[e] = (i0 + e < n) ? s.a[i0 + e] : 0.0;
@@ -904,6 +912,16 @@ __device__ __forceinline__ void cell_solves(const CollideArgs& a, const TriRows&
         // rows as stored: the next plane's loads stay in flight during this plane's solve
         TP raw[R];
         auto load = [&](int b) {
+            if (VW > 1 && vec) {
+#pragma unroll
+                for (int e = 0; e < R; e += VW) {
+                    Pack v{};
+                    if (b < cnt && i0 + e < n) v = *reinterpret_cast<const Pack*>(g + b * a.pstride + e);
+#pragma unroll
+                    for (int w = 0; w < VW; ++w) raw[e + w] = v.v[w];
+                }
+                return;
+            }
 #pragma unroll
             for (int e = 0; e < R; ++e) raw[e] = (b < cnt && i0 + e < n) ? g[b * a.pstride + e] : TP(0);
         };
@@ -969,12 +987,88 @@ __device__ __forceinline__ void cell_solves(const CollideArgs& a, const TriRows&
 #pragma unroll
             for (int e = R - 1; e >= 0; --e) {
                 x = fma_rn(-cp[e], x, cur[e]);
-                if (b < cnt && i0 + e < n) o[e] = (TP)(rp ? sub_rn(x, (double)__ldg(rp + i0 + e)) : x);
+                cur[e] = rp && i0 + e < n ? sub_rn(x, (double)__ldg(rp + i0 + e)) : x;
+                if (!(VW > 1 && vec) && b < cnt && i0 + e < n) o[e] = (TP)cur[e];
+            }
+            if (VW > 1 && vec) {
+#pragma unroll
+                for (int e = 0; e < R; e += VW) {
+                    Pack v;
+#pragma unroll
+                    for (int w = 0; w < VW; ++w) v.v[w] = (TP)cur[e + w];
+                    if (b < cnt && i0 + e < n) *reinterpret_cast<Pack*>(o + e) = v;
+                }
             }
         }
         k += ng;
         settle();
     }
+}
+
+// RK4 substeps of Explicit_EC_FP::loop (RungeKutta4_ee::advance,
+// def-FokkerPlanck.cpp:518-553) on a thread's points of the cell's f00
+template <int PT>
+__device__ __forceinline__ void cell_ee(const CollideArgs& a, const StepP& sp, const CellSmem& s, const PointTab<PT>& t,
+                                        const int k0, double (&f)[PT]) {
+    const double h = sp.hsub;
+    for (int sub = 0; sub < sp.nsub; ++sub) {
+        double f0[PT], f1[PT], fh[PT];
+#pragma unroll
+        for (int j = 0; j < PT; ++j) { f0[j] = f[j]; f1[j] = f[j]; }
+        // one call site of the slope for the four stages
+        for (int st = 0; st < 4; ++st) {
+            cell_ee_slope<PT>(a, s, t, k0, f1, fh);
+            const double w = st < 2 ? 0.5 * h : (st == 2 ? h : h / 6.0);
+            const double u = st == 1 ? 2.0 / 3.0 : (st == 3 ? 1.0 : 1.0 / 3.0);
+#pragma unroll
+            for (int j = 0; j < PT; ++j) {
+                const double d = mul_rn(fh[j], w);
+                f1[j] = add_rn(f0[j], d);
+                f[j] = fma_rn(d, u, f[j]);
+            }
+        }
+    }
+}
+
+// Implicit_FLM_step::reset_coeff (def-FokkerPlanck.cpp:808-939), tridiagonal
+// part: the coefficients of the cell in units of the logarithms and moments
+struct CoeffP {
+    double lnee, zlnei, density, scale, kDt;
+};
+__device__ __forceinline__ CoeffP coeff_params(const CollideArgs& a, const StepP& sp, const double lnee,
+                                               const double zlnei, const double density) {
+    return CoeffP{lnee, zlnei, density, (-1.0) * lnee * a.kpre * sp.Dt, a.kpre * sp.Dt};
+}
+// ... at point k, from its integrals I2, I0, J_{-1}; U3: v^3
+__device__ __forceinline__ void point_coeffs(const CollideArgs& a, const CoeffP& c, const TriRows& tri, const int k,
+                                             const double f, const double I2, const double I0, const double J1m,
+                                             const double U3) {
+    const double* vr = a.vr;
+    const double v = vr[k];
+    double i2 = I2 * (4.0 * M_PI);
+    i2 /= v * v;
+    const double i0 = I0 * (4.0 * M_PI);
+    const double j1m = J1m * (4.0 * M_PI * v);
+    const double t1 = add_rn(i0, fma_rn(2.0, j1m, -i2) / 3.0);
+    const double t2 = add_rn(i2, j1m) / 3.0;
+    double sc = fma_rn(c.zlnei, c.density, (k == 0) ? 0.0 : mul_rn(t1, c.lnee));
+    sc /= U3;
+    sc *= c.kDt;
+    tri.scat[k] = sc;
+    double ta = 0.0, tb = 0.0, tc = 0.0;
+    if (k == 0) {
+        tb = 8.0 * M_PI * f * c.scale;
+    } else if (k < a.np - 1) {
+        const double vp = vr[k + 1], vm = vr[k - 1];
+        const double IvDnDm1 = 1.0 / (v * 0.5 * (vp - vm) * (v - vm));
+        const double IvDnDp1 = 1.0 / (v * 0.5 * (vp - vm) * (vp - v));
+        const double Ivsq2Dn = 1.0 / (v * v * (vp - vm));
+        const double t1s = mul_rn(t1, Ivsq2Dn);
+        tb = mul_rn(fma_rn(-t2, add_rn(IvDnDm1, IvDnDp1), mul_rn(8.0 * M_PI, f)), c.scale);
+        ta = mul_rn(fma_rn(t2, IvDnDm1, -t1s), c.scale);
+        tc = mul_rn(fma_rn(t2, IvDnDp1, t1s), c.scale);
+    }
+    tri.a[k] = ta; tri.b[k] = tb; tri.c[k] = tc;
 }
 
 template <typename TP, int G, int R, int PT>
@@ -983,8 +1077,6 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
     const int pts = PT * (int)blockDim.x;
     const CellSmem s = carve_cell(smem, n, pts);
     const int k0 = PT * (int)threadIdx.x;
-    const double* vr = a.vr;
-    const bool solve = a.do_l1 || a.do_lm;
     PointTab<PT> t;
     load_tab<PT>(a, k0, t);
     const StepP sp = step_params(a);
@@ -993,93 +1085,163 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
     for (int j = 0; j < PT; ++j) f[j] = k0 + j < n ? a.f00[cell * n + k0 + j] : 0.0;
     if (threadIdx.x == 0) { s.f[-1] = 0.0; s.f[pts] = 0.0; s.g[-1] = 0.0; s.g[pts] = 0.0; }
     if (a.do_ee) {
-        // RK4 substeps of Explicit_EC_FP::loop (RungeKutta4_ee::advance, def-FokkerPlanck.cpp:518-553)
-        const double h = sp.hsub;
-        for (int sub = 0; sub < sp.nsub; ++sub) {
-            double f0[PT], f1[PT], fh[PT];
-#pragma unroll
-            for (int j = 0; j < PT; ++j) { f0[j] = f[j]; f1[j] = f[j]; }
-            // one call site of the slope for the four stages
-            for (int st = 0; st < 4; ++st) {
-                cell_ee_slope<PT>(a, s, t, k0, f1, fh);
-                const double w = st < 2 ? 0.5 * h : (st == 2 ? h : h / 6.0);
-                const double u = st == 1 ? 2.0 / 3.0 : (st == 3 ? 1.0 : 1.0 / 3.0);
-#pragma unroll
-                for (int j = 0; j < PT; ++j) {
-                    const double d = mul_rn(fh[j], w);
-                    f1[j] = add_rn(f0[j], d);
-                    f[j] = fma_rn(d, u, f[j]);
-                }
-            }
-        }
+        cell_ee<PT>(a, sp, s, t, k0, f);
 #pragma unroll
         for (int j = 0; j < PT; ++j)
             if (k0 + j < n) a.f00[cell * n + k0 + j] = f[j];
     }
-    if (!solve) return;
-    // Implicit_FLM_step::reset_coeff (def-FokkerPlanck.cpp:808-939), tridiagonal part
+    if (!a.do_l1 && !a.do_lm) return;
     double fm[PT], fp[PT], I2[PT], I0[PT], J1m[PT], S4, S2;
     neighbours<PT>(s.f, k0, f, fm, fp);
     cell_scans<PT>(t, f, fm, fp, s.tot, I2, I0, J1m, S4, S2);
-    const double I2_temperature = S4 * (4.0 * M_PI);
-    const double I0_density = S2 * (4.0 * M_PI);
+    const double temperature = S4 * (4.0 * M_PI), density = S2 * (4.0 * M_PI);
     if (threadIdx.x + 32 >= blockDim.x) {
-        const double l = log_ee(I0_density, I2_temperature, a.density_np);
+        const double l = log_ee(density, temperature, a.density_np);
         if ((threadIdx.x & 31) == 0) s.one[0] = l;
     }
     if (threadIdx.x < 32) {
-        const double l = zlog_ei(I0_density, I2_temperature, a.density_np, a.Zeta);
+        const double l = zlog_ei(density, temperature, a.density_np, a.Zeta);
         if (threadIdx.x == 0) s.one[1] = l;
     }
     __syncthreads();
-    const double lnee = s.one[0], zlnei = s.one[1];
-    const double scale = (-1.0) * lnee * a.kpre * sp.Dt;
+    const CoeffP c = coeff_params(a, sp, s.one[0], s.one[1], density);
 #pragma unroll
-    for (int j = 0; j < PT; ++j) {
-        const int k = k0 + j;
-        if (k >= n) continue;
-        const double v = vr[k];
-        double i2 = I2[j] * (4.0 * M_PI);
-        i2 /= v * v;
-        const double i0 = I0[j] * (4.0 * M_PI);
-        const double j1m = J1m[j] * (4.0 * M_PI * v);
-        const double t1 = add_rn(i0, fma_rn(2.0, j1m, -i2) / 3.0);
-        const double t2 = add_rn(i2, j1m) / 3.0;
-        double sc = fma_rn(zlnei, I0_density, (k == 0) ? 0.0 : mul_rn(t1, lnee));
-        sc /= t.U3[j];
-        sc *= a.kpre * sp.Dt;
-        s.tri.scat[k] = sc;
-        double ta = 0.0, tb = 0.0, tc = 0.0;
-        if (k == 0) {
-            tb = 8.0 * M_PI * f[j] * scale;
-        } else if (k < n - 1) {
-            const double vp = vr[k + 1], vm = vr[k - 1];
-            const double IvDnDm1 = 1.0 / (v * 0.5 * (vp - vm) * (v - vm));
-            const double IvDnDp1 = 1.0 / (v * 0.5 * (vp - vm) * (vp - v));
-            const double Ivsq2Dn = 1.0 / (v * v * (vp - vm));
-            const double t1s = mul_rn(t1, Ivsq2Dn);
-            tb = mul_rn(fma_rn(-t2, add_rn(IvDnDm1, IvDnDp1), mul_rn(8.0 * M_PI, f[j])), scale);
-            ta = mul_rn(fma_rn(t2, IvDnDm1, -t1s), scale);
-            tc = mul_rn(fma_rn(t2, IvDnDp1, t1s), scale);
-        }
-        s.tri.a[k] = ta; s.tri.b[k] = tb; s.tri.c[k] = tc;
-    }
+    for (int j = 0; j < PT; ++j)
+        if (k0 + j < n) point_coeffs(a, c, s.tri, k0 + j, f[j], I2[j], I0[j], J1m[j], t.U3[j]);
     __syncthreads();
     cell_solves<TP, G, R>(a, s.tri, cell);
 }
 
+// The coefficients and the solves of one cell on one warp: virtual warp v of
+// the CTA form is this warp's v-th sweep, with the sums in the same order, so
+// that the results have its bits.
+template <typename TP, int G, int R, int PT, int V>
+__device__ __forceinline__ void solve_cell(const CollideArgs& a, const long long cell, double* smem) {
+    const int n = a.np;
+    const int lane = threadIdx.x & 31;
+    TriRows tri;
+    tri.a = smem; tri.b = smem + n; tri.c = smem + 2 * n; tri.scat = smem + 3 * n;
+    const StepP sp = step_params(a);
+    double f[V][PT];
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int j = 0; j < PT; ++j) {
+            const int k = PT * (32 * v + lane) + j;
+            f[v][j] = k < n ? a.f00[cell * n + k] : 0.0;
+        }
+    double I2[V][PT], I0[V][PT], J1m[V][PT], r2[V], r0[V], r1[V], T2[V], T0[V], T1[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        double lo = __shfl_up_sync(kFull, f[v][PT - 1], 1), hi = __shfl_down_sync(kFull, f[v][0], 1);
+        const double below = v > 0 ? __shfl_sync(kFull, f[v > 0 ? v - 1 : 0][PT - 1], 31) : 0.0;
+        const double over = v + 1 < V ? __shfl_sync(kFull, f[v + 1 < V ? v + 1 : 0][0], 0) : 0.0;
+        if (lane == 0) lo = below;
+        if (lane == 31) hi = over;
+        double s2 = 0.0, s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int j = 0; j < PT; ++j) {
+            const int k = PT * (32 * v + lane) + j;
+            const bool in = k < n, up = k + 1 < n;
+            const double fm = j > 0 ? f[v][j > 0 ? j - 1 : 0] : lo, fp = j + 1 < PT ? f[v][j + 1 < PT ? j + 1 : 0] : hi;
+            I2[v][j] = fma_rn(in ? __ldg(a.U4 + k) : 0.0, f[v][j], mul_rn(in ? __ldg(a.U4m1 + k) : 0.0, fm));
+            I0[v][j] = fma_rn(in ? __ldg(a.U2 + k) : 0.0, f[v][j], mul_rn(in ? __ldg(a.U2m1 + k) : 0.0, fm));
+            J1m[v][j] = fma_rn(up ? __ldg(a.U1 + k + 1) : 0.0, fp, mul_rn(up ? __ldg(a.U1m1 + k + 1) : 0.0, f[v][j]));
+            s2 += I2[v][j]; s0 += I0[v][j]; s1 += J1m[v][j];
+        }
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const double u2 = __shfl_up_sync(kFull, s2, off), u0 = __shfl_up_sync(kFull, s0, off);
+            const double u1 = __shfl_down_sync(kFull, s1, off);
+            if (lane >= off) { s2 += u2; s0 += u0; }
+            if (lane + off < 32) s1 += u1;
+        }
+        T2[v] = __shfl_sync(kFull, s2, 31);
+        T0[v] = __shfl_sync(kFull, s0, 31);
+        T1[v] = __shfl_sync(kFull, s1, 0);
+        r2[v] = __shfl_up_sync(kFull, s2, 1);
+        r0[v] = __shfl_up_sync(kFull, s0, 1);
+        r1[v] = __shfl_down_sync(kFull, s1, 1);
+        if (lane == 0) { r2[v] = 0.0; r0[v] = 0.0; }
+        if (lane == 31) r1[v] = 0.0;
+    }
+    double S2 = 0.0, S0 = 0.0;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        double b1 = 0.0;
+#pragma unroll
+        for (int w = v + 1; w < V; ++w) b1 += T1[w];
+        r2[v] += S2; r0[v] += S0; r1[v] += b1;
+        S2 += T2[v]; S0 += T0[v];
+#pragma unroll
+        for (int j = 0; j < PT; ++j) {
+            r2[v] += I2[v][j]; I2[v][j] = r2[v];
+            r0[v] += I0[v][j]; I0[v][j] = r0[v];
+        }
+#pragma unroll
+        for (int j = PT - 1; j >= 0; --j) { r1[v] += J1m[v][j]; J1m[v][j] = r1[v]; }
+    }
+    const double temperature = S2 * (4.0 * M_PI), density = S0 * (4.0 * M_PI);
+    const CoeffP c = coeff_params(a, sp, log_ee(density, temperature, a.density_np),
+                                  zlog_ei(density, temperature, a.density_np, a.Zeta), density);
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int j = 0; j < PT; ++j) {
+            const int k = PT * (32 * v + lane) + j;
+            if (k < n) point_coeffs(a, c, tri, k, f[v][j], I2[v][j], I0[v][j], J1m[v][j], __ldg(a.U3 + k));
+        }
+    __syncwarp();
+    cell_solves<TP, G, R>(a, tri, cell);
+}
+
 // What it measured (B200, the collision launch, one cell a warp before -> now): 256 cells of 128 points, l0 = 1, ten e-e
 // substeps 0.21 -> 0.10 ms for the three calls of a step; 384 cells of 432 points, l0 = 31 (the staged-chunk kernel
-// before) 0.88 -> 0.2 ms; Weibel (16384 cells of 96 points, 48 planes) equal in FP64, 0.65 -> 0.60 ms in the FP32 split;
-// 20833 cells of 96 points 0.50 -> 0.44 ms with l0 = 8, but 0.26 -> 0.30 ms with l0 = 1, whose e-e part a warp a cell does
-// with fewer scans; 512 uneven 1D problems 9.0 -> 7.2 ms a step.  Long e-e runs on few cells wait on the slope's three
-// barriers and its logarithm; many cells on FP64 latency.
+// before) 0.88 -> 0.2 ms; 512 uneven 1D problems 9.0 -> 7.2 ms a step.  Long e-e runs on few cells wait on the slope's
+// three barriers and its logarithm; for many cells see collide_solve_kernel.
 template <typename TP, int K, bool MANY>
 __global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K, MANY)) collide_cell_kernel(const CollideArgs a) {
     extern __shared__ double smem[];
     for (long long cell = blockIdx.x; cell < a.cells; cell += gridDim.x) {
         collide_cell<TP, form_lanes(K), form_run(K), form_points(K)>(a, cell, smem);
         __syncthreads();
+    }
+}
+
+// The e-e substeps alone, for more cells than a wave: without the solves' registers 18 to 24 warps an SM (ee_blocks).
+// 20000 cells, one substep, in the kernel above -> here: 96 points 169 -> 162 us, 128 228 -> 198, 200 443 -> 389, 257
+// 877 -> 372 (two CTAs an SM for one).
+template <int K>
+__global__ void __launch_bounds__(32 * form_warps(K), ee_blocks(K)) collide_ee_kernel(const CollideArgs a) {
+    extern __shared__ double smem[];
+    constexpr int PT = form_points(K);
+    const int n = a.np, pts = PT * (int)blockDim.x, k0 = PT * (int)threadIdx.x;
+    const CellSmem s = carve_cell(smem, n, pts);
+    PointTab<PT> t;
+    load_tab<PT>(a, k0, t);
+    const StepP sp = step_params(a);
+    if (threadIdx.x == 0) { s.f[-1] = 0.0; s.f[pts] = 0.0; s.g[-1] = 0.0; s.g[pts] = 0.0; }
+    for (long long cell = blockIdx.x; cell < a.cells; cell += gridDim.x) {
+        double f[PT];
+#pragma unroll
+        for (int j = 0; j < PT; ++j) f[j] = k0 + j < n ? a.f00[cell * n + k0 + j] : 0.0;
+        cell_ee<PT>(a, sp, s, t, k0, f);
+#pragma unroll
+        for (int j = 0; j < PT; ++j)
+            if (k0 + j < n) a.f00[cell * n + k0 + j] = f[j];
+    }
+}
+
+// Coefficients and solves of many cells, one warp a cell: 16 cells an SM under way where CTAs of their own leave 2 to 8,
+// most of whose lanes wait for the one that has the plane.  collide_f1 alone, l0 = 1, 20000 cells, a CTA a cell -> here:
+// 64 points 150 -> 96 us, 128 289 -> 101, 257 1161 -> 250; a whole collision step of 96 points 289 -> 237, of 200
+// 788 -> 530; Weibel (16384 cells of 96 points, 48 planes), the whole step 3.55 -> 3.47 ms, FP32 split 2.68 -> 2.61.
+template <typename TP, int K>
+__global__ void __launch_bounds__(32, solve_blocks(K)) collide_solve_kernel(const CollideArgs a) {
+    extern __shared__ double smem[];
+    for (long long cell = blockIdx.x; cell < a.cells; cell += gridDim.x) {
+        solve_cell<TP, form_lanes(K), form_run(K), form_points(K), form_warps(K)>(a, cell, smem);
+        __syncwarp();
     }
 }
 
@@ -1153,9 +1315,9 @@ int collide_form(int np) {
 }
 // Planes of one l a lane group takes at a time: as many as make the longest
 // group's work shortest, a unit's pivots counted as three planes
-int collide_unit_planes(int np, int l0, int m0, int mmax_coll, int do_l1, int do_lm) {
+int collide_unit_planes(int np, int l0, int m0, int mmax_coll, int do_l1, int do_lm, int warps) {
     if (np > 512) return 1;
-    const int K = collide_form(np), groups = 32 * form_warps(K) / form_lanes(K);
+    const int K = collide_form(np), groups = 32 * (warps ? warps : form_warps(K)) / form_lanes(K);
     int best = 1, cost = 1 << 30;
     const int widest = 1 + 2 * std::min(std::min(l0, m0), mmax_coll);
     for (int C = 1; C <= widest; ++C) {
@@ -1175,12 +1337,37 @@ size_t collide_tri_smem_per_cell(int np, int l0) {
 
 namespace {
 template <typename TP>
-cudaError_t launch_cell(const CollideArgs& a, cudaStream_t st, int blocks) {
-    return with_form(collide_form(a.np), [&](auto form) {
+cudaError_t launch_cell(const CollideArgs& a0, cudaStream_t st, int blocks) {
+    return with_form(collide_form(a0.np), [&](auto form) {
         constexpr int K = decltype(form)::value;
-        // more cells than a wave, few planes: see form_blocks
+        CollideArgs a = a0;
+        int planes = 0;   // that this call solves
+        for (int l = 1; l <= a.l0; ++l)
+            if (l == 1 ? a.do_l1 : a.do_lm) planes += 1 + 2 * std::min(std::min(l, a.m0), a.mmax_coll);
+        const int groups = 32 * form_warps(K) / form_lanes(K);
+        // A CTA a cell leaves the lane groups that have no plane idle while the others solve, and only few cells are
+        // resident.  A wave of such CTAs is as good as warps of their own (collide_solve_kernel) up to these numbers of
+        // cells: one wave where most groups are idle, about one wave of the warps (one and a half with e-e substeps, which
+        // then take a launch of their own) where all find a plane at most once, four beyond.  Both sides at 96 points, in
+        // us, CTA / warp: one plane and e-e, 2400 cells 47 / 47, 8000 125 / 104; 16 planes 2400 cells 84 / 98, 8000
+        // 231 / 219, 16000 455 / 408; 48 planes 2400 cells 168 / 215, 8000 481 / 461, 16000 901 / 811.
+        const long long sms = sm_count(), wave = solve_blocks(K) * sms;
+        const bool idle = a.do_ee || K > 32 ? 4 * planes <= groups : 5 * planes <= 3 * groups;
+        const long long limit = idle ? form_blocks(K, true) * sms : planes > groups ? 4 * wave : a.do_ee ? 3 * wave / 2 : wave;
+        const bool split = a.cells > limit, wide = a.cells > form_blocks(K, false) * sms;   // wide: more than a wave
+        if (a.do_ee && (split || (!planes && wide))) {
+            collide_ee_kernel<K><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess || !planes) return e;
+            a.do_ee = 0;
+        }
+        if (split) {
+            a.unit_planes = collide_unit_planes(a.np, a.l0, a.m0, a.mmax_coll, a.do_l1, a.do_lm, 1);
+            collide_solve_kernel<TP, K><<<blocks, 32, 4 * sizeof(double) * a.np, st>>>(a);
+            return cudaGetLastError();
+        }
         if constexpr (form_blocks(K, true) > form_blocks(K, false)) {
-            if (a.cells > (long long)form_blocks(K, false) * sm_count() && a.nplanes <= kManyPlanes) {
+            if (wide && planes <= kManyPlanes) {
                 collide_cell_kernel<TP, K, true><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
                 return cudaGetLastError();
             }

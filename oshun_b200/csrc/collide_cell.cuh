@@ -17,25 +17,36 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 
 // The forms: K = G R / 8 (the row's points, rounded up to the form's, over 8).
-// One thread a point up to 256 points, two beyond.
-constexpr int form_lanes(int K) { return K <= 8 ? 8 : (K <= 16 ? 16 : 32); }
+// One thread a point up to 256 points, two beyond.  113 to 128 points take runs
+// of 4 on 32 lanes: with 8 on 16 lanes two planes share a warp, but a row's
+// pieces lie 64 bytes apart (20000 cells, l0 = 1, the f1 call 150 -> 101 us;
+// 5000 cells, 15 planes, their call 143 -> 93; 64 cells of 48 planes 29 -> 33).
+constexpr int form_lanes(int K) { return K <= 8 ? 8 : (K < 16 ? 16 : 32); }
 constexpr int form_run(int K) { return 8 * K / form_lanes(K); }
 constexpr int form_points(int K) { return K <= 32 ? 1 : 2; }
 constexpr int form_warps(int K) { return (8 * K + 32 * form_points(K) - 1) / (32 * form_points(K)); }
-// resident CTAs per SM up to 256 points, of 128 registers a thread; more of 80
-// registers for launches of many cells (`many`), where a lane's run is shorter
-// than 8 points.  Many cells are bound by FP64 latency, which more warps hide:
-// 20833 cells of 96 points 0.35 -> 0.30 ms (l0 = 1), 12500 of 160 0.345 ->
-// 0.285 ms.  On few cells the slopes pay for their spills (256 cells of 96
-// points, ten e-e substeps: 118 us against 135), and with runs of 8 points
-// they do on any number (256 cells of 128 points: 119 against 140).  With many
-// planes the solves do: a step of 16384 cells of 96 points with 48 planes took
-// 3.60 ms against 3.56, one of 4096 cells of 184 points with 29 planes 1.43
-// against 1.45.
+// Resident CTAs per SM up to 256 points, of 128 registers a thread; more of 80
+// registers for launches of many cells (`many`) and for batches, where a lane's
+// run is shorter than 8 points: more warps hide the FP64 latency.  On few cells
+// the spills cost more (256 cells of 96 points, ten e-e substeps: 118 us
+// against 135).  With few planes (kManyPlanes) the many form is the faster one:
+// 8000 cells of 96 points, 1D, 2 / 8 / 24 planes 138 / 187 / 307 -> 123 / 166 /
+// 293 us; of 184 points 336 / 466 / 750 -> 246 / 350 / 600.  With several
+// planes of one l (m0 >= 2) it depends on how far a row length's form spills: 15
+// planes, 5000 cells, 40 / 72 / 96 / 112 / 128 / 184 points x 1.02 / 0.93 /
+// 1.04 / 1.08 / 0.93 / 0.84; 48 planes x 1.07 / 0.98 / 1.11 / 1.16 / 0.92 /
+// 0.89.
 constexpr int kManyPlanes = 32;
 constexpr int form_blocks(int K, bool many) {
     return K <= 32 ? (many && form_run(K) < 8 ? 24 : 16) / form_warps(K) : 1;
 }
+// the e-e substeps alone: 96 registers a thread (no spills) where that leaves a
+// CTA as many, 20000 cells of 64 / 128 / 184 points 124 / 226 / 364 -> 114 / 198
+// / 331 us against 80 registers; 7 or 8 warps a CTA would then leave two (200
+// points 389 -> 458 us)
+constexpr int ee_blocks(int K) { return K > 32 ? 16 / form_warps(K) : K >= 28 ? 3 : 20 / form_warps(K); }
+// the solves on a warp a cell
+constexpr int solve_blocks(int K) { return K <= 32 ? 16 : 8; }
 template <typename F>
 cudaError_t with_form(int K, F&& go) {
     switch (K) {

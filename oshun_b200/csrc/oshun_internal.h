@@ -235,7 +235,8 @@ cudaError_t launch_rk_combine(double* out, const double* v0, double a0, const do
                               const double* base, long long n, cudaStream_t st);
 // the tridiagonal collision kernel's form for rows of np <= 512 points
 int collide_form(int np);
-int collide_unit_planes(int np, int l0, int m0, int mmax_coll, int do_l1, int do_lm);
+// warps: those of a cell (0: the CTA form's)
+int collide_unit_planes(int np, int l0, int m0, int mmax_coll, int do_l1, int do_lm, int warps = 0);
 // tridiagonal collision step of a batch whose problems share the form
 cudaError_t launch_collide_batch(const CollideBatch& b, int form, int planes_fp32, size_t smem, cudaStream_t s);
 // device clocks {t, t_ee, t_eb} of n problems: t += dt; after a collision step t_ee = t_eb = t
