@@ -92,8 +92,12 @@ struct StageArgs {
     int parts;            // kPart* bits of the RHS evaluated (kPartAll: Actions::Adv; others: the implicit-E actions)
     int withhold;         // fault injection for tests: CTA 0's source producer skips this copy (-1: none)
     // an FP32 gradient on rows that are no multiple of 16 bytes: the global-load
-    // kernel.  Its results are FP64 vectors, which follow the FP32 roundings to
-    // 1e-7; this keeps the order of roundings that they are known by.
+    // kernel.  Its results are FP64 vectors that follow the FP32 roundings, and
+    // this keeps the order of roundings that they are known by.  The two-point
+    // kernel is as accurate in the gradient (3e-8 against FP64 by either) and
+    // more so in the forward step, whose f00 differences it takes in FP64 (a
+    // 20-step heat flux 1e-8 off instead of up to 4e-5), so the two differ by
+    // more than a repeated FP64 result may.
     int global_rows;
     const void* coef_ts;  // coupling table in the arithmetic type (batched launches)
     double* jw;           // [cells][3][8]: per-warp partial sums of Jx, Re Jy, Im Jy (one-point kernels)
@@ -182,7 +186,7 @@ struct CollideBatch {
 // cudaErrorNotSupported when the shape does not fit
 template <typename TS>
 cudaError_t launch_stage_pipe(const StageArgs<TS>& a, int mc, cudaStream_t s);
-// two-point stage kernel (stage_pair.cu): any row length, any parts; cudaErrorNotSupported when the row does not fit
+// two-point stage kernel (stage_pair.cu): rows of any number of points that fit a CTA, any parts; else cudaErrorNotSupported
 template <typename TS>
 cudaError_t launch_stage_pair(const StageArgs<TS>& a, cudaStream_t s);
 cudaError_t launch_stage_fp64(const StageArgs<double>& a, int mc, cudaStream_t s);

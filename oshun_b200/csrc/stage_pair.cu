@@ -1,6 +1,9 @@
-// Two-point pipelined RK4-stage kernel, any row length: Actions::Adv (OSHUN-1/def-Actions.cpp:73-94),
+// Two-point pipelined RK4-stage kernel: Actions::Adv (OSHUN-1/def-Actions.cpp:73-94),
 // or a part of it, on one stage input folded into the stage update of
-// Runge_Kutta_4::advance_p1 (OSHUN-1/def-RK.cpp:110-145).
+// Runge_Kutta_4::advance_p1 (OSHUN-1/def-RK.cpp:110-145).  Rows may have any
+// number of points up to what a CTA's consumers hold (points() and
+// consumer_warps() below): 512 with m0 = 0; 640 (FP32: 896) with m0 = 1, 2; 320
+// (640) with m0 = 3 to 6; 192 (384) with m0 = 7, 8.
 //
 // The launcher of vlasov.cu takes it for m0 = 0, for momentum rows that are
 // no multiple of 16 bytes and for partial right-hand sides (the implicit-E
@@ -12,7 +15,10 @@
 // issues one barrier round trip a harmonic -- 8192 cells, l0 = 16, np = 256,
 // FP64 1.40 -> 0.96 ms (the one-point kernel); rows of 75 points on 61 x 45
 // cells, l0 = 5, m0 = 3, with collisions 1.48 -> 0.94 ms (the global-load
-// kernel re-read every neighbour through L1); the RK2 actions on 64 x 48 cells,
+// kernel re-read every neighbour through L1); rows of 75 points, 4000 cells, l0 = 8,
+// m0 = 0, two steps, one point a thread -> two: FP64 575 -> 340 us, FP32 577 -> 340
+// (the global-load kernel 625 and 478: with one point a tile held 2 cells and
+// copied as many neighbours; two points halve the threads of a cell); the RK2 actions on 64 x 48 cells,
 // l0 = 8, m0 = 3, np = 96, with collisions 2.46 -> 0.95 ms (global loads).  The
 // full right-hand side of m0 >= 3 on 16-byte rows is not taken: its registers
 // leave 8 to 12 warps an SM here, and Weibel (128 x 128, l0 = m0 = 6, np = 96)
@@ -38,8 +44,8 @@
 // neighbours and their y-1/y+1 cells, every momentum point, with the tile's
 // six fields beside f00 -- into a ring of slots; the other streams the RK
 // operands of each target (l, m) into a ring of their own.  Rows that are no
-// multiple of 16 bytes come as the aligned spans that hold them (SHIFT), one
-// point a thread.  Copies complete on mbarriers, and every wait is bounded.
+// multiple of 16 bytes come as the aligned spans that hold them (SHIFT), and
+// a thread loads its two points of them one by one.  Copies complete on mbarriers, and every wait is bounded.
 //
 // The consumer warps share no barrier: each half-warp writes its sums of the
 // current to shared memory and the last one of a cell to do so adds them in
@@ -160,10 +166,13 @@ __device__ __forceinline__ auto second(const V& v) {
     if constexpr (kOne<V>) return V(0);
     else return v.y;
 }
-// a thread's points from shared memory (a pair's address is aligned)
-template <typename V, typename T>
-__device__ __forceinline__ V ld_v(const T* p) {
+// a thread's points from shared memory; o2: from the first to the second.  A
+// pair's address is aligned, except in rows that are no multiple of 16 bytes
+// (SHIFT).
+template <bool SHIFT, typename V, typename T>
+__device__ __forceinline__ V ld_v(const T* p, const int o2) {
     if constexpr (kOne<V>) return *p;
+    else if constexpr (SHIFT) return V{p[0], p[o2]};
     else return *reinterpret_cast<const V*>(p);
 }
 // sums of three and two products added to an accumulator.  FP64: the products
@@ -239,6 +248,7 @@ struct Ops {
 // the planes' distance in elements, q the plane.
 struct Nb {
     int ctr, pp;
+    int o2;                   // from the first point to the second (SHIFT: 0 where the row ends between them)
     int x, ym, yp;            // from ctr: x-1 is -x, x+1 is +x (SHIFT: ym and yp are offsets in the slot)
     int xm, xp;               // SHIFT: offsets in the slot
     int ac, axm, axp, aym, ayp, b, bxm, bxp;   // SHIFT: A of each piece, B of the planes and of the x neighbours
@@ -290,15 +300,16 @@ __device__ __forceinline__ T above(const V f, const T fp) {
 }
 
 // stencils of one component of a source: value, G, H, x and y differences (times v)
-template <typename TS, typename V, bool Y>
+template <typename TS, typename V, bool Y, bool SHIFT>
 __device__ __forceinline__ void stencils(const Ops<TS> op, const Nb& nb, const Th<TS, V>& th, const V ipx,
                                          const typename Arith<TS>::S gfac, const typename Arith<TS>::S hp0,
                                          const TS* __restrict__ ref, V& f, V& G, V& H, V& dx, V& dy) {
-    f = ld_v<V>(op.c);
+    auto ld = [&](const TS* q) { return ld_v<SHIFT, V>(q, nb.o2); };
+    f = ld(op.c);
     // below p = 0 lies another point of the slot: G and H there do not use it
     TS fm = op.c[-1], fp = op.c[nb.pp];
-    dx = v_mul(v_sub(ld_v<V>(op.xm), ld_v<V>(op.xp)), th.vr);
-    if constexpr (Y) dy = v_mul(v_sub(ld_v<V>(op.ym), ld_v<V>(op.yp)), th.vr);
+    dx = v_mul(v_sub(ld(op.xm), ld(op.xp)), th.vr);
+    if constexpr (Y) dy = v_mul(v_sub(ld(op.ym), ld(op.yp)), th.vr);
     if constexpr (sizeof(TS) == 4) {
         // FP32 planes hold f - ref (the plane's momentum profile, if it keeps
         // one): the differences above act on the stored deviation alone, the
@@ -333,9 +344,9 @@ __device__ __forceinline__ void couple_src(Acc<V, MC>& A0, Acc<V, MC>& A1, Acc<V
     const S2<S> cg = coef2(c, kBm2), ch = coef2(c, kInvpax);   // (2 b_m, gfac), (invpax, hp0)
     const V ipx = v_mul(ch.a, th.invp);
     V fr, Gr, Hr, dxr, dyr, fi, Gi, Hi, dxi, dyi;
-    stencils<TS, V, MC >= 1>(operands<SHIFT>(sb, nb, q), nb, th, ipx, cg.b, ch.b, ref, fr, Gr, Hr, dxr, dyr);
+    stencils<TS, V, MC >= 1, SHIFT>(operands<SHIFT>(sb, nb, q), nb, th, ipx, cg.b, ch.b, ref, fr, Gr, Hr, dxr, dyr);
     if constexpr (DN)
-        stencils<TS, V, true>(operands<SHIFT>(sb + seg, nb, q + 1), nb, th, ipx, cg.b, ch.b, ref ? ref + np : ref, fi, Gi,
+        stencils<TS, V, true, SHIFT>(operands<SHIFT>(sb + seg, nb, q + 1), nb, th, ipx, cg.b, ch.b, ref ? ref + np : ref, fi, Gi,
                               Hi, dxi, dyi);
     // Ex and x advection: (s+1, M), (s-1, M)
     {
@@ -396,7 +407,7 @@ __device__ __forceinline__ void couple_src(Acc<V, MC>& A0, Acc<V, MC>& A1, Acc<V
 
 // couplings of the f00 source into row 1 (A, from zero); G00 at p = 0 from
 // the extrapolated f00(p=0) (OSHUN-1/def-VlasovMax.cpp:520-535)
-template <int MC, typename TS, typename V>
+template <int MC, bool SHIFT, typename TS, typename V>
 __device__ __forceinline__ void couple_f00(Acc<V, MC>& A, const CoefS<TS>* __restrict__ c,
                                            const Ops<double> op, const Nb& nb, const Th<TS, V>& th,
                                            const double g00_s, const double g00_inv, const double g00_gr) {
@@ -406,9 +417,10 @@ __device__ __forceinline__ void couple_f00(Acc<V, MC>& A, const CoefS<TS>* __res
         if constexpr (sizeof(TS) == 8) return v;
         else return make_v<V>((float)first(v), (float)second(v));
     };
-    const V f = round(ld_v<VD>(op.c));
+    auto ld = [&](const double* q) { return ld_v<SHIFT, VD>(q, nb.o2); };
+    const V f = round(ld(op.c));
     const TS fm = (TS)op.c[-1], fp = (TS)op.c[nb.pp];
-    const V dx = v_mul(round(v_sub(ld_v<VD>(op.xm), ld_v<VD>(op.xp))), th.vr);
+    const V dx = v_mul(round(v_sub(ld(op.xm), ld(op.xp))), th.vr);
     V G = p_diff(f, fm, fp);
     if (th.is0) {
         const TS f1 = above(f, fp);
@@ -418,7 +430,7 @@ __device__ __forceinline__ void couple_f00(Acc<V, MC>& A, const CoefS<TS>* __res
     const S2<S> e = coef2(c, kExG);
     A.R[0] = v_fma(s_mul(e.a, th.ex), G, v_mul(e.b, dx));
     if constexpr (MC >= 1) {
-        const V dy = v_mul(round(v_sub(ld_v<VD>(op.ym), ld_v<VD>(op.yp))), th.vr);
+        const V dy = v_mul(round(v_sub(ld(op.ym), ld(op.yp))), th.vr);
         const S2<S> g2 = coef2(c, kEmG);
         A.R[1] = v_fma(s_mul(g2.a, th.ey), G, v_mul(g2.b, dy));
         A.I[1] = v_mul(s_neg(s_mul(g2.a, th.ez)), G);
@@ -747,6 +759,7 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
 
     Nb nb;
     nb.pp = PT == 1 ? (pc + 1 < np ? 1 : 0) : (pc + 2 < np ? 2 : 1);
+    nb.o2 = pc1 - pc;
     nb.p = pc;
     nb.p_1 = pc1;
     nb.p_m = pc - (pc > 0 ? 1 : 0);
@@ -830,8 +843,14 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
     TS* out = has_out ? a.pl_out + o : nullptr;
     TS* acc = a.pl_A + o;
     auto put = [&](TS* d, const V v) {
-        if (pv) *reinterpret_cast<V*>(d) = v;
+        if constexpr (SHIFT && PT > 1) {
+            if (pv) d[0] = first(v);
+            if (pv1) d[1] = second(v);
+        } else {
+            if (pv) *reinterpret_cast<V*>(d) = v;
+        }
     };
+    auto ld = [&](const TS* q) { return ld_v<SHIFT, V>(q, nb.o2); };
     auto tgt_acquire = [&]() { if (staged) mbar_wait_or_exit(cs.tgt.bar, cs.tgt.phase, err, wlim); };
     auto tgt_release = [&]() {
         if (staged) {
@@ -846,9 +865,9 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
         }
         if (staged) {
             const V tt = v_mul(k, make_v<V>((TS)a.c1, (TS)a.c1));
-            if (has_out) put(out, v_add(ld_v<V>(B), tt));
+            if (has_out) put(out, v_add(ld(B), tt));
             const TS* Y = reinterpret_cast<const TS*>(reinterpret_cast<const unsigned char*>(B) + yoff);
-            put(acc, v_fma(tt, make_v<V>((TS)a.c2, (TS)a.c2), ld_v<V>(Y)));
+            put(acc, v_fma(tt, make_v<V>((TS)a.c2, (TS)a.c2), ld(Y)));
         } else {
             put(out, k);
         }
@@ -902,7 +921,7 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
     {
         Nb n0 = nb;
         if constexpr (sizeof(TS) == 4) place(n0, 8);
-        couple_f00<MC, TS, V>(A1, BATCH ? slot_coef() : coef, operands<SHIFT>(reinterpret_cast<const double*>(smem + cs.src.off), n0, 0), n0, th,
+        couple_f00<MC, SHIFT, TS, V>(A1, BATCH ? slot_coef() : coef, operands<SHIFT>(reinterpret_cast<const double*>(smem + cs.src.off), n0, 0), n0, th,
                               a.g00_s, a.g00_inv, a.g00_gr);
     }
     release();
@@ -930,7 +949,7 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
                     auto quad = [&](double (&j)[PT], const TS* v, const TS* rf) {
 #pragma unroll
                         for (int k = 0; k < PT; ++k) {
-                            double f = (double)v[k];
+                            double f = (double)v[k == 0 ? 0 : nb.o2];
                             if (rf) f = add_rn(f, (double)rf[k == 0 ? pc : pc1]);
                             if (k == 0 ? pv : pv1) j[k] = mul_rn(ldg(a.wj + (k == 0 ? pc : pc1)), f);
                         }
@@ -1016,15 +1035,16 @@ inline int tile_cells(int np, int nx, int segments) { return batch_cells(np, nx,
 // multiples of 4 warps: 8 warps leave 255 registers a thread, 12 warps 168, 16
 // warps 128; each form takes the most warps whose registers hold its
 // accumulators without spilling (the rings leave the L1 too small to hold
-// spilled registers).  Two points a thread where that fits and rows are
-// 16-byte multiples (a pair's loads are aligned then), else one.
+// spilled registers).  Two points a thread where that fits, else one (FP64, m0
+// >= 3).  FP32 rows of 51 points on 64 x 64 cells, l0 = m0 = 6, two steps 2.18
+// -> 1.60 ms with two, in spite of 376 bytes spilled; FP64 rows of 129 points
+// on 30 x 31 cells, l0 = 4, m0 = 2, 646 -> 407 us (128 bytes spilled).
 template <int MC, typename TS, bool SHIFT>
-constexpr int points() { return !SHIFT && (sizeof(TS) == 4 || MC <= 2) ? 2 : 1; }
+constexpr int points() { return sizeof(TS) == 4 || MC <= 2 ? 2 : 1; }
 template <int MC, typename TS, bool SHIFT>
 constexpr int consumer_warps() {
     if (MC == 0) return 8;
     if (sizeof(TS) == 8) return MC <= 6 ? 10 : 6;
-    if (SHIFT) return MC <= 4 ? 14 : 10;
     return MC <= 2 ? 14 : MC <= 6 ? 10 : 6;
 }
 // CTAs per SM: two for m0 = 0, so that one CTA's tile starts and ends overlap

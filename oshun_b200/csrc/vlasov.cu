@@ -1,7 +1,10 @@
 // Fused RHS + RK4-stage kernel on global loads, for momentum rows too long
-// for the pipelined kernel of stage_pipe.cu (nump above 512 with m0 = 0, 640
-// to 896 for a few m0, 384 for FP64 with m0 >= 4, or rings that do not fit in
-// shared memory); the launcher below takes the pipelined kernel elsewhere.
+// for the pipelined kernels: more points than stage_pair.cu takes (512 with m0
+// = 0; FP64 640 with m0 = 1, 2, 320 with m0 = 3 to 6, 192 with m0 = 7, 8; FP32
+// 896, 640 and 384), unless stage_pipe.cu takes them (the full right-hand side
+// of m0 >= 1, rows of 16-byte multiples to 256 points), or rings that do not
+// fit in shared memory; and for FP32 gradients on rows that are no multiple of
+// 16 bytes (StageArgs.global_rows).
 //
 // One thread owns one (cell, p) point of every harmonic, walks the source
 // harmonics row by row (l = 0..l0, all m of a row unrolled) and scatters
