@@ -96,7 +96,7 @@ struct StageArgs {
     // this keeps the order of roundings that they are known by.  The two-point
     // kernel is as accurate in the gradient (3e-8 against FP64 by either) and
     // more so in the forward step, whose f00 differences it takes in FP64 (a
-    // 20-step heat flux 1e-8 off instead of up to 4e-5), so the two differ by
+    // 6-step heat flux 1e-8 off instead of up to 4e-5), so the two differ by
     // more than a repeated FP64 result may.
     int global_rows;
     const void* coef_ts;  // coupling table in the arithmetic type (batched launches)

@@ -1117,9 +1117,18 @@ cudaError_t pair_form(const StageArgs<TS>& a, cudaStream_t s) {
     constexpr int elem = (int)sizeof(TS);
     if ((a.np + 31) / 32 > max_hw) return cudaErrorNotSupported;
     int tx = tile_cells(a.np, a.nx, max_hw);
+    const int widest = tx;
+    auto tiles_of = [&](int t) { return (long long)a.ny * ((a.nx + t - 1) / t); };
     // at least one tile per SM where the grid has the cells for it
     const long long per_sm = (long long)a.nx * a.ny / sm_count();
     if (tx > per_sm) tx = per_sm > 1 ? (int)per_sm : 1;
+    // one CTA an SM: the fewest cells that leave no CTA a second tile, since a
+    // tile's time is mostly latency (FP32, 16 x 17 cells of 201 points, l0 = 6,
+    // m0 = 4, two steps: tiles of one cell 699 us, of two 401; the global-load
+    // kernel 584)
+    if (MC > 0)
+        for (int t = tx; t <= widest; ++t)
+            if (tiles_of(t) <= sm_count()) { tx = t; break; }
     const int ncoef = (a.l0 + 1) * (a.m0 + 1);
     Plan P;
     auto plan = [&](size_t cap, int t) {
@@ -1140,7 +1149,7 @@ cudaError_t pair_form(const StageArgs<TS>& a, cudaStream_t s) {
     cudaError_t e = ensure_dyn_smem((const void*)kernel, P.total);
     if (e != cudaSuccess) return e;
     const int threads = P.hw * (32 / per_warp) + 64;
-    const long long tiles = (long long)a.ny * ((a.nx + tx - 1) / tx);
+    const long long tiles = tiles_of(tx);
     int per_sm_ctas = 1;
     if (tile_min_blocks<MC>() > 1) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_ctas, kernel, threads, P.total);

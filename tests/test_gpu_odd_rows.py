@@ -27,6 +27,7 @@ ROWS = [
     dict(l0=3, m0=1, nump=641, numx=3, numy=2),
     dict(l0=5, m0=2, nump=65, numx=23, numy=9),
     dict(l0=4, m0=3, nump=319, numx=3, numy=2),
+    dict(l0=3, m0=1, nump=201, numx=16, numy=17),   # few more cells than SMs: tiles of more than one
 ]
 ROWS32 = [dict(l0=l0, m0=m0, nump=n, numx=nx, numy=ny)
           for l0, m0, nx, ny in [(3, 0, 9, 1), (3, 1, 7, 3), (4, 2, 5, 4), (4, 3, 5, 3), (5, 4, 4, 3), (6, 5, 3, 3),
