@@ -316,14 +316,14 @@ __global__ void to_fp64_kernel(const float* __restrict__ src, double* __restrict
 // an SM: the e-e sweeps, most of a cell's time, hold far fewer registers than
 // the solves, which spill a little for it.
 template <int K>
-__global__ void __launch_bounds__(32 * form_warps(K), 16 / form_warps(K))
+__global__ void __launch_bounds__(32 * point_warps(K), 16 / point_warps(K))
     collide_adj_kernel(const CollTables T, const adjc::StepT st, const double* __restrict__ y, double* __restrict__ lam,
                        double* __restrict__ ws, const long long wsz, const int smem_ws) {
     extern __shared__ double smem[];
     const long long x = blockIdx.x;
     const int np = T.np;
     double* starts = smem_ws ? smem + adjc::cell_doubles(np, blockDim.x) : ws + x * wsz;
-    adjc::collide_cell_T<form_lanes(K), form_run(K)>(T, st, y + x * np, y + st.pstride + x * np, lam + x * np,
+    adjc::collide_cell_T<form_lanes(K), form_run(K), point_warps(K)>(T, st, y + x * np, y + st.pstride + x * np, lam + x * np,
                                                      lam + st.pstride + x * np, smem, starts);
 }
 
@@ -374,13 +374,13 @@ cudaError_t launch_collide_adj(const CollTables& T, int l0, int nx, const double
     return with_form(K, [&](auto form) {
         constexpr int F = decltype(form)::value;
         if constexpr (F <= 32) {
-            const size_t base = sizeof(double) * adjc::cell_doubles(T.np, 32 * form_warps(F));
+            const size_t base = sizeof(double) * adjc::cell_doubles(T.np, 32 * point_warps(F));
             const size_t starts = sizeof(double) * (size_t)nsub * T.np;
             const int in_smem = base + starts <= 100 * 1024;
             const size_t smem = base + (in_smem ? starts : 0);
             const cudaError_t e = ensure_dyn_smem((const void*)collide_adj_kernel<F>, smem);
             if (e != cudaSuccess) return e;
-            collide_adj_kernel<F><<<nx, 32 * form_warps(F), smem, st>>>(T, s, y, lam, ws, wsz, in_smem);
+            collide_adj_kernel<F><<<nx, 32 * point_warps(F), smem, st>>>(T, s, y, lam, ws, wsz, in_smem);
             return cudaGetLastError();
         }
         return cudaErrorInvalidValue;

@@ -118,14 +118,15 @@ __device__ __forceinline__ double scans_T(const Tab& t, const int k, const int n
 struct Slope {
     double I4, I2, J1, raw, lnee, dn, dT, fa, fb;
 };
+template <int W>
 __device__ __forceinline__ double ee_slope(const CollTables& T, const Mem& s, const Tab& t, const int k,
                                            const double f, Slope& o) {
     const int n = T.np;
     double fin[1] = {f}, fm[1], fp[1], I4[1], I2[1], J1[1], S4, S2;
-    neighbours<1>(s.f, k, fin, fm, fp);
+    neighbours<1, W>(s.f, k, fin, fm, fp);
     o.fa = s.f[0];
     o.fb = s.f[1];
-    cell_scans<1>(t.t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
+    cell_scans<1, W>(t.t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
     double G[1], Gm[1], Gp[1];
     if (k < T.NB) {
         const double f00 = (o.fa - o.fb * t.t.r) * t.t.inv1r, df = o.fb - f00;
@@ -136,20 +137,21 @@ __device__ __forceinline__ double ee_slope(const CollTables& T, const Mem& s, co
         G[0] = (I4[0] + t.t.U3[0] * J1[0]) * f - 3.0 * I2[0] * J1[0];
     }
     o.lnee = adj::log_ee_d(4.0 * adj::kPi * S2, 4.0 * adj::kPi * S4, T.density_np, &o.dn, &o.dT);
-    neighbours<1>(s.g, k, G, Gm, Gp);
+    neighbours<1, W>(s.g, k, G, Gm, Gp);
     const double D = k < n - 1 ? (G[0] - Gp[0]) * t.t.Pn[0] : G[0];
     o.raw = (k == 0 ? ((-G[0]) * t.t.two_v0s - D) : ((Gm[0] - G[0]) * t.t.Pm[0] - D)) * t.t.Qn[0];
     o.I4 = I4[0]; o.I2 = I2[0]; o.J1 = J1[0];
     return o.raw * (T.c_kpre * o.lnee);
 }
 // transpose of the slope's derivative at f (adj::ee_slope_T): mu -> the cotangent of f
+template <int W>
 __device__ __forceinline__ double ee_slope_T(const CollTables& T, const Mem& s, const Tab& t, const int k,
                                              const double f, const Slope& o,
                                              const double mu) {
     const int n = T.np;
     const double norm = T.c_kpre * o.lnee;
     double w[1] = {k < n ? mu * norm * t.t.Qn[0] : 0.0}, wm[1], wp[1];
-    neighbours<1>(s.f, k, w, wm, wp);   // (s.g may still be read by the slope before)
+    neighbours<1, W>(s.f, k, w, wm, wp);   // (s.g may still be read by the slope before)
     double sum[3] = {k < n ? mu * o.raw : 0.0, 0.0, 0.0};   // of the norm, f00 (the fit's f at v = 0) and f[1]
     double lf = 0.0, l4 = 0.0, l2 = 0.0, l1 = 0.0;
     if (k < n) {
@@ -349,7 +351,7 @@ __device__ __forceinline__ void solves_T(const CollTables& T, const StepT& p, co
 
 // adj::collide_cell_T: lam00 / laml hold the cotangents of the outputs and
 // receive those of the inputs; starts: nsub rows for the substeps' starts
-template <int G, int R>
+template <int G, int R, int W>
 __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT& p, const double* f00_in,
                                                const double* fl_in, double* lam00, double* laml, double* smem,
                                                double* starts) {
@@ -369,7 +371,7 @@ __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT&
             double fs = f, acc = 0.0;
             for (int st = 0; st < 4; ++st) {
                 Slope o;
-                const double d = ee_slope(T, s, t, k, fs, o);
+                const double d = ee_slope<W>(T, s, t, k, fs, o);
                 acc = fma(st == 0 || st == 3 ? h / 6.0 : h / 3.0, d, acc);
                 fs = fma(st == 2 ? h : 0.5 * h, d, f);
             }
@@ -378,8 +380,8 @@ __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT&
     if (p.eb) {
         // coefficients (adj::reset_coeff)
         double fin[1] = {f}, fm[1], fp[1], I2[1], I0[1], J1[1], S4, S2;
-        neighbours<1>(s.f, k, fin, fm, fp);
-        cell_scans<1>(t.t, fin, fm, fp, s.tot, I2, I0, J1, S4, S2);
+        neighbours<1, W>(s.f, k, fin, fm, fp);
+        cell_scans<1, W>(t.t, fin, fm, fp, s.tot, I2, I0, J1, S4, S2);
         const double Tt = S4 * (4.0 * adj::kPi), N = S2 * (4.0 * adj::kPi);
         double le_dN, le_dT, zl_dN, zl_dT;
         const double lnee = adj::log_ee_d(N, Tt, T.density_np, &le_dN, &le_dT);
@@ -448,7 +450,7 @@ __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT&
             S[0] = fs;
 #pragma unroll
             for (int st = 0; st < 4; ++st) {
-                const double d = ee_slope(T, s, t, k, S[st], o[st]);
+                const double d = ee_slope<W>(T, s, t, k, S[st], o[st]);
                 if (st < 3) S[st < 3 ? st + 1 : 0] = fma(st == 2 ? h : 0.5 * h, d, fs);
             }
             const double out = lam;
@@ -456,7 +458,7 @@ __device__ __forceinline__ void collide_cell_T(const CollTables& T, const StepT&
 #pragma unroll
             for (int st = 3; st >= 0; --st) {
                 const double c = (st == 0 || st == 3 ? h / 6.0 : h / 3.0) * out + (st == 3 ? 0.0 : st == 2 ? h : 0.5 * h) * a;
-                a = ee_slope_T(T, s, t, k, S[st], o[st], c);
+                a = ee_slope_T<W>(T, s, t, k, S[st], o[st], c);
                 lam += a;
             }
         }

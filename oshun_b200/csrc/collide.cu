@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(32) collide_warp_kernel(const CollideArgs a) {
 // Tridiagonal collision step for nump <= 512, one CTA per cell (of many cells,
 // launch_cell: the e-e substeps so and the rest on a warp a cell):
 //   1. f00 e-e substeps and the coefficients of reset_coeff with one thread
-//      per momentum point (two from 257 points on): f, the RK4 stages and the
+//      per momentum point (two from 129 points on): f, the RK4 stages and the
 //      point's velocity tables in registers, the three cumulative integrals as
 //      warp scans joined through the warps' totals, neighbours through shared
 //      memory, three barriers a slope.
@@ -824,17 +824,17 @@ __global__ void __launch_bounds__(32) collide_warp_kernel(const CollideArgs a) {
 //      plane.
 
 // EE_isotropic_conserva::Getslope (def-FokkerPlanck.cpp:192-267): fh = C_ee(fin)
-template <int PT>
+template <int PT, int W>
 __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSmem& s, const PointTab<PT>& t,
                                               const int k0, const double (&fin)[PT], double (&fh)[PT]) {
     const int n = a.np;
     double fm[PT], fp[PT], I4[PT], I2[PT], J1[PT], S4, S2;
-    neighbours<PT>(s.f, k0, fin, fm, fp);
+    neighbours<PT, W>(s.f, k0, fin, fm, fp);
     const double fa = s.f[0], fb = s.f[1];
-    cell_scans<PT>(t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
+    cell_scans<PT, W>(t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
     // the logarithm of the whole cell on the last warp (the first has the fit below): every warp
     // of its own would spend as many FP64 instructions on it as on all the rest of the slope
-    if (threadIdx.x + 32 >= blockDim.x) {
+    if ((int)threadIdx.x >= 32 * (W - 1)) {
         const double norm = a.c_kpre * log_ee(4.0 * M_PI * S2, 4.0 * M_PI * S4, a.density_np);
         if ((threadIdx.x & 31) == 0) s.one[0] = norm;
     }
@@ -852,7 +852,7 @@ __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSm
             G[j] = fma_rn(fma_rn(t.U3[j], J1[j], I4[j]), fin[j], i2);
         }
     }
-    neighbours<PT>(s.g, k0, G, Gm, Gp);
+    neighbours<PT, W>(s.g, k0, G, Gm, Gp);
     const double norm = s.one[0];
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
@@ -1007,7 +1007,7 @@ __device__ __forceinline__ void cell_solves(const CollideArgs& a, const TriRows&
 
 // RK4 substeps of Explicit_EC_FP::loop (RungeKutta4_ee::advance,
 // def-FokkerPlanck.cpp:518-553) on a thread's points of the cell's f00
-template <int PT>
+template <int PT, int W>
 __device__ __forceinline__ void cell_ee(const CollideArgs& a, const StepP& sp, const CellSmem& s, const PointTab<PT>& t,
                                         const int k0, double (&f)[PT]) {
     const double h = sp.hsub;
@@ -1017,7 +1017,7 @@ __device__ __forceinline__ void cell_ee(const CollideArgs& a, const StepP& sp, c
         for (int j = 0; j < PT; ++j) { f0[j] = f[j]; f1[j] = f[j]; }
         // one call site of the slope for the four stages
         for (int st = 0; st < 4; ++st) {
-            cell_ee_slope<PT>(a, s, t, k0, f1, fh);
+            cell_ee_slope<PT, W>(a, s, t, k0, f1, fh);
             const double w = st < 2 ? 0.5 * h : (st == 2 ? h : h / 6.0);
             const double u = st == 1 ? 2.0 / 3.0 : (st == 3 ? 1.0 : 1.0 / 3.0);
 #pragma unroll
@@ -1071,44 +1071,64 @@ __device__ __forceinline__ void point_coeffs(const CollideArgs& a, const CoeffP&
     tri.a[k] = ta; tri.b[k] = tb; tri.c[k] = tc;
 }
 
-template <typename TP, int G, int R, int PT>
+// W: the warps that hold the row, PT points a thread; CW: the CTA's.  The CTA's other warps join for the coefficients (a
+// point a thread, whose divisions are a chain each) and the solves.
+template <typename TP, int G, int R, int PT, int W, int CW>
 __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long long cell, double* smem) {
     const int n = a.np;
-    const int pts = PT * (int)blockDim.x;
+    constexpr int pts = PT * 32 * W;
     const CellSmem s = carve_cell(smem, n, pts);
-    const int k0 = PT * (int)threadIdx.x;
-    PointTab<PT> t;
-    load_tab<PT>(a, k0, t);
-    const StepP sp = step_params(a);
-    double f[PT];
+    if (threadIdx.x < 32 * W) {
+        const int k0 = PT * (int)threadIdx.x;
+        PointTab<PT> t;
+        load_tab<PT>(a, k0, t);
+        const StepP sp = step_params(a);
+        double f[PT];
 #pragma unroll
-    for (int j = 0; j < PT; ++j) f[j] = k0 + j < n ? a.f00[cell * n + k0 + j] : 0.0;
-    if (threadIdx.x == 0) { s.f[-1] = 0.0; s.f[pts] = 0.0; s.g[-1] = 0.0; s.g[pts] = 0.0; }
-    if (a.do_ee) {
-        cell_ee<PT>(a, sp, s, t, k0, f);
+        for (int j = 0; j < PT; ++j) f[j] = k0 + j < n ? a.f00[cell * n + k0 + j] : 0.0;
+        if (threadIdx.x == 0) { s.f[-1] = 0.0; s.f[pts] = 0.0; s.g[-1] = 0.0; s.g[pts] = 0.0; }
+        if (a.do_ee) {
+            cell_ee<PT, W>(a, sp, s, t, k0, f);
 #pragma unroll
-        for (int j = 0; j < PT; ++j)
-            if (k0 + j < n) a.f00[cell * n + k0 + j] = f[j];
+            for (int j = 0; j < PT; ++j)
+                if (k0 + j < n) a.f00[cell * n + k0 + j] = f[j];
+        }
+        if (a.do_l1 || a.do_lm) {
+            double fm[PT], fp[PT], I2[PT], I0[PT], J1m[PT], S4, S2;
+            neighbours<PT, W>(s.f, k0, f, fm, fp);
+            cell_scans<PT, W>(t, f, fm, fp, s.tot, I2, I0, J1m, S4, S2);
+            const double temperature = S4 * (4.0 * M_PI), density = S2 * (4.0 * M_PI);
+            if ((int)threadIdx.x >= 32 * (W - 1)) {
+                const double l = log_ee(density, temperature, a.density_np);
+                if ((threadIdx.x & 31) == 0) s.one[0] = l;
+            }
+            if (threadIdx.x < 32) {
+                const double l = zlog_ei(density, temperature, a.density_np, a.Zeta);
+                if (threadIdx.x == 0) { s.one[1] = l; s.one[2] = density; }
+            }
+            if constexpr (CW > W) {
+#pragma unroll
+                for (int j = 0; j < PT; ++j)
+                    if (k0 + j < n) {
+                        s.tri.a[k0 + j] = I2[j]; s.tri.b[k0 + j] = I0[j]; s.tri.c[k0 + j] = J1m[j]; s.tri.scat[k0 + j] = f[j];
+                    }
+            } else {
+                __syncthreads();
+                const CoeffP c = coeff_params(a, sp, s.one[0], s.one[1], density);
+#pragma unroll
+                for (int j = 0; j < PT; ++j)
+                    if (k0 + j < n) point_coeffs(a, c, s.tri, k0 + j, f[j], I2[j], I0[j], J1m[j], t.U3[j]);
+            }
+        }
     }
     if (!a.do_l1 && !a.do_lm) return;
-    double fm[PT], fp[PT], I2[PT], I0[PT], J1m[PT], S4, S2;
-    neighbours<PT>(s.f, k0, f, fm, fp);
-    cell_scans<PT>(t, f, fm, fp, s.tot, I2, I0, J1m, S4, S2);
-    const double temperature = S4 * (4.0 * M_PI), density = S2 * (4.0 * M_PI);
-    if (threadIdx.x + 32 >= blockDim.x) {
-        const double l = log_ee(density, temperature, a.density_np);
-        if ((threadIdx.x & 31) == 0) s.one[0] = l;
-    }
-    if (threadIdx.x < 32) {
-        const double l = zlog_ei(density, temperature, a.density_np, a.Zeta);
-        if (threadIdx.x == 0) s.one[1] = l;
-    }
     __syncthreads();
-    const CoeffP c = coeff_params(a, sp, s.one[0], s.one[1], density);
-#pragma unroll
-    for (int j = 0; j < PT; ++j)
-        if (k0 + j < n) point_coeffs(a, c, s.tri, k0 + j, f[j], I2[j], I0[j], J1m[j], t.U3[j]);
-    __syncthreads();
+    if constexpr (CW > W) {
+        const int k = threadIdx.x;
+        const CoeffP c = coeff_params(a, step_params(a), s.one[0], s.one[1], s.one[2]);
+        if (k < n) point_coeffs(a, c, s.tri, k, s.tri.scat[k], s.tri.a[k], s.tri.b[k], s.tri.c[k], __ldg(a.U3 + k));
+        __syncthreads();
+    }
     cell_solves<TP, G, R>(a, s.tri, cell);
 }
 
@@ -1200,17 +1220,18 @@ __device__ __forceinline__ void solve_cell(const CollideArgs& a, const long long
 // before) 0.88 -> 0.2 ms; 512 uneven 1D problems 9.0 -> 7.2 ms a step.  Long e-e runs on few cells wait on the slope's
 // three barriers and its logarithm; for many cells see collide_solve_kernel.
 template <typename TP, int K, bool MANY>
-__global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K, MANY)) collide_cell_kernel(const CollideArgs a) {
+__global__ void __launch_bounds__(32 * cell_warps(K, MANY), form_blocks(K, MANY)) collide_cell_kernel(const CollideArgs a) {
     extern __shared__ double smem[];
     for (long long cell = blockIdx.x; cell < a.cells; cell += gridDim.x) {
-        collide_cell<TP, form_lanes(K), form_run(K), form_points(K)>(a, cell, smem);
+        collide_cell<TP, form_lanes(K), form_run(K), form_points(K), form_warps(K), cell_warps(K, MANY)>(a, cell, smem);
         __syncthreads();
     }
 }
 
-// The e-e substeps alone, for more cells than a wave: without the solves' registers 18 to 24 warps an SM (ee_blocks).
-// 20000 cells, one substep, in the kernel above -> here: 96 points 169 -> 162 us, 128 228 -> 198, 200 443 -> 389, 257
-// 877 -> 372 (two CTAs an SM for one).
+// The e-e substeps alone, for more cells than a wave: without the solves' registers 18 to 20 warps an SM of one thread a
+// point, 15 or 16 of two (ee_blocks).
+// 20000 cells, one substep, in the kernel above -> here: 96 points 169 -> 162 us, 128 228 -> 198, 257 877 -> 372 (two
+// CTAs an SM for one); with the joins' counts known to the compiler 154, 189, 282.
 template <int K>
 __global__ void __launch_bounds__(32 * form_warps(K), ee_blocks(K)) collide_ee_kernel(const CollideArgs a) {
     extern __shared__ double smem[];
@@ -1225,7 +1246,7 @@ __global__ void __launch_bounds__(32 * form_warps(K), ee_blocks(K)) collide_ee_k
         double f[PT];
 #pragma unroll
         for (int j = 0; j < PT; ++j) f[j] = k0 + j < n ? a.f00[cell * n + k0 + j] : 0.0;
-        cell_ee<PT>(a, sp, s, t, k0, f);
+        cell_ee<PT, form_warps(K)>(a, sp, s, t, k0, f);
 #pragma unroll
         for (int j = 0; j < PT; ++j)
             if (k0 + j < n) a.f00[cell * n + k0 + j] = f[j];
@@ -1235,7 +1256,7 @@ __global__ void __launch_bounds__(32 * form_warps(K), ee_blocks(K)) collide_ee_k
 // Coefficients and solves of many cells, one warp a cell: 16 cells an SM under way where CTAs of their own leave 2 to 8,
 // most of whose lanes wait for the one that has the plane.  collide_f1 alone, l0 = 1, 20000 cells, a CTA a cell -> here:
 // 64 points 150 -> 96 us, 128 289 -> 101, 257 1161 -> 250; a whole collision step of 96 points 289 -> 237, of 200
-// 788 -> 530; Weibel (16384 cells of 96 points, 48 planes), the whole step 3.55 -> 3.47 ms, FP32 split 2.68 -> 2.61.
+// 788 -> 530 (of 129 points and more the form has changed since); Weibel (16384 cells of 96 points, 48 planes), the whole step 3.55 -> 3.47 ms, FP32 split 2.68 -> 2.61.
 template <typename TP, int K>
 __global__ void __launch_bounds__(32, solve_blocks(K)) collide_solve_kernel(const CollideArgs a) {
     extern __shared__ double smem[];
@@ -1256,7 +1277,7 @@ __global__ void __launch_bounds__(32 * form_warps(K), form_blocks(K, true)) coll
         const int* src = reinterpret_cast<const int*>(b.probs + w.x);
         for (int i = threadIdx.x; i < (int)(sizeof(CollideArgs) / 4); i += blockDim.x) reinterpret_cast<int*>(&a)[i] = src[i];
         __syncthreads();
-        collide_cell<TP, form_lanes(K), form_run(K), form_points(K)>(a, (long long)w.y, smem);
+        collide_cell<TP, form_lanes(K), form_run(K), form_points(K), form_warps(K), form_warps(K)>(a, (long long)w.y, smem);
         __syncthreads();
     }
 }
@@ -1317,7 +1338,7 @@ int collide_form(int np) {
 // group's work shortest, a unit's pivots counted as three planes
 int collide_unit_planes(int np, int l0, int m0, int mmax_coll, int do_l1, int do_lm, int warps) {
     if (np > 512) return 1;
-    const int K = collide_form(np), groups = 32 * (warps ? warps : form_warps(K)) / form_lanes(K);
+    const int K = collide_form(np), groups = 32 * (warps ? warps : cell_warps(K, false)) / form_lanes(K);
     int best = 1, cost = 1 << 30;
     const int widest = 1 + 2 * std::min(std::min(l0, m0), mmax_coll);
     for (int C = 1; C <= widest; ++C) {
@@ -1344,7 +1365,7 @@ cudaError_t launch_cell(const CollideArgs& a0, cudaStream_t st, int blocks) {
         int planes = 0;   // that this call solves
         for (int l = 1; l <= a.l0; ++l)
             if (l == 1 ? a.do_l1 : a.do_lm) planes += 1 + 2 * std::min(std::min(l, a.m0), a.mmax_coll);
-        const int groups = 32 * form_warps(K) / form_lanes(K);
+        const int groups = 32 * cell_warps(K, false) / form_lanes(K);
         // A CTA a cell leaves the lane groups that have no plane idle while the others solve, and only few cells are
         // resident.  A wave of such CTAs is as good as warps of their own (collide_solve_kernel) up to these numbers of
         // cells: one wave where most groups are idle, about one wave of the warps (one and a half with e-e substeps, which
@@ -1355,7 +1376,9 @@ cudaError_t launch_cell(const CollideArgs& a0, cudaStream_t st, int blocks) {
         const bool idle = a.do_ee || K > 32 ? 4 * planes <= groups : 5 * planes <= 3 * groups;
         const long long limit = idle ? form_blocks(K, true) * sms : planes > groups ? 4 * wave : a.do_ee ? 3 * wave / 2 : wave;
         const bool split = a.cells > limit, wide = a.cells > form_blocks(K, false) * sms;   // wide: more than a wave
-        if (a.do_ee && (split || (!planes && wide))) {
+        // (e-e alone on cells that only the many form's wave holds: 1000 cells of 96 points, 15 substeps, 208 -> 191 us)
+        const bool in_wave = !planes && a.cells > ee_blocks(K) * sms && a.cells <= form_blocks(K, true) * sms;
+        if (a.do_ee && !in_wave && (split || (!planes && wide))) {
             collide_ee_kernel<K><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
             const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess || !planes) return e;
@@ -1367,12 +1390,12 @@ cudaError_t launch_cell(const CollideArgs& a0, cudaStream_t st, int blocks) {
             return cudaGetLastError();
         }
         if constexpr (form_blocks(K, true) > form_blocks(K, false)) {
-            if (wide && planes <= kManyPlanes) {
+            if (wide && (form_points(K) > 1 || planes <= kManyPlanes)) {
                 collide_cell_kernel<TP, K, true><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
                 return cudaGetLastError();
             }
         }
-        collide_cell_kernel<TP, K, false><<<blocks, 32 * form_warps(K), cell_smem(a.np), st>>>(a);
+        collide_cell_kernel<TP, K, false><<<blocks, 32 * cell_warps(K, false), cell_smem(a.np), st>>>(a);
         return cudaGetLastError();
     });
 }

@@ -1,5 +1,5 @@
 // Pieces of the CTA-per-cell collision kernels (collide.cu, adjoint.cu): one
-// thread per momentum point (two from 257 points on) for the pointwise work
+// thread per momentum point (in collide.cu two from 129 points on) for the pointwise work
 // and the cumulative integrals, groups of G lanes holding runs of R points for
 // the tridiagonal solves.  Sums of products that end in a state are written with
 // explicit roundings (rounding.cuh): the instances of few and of many cells and
@@ -17,34 +17,41 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 
 // The forms: K = G R / 8 (the row's points, rounded up to the form's, over 8).
-// One thread a point up to 256 points, two beyond.  113 to 128 points take runs
+// One thread a point up to 128 points, two beyond (half the warps' scans and
+// barriers: e-e substeps of 20000 cells of 184 / 200 points 354 / 444 -> 208 / 260
+// us, 1433 cells of 201 points, 15 substeps, f1 and f_lm with them, 575 -> 331,
+// where a warp a cell took 447; 100 cells of 224 points 144 -> 150).  113 to 128 points take runs
 // of 4 on 32 lanes: with 8 on 16 lanes two planes share a warp, but a row's
 // pieces lie 64 bytes apart (20000 cells, l0 = 1, the f1 call 150 -> 101 us;
 // 5000 cells, 15 planes, their call 143 -> 93; 64 cells of 48 planes 29 -> 33).
 constexpr int form_lanes(int K) { return K <= 8 ? 8 : (K < 16 ? 16 : 32); }
 constexpr int form_run(int K) { return 8 * K / form_lanes(K); }
-constexpr int form_points(int K) { return K <= 32 ? 1 : 2; }
+constexpr int form_points(int K) { return K <= 16 ? 1 : 2; }
 constexpr int form_warps(int K) { return (8 * K + 32 * form_points(K) - 1) / (32 * form_points(K)); }
-// Resident CTAs per SM up to 256 points, of 128 registers a thread; more of 80
-// registers for launches of many cells (`many`) and for batches, where a lane's
-// run is shorter than 8 points: more warps hide the FP64 latency.  On few cells
-// the spills cost more (256 cells of 96 points, ten e-e substeps: 118 us
-// against 135).  With few planes (kManyPlanes) the many form is the faster one:
-// 8000 cells of 96 points, 1D, 2 / 8 / 24 planes 138 / 187 / 307 -> 123 / 166 /
-// 293 us; of 184 points 336 / 466 / 750 -> 246 / 350 / 600.  With several
-// planes of one l (m0 >= 2) it depends on how far a row length's form spills: 15
-// planes, 5000 cells, 40 / 72 / 96 / 112 / 128 / 184 points x 1.02 / 0.93 /
-// 1.04 / 1.08 / 0.93 / 0.84; 48 planes x 1.07 / 0.98 / 1.11 / 1.16 / 0.92 /
-// 0.89.
+// warps of one thread a point
+constexpr int point_warps(int K) { return (8 * K + 31) / 32; }
+// Warps of a cell's CTA: of 129 to 256 points, and unless launches of many cells
+// (`many`), twice as many as the pointwise work takes, for the solves
+constexpr int cell_warps(int K, bool many) { return !many && form_points(K) > 1 && K <= 32 ? point_warps(K) : form_warps(K); }
+// Resident CTAs per SM up to 256 points, of 128 registers a thread; up to 128
+// points more of 80 registers for launches of many cells (`many`) and for
+// batches, where a lane's run is shorter than 8 points: more warps hide the FP64
+// latency.  On few cells the spills cost more (256 cells of 96 points, ten e-e
+// substeps: 118 us against 135).  With few planes (kManyPlanes) the many form is
+// the faster one: 8000 cells of 96 points, 1D, 2 / 8 / 24 planes 138 / 187 / 307
+// -> 123 / 166 / 293 us.  With several planes of one l (m0 >= 2) it depends on how
+// far a row length's form spills: 15 planes, 5000 cells, 40 / 72 / 96 / 112 / 128
+// points x 1.02 / 0.93 / 1.04 / 1.08 / 0.93; 48 planes x 1.07 / 0.98 / 1.11 / 1.16
+// / 0.92.  From 129 points on the many form has half the warps and its CTAs hold
+// more cells, whatever the planes (48 planes, 5000 cells of 136 / 192 / 256 points
+// 318 / 382 / 542 -> 296 / 298 / 512 us).
 constexpr int kManyPlanes = 32;
 constexpr int form_blocks(int K, bool many) {
-    return K <= 32 ? (many && form_run(K) < 8 ? 24 : 16) / form_warps(K) : 1;
+    return K > 32 ? 1 : (many && form_points(K) == 1 && form_run(K) < 8 ? 24 : 16) / cell_warps(K, many);
 }
-// the e-e substeps alone: 96 registers a thread (no spills) where that leaves a
-// CTA as many, 20000 cells of 64 / 128 / 184 points 124 / 226 / 364 -> 114 / 198
-// / 331 us against 80 registers; 7 or 8 warps a CTA would then leave two (200
-// points 389 -> 458 us)
-constexpr int ee_blocks(int K) { return K > 32 ? 16 / form_warps(K) : K >= 28 ? 3 : 20 / form_warps(K); }
+// the e-e substeps alone, one thread a point: 96 registers a thread (no spills),
+// 20000 cells of 64 / 128 points 124 / 226 -> 114 / 198 us against 80 registers
+constexpr int ee_blocks(int K) { return (form_points(K) > 1 ? 16 : 20) / form_warps(K); }
 // the solves on a warp a cell
 constexpr int solve_blocks(int K) { return K <= 32 ? 16 : 8; }
 template <typename F>
@@ -192,9 +199,9 @@ __device__ __forceinline__ void load_tab(const A& a, const int k0, PointTab<PT>&
     }
 }
 // shared memory of one cell's CTA (doubles): tri_a, tri_b, tri_c, scat [np],
-// f and G with a point of padding on both sides, the warps' totals [3][16], two
-// values that one warp computes for all
-__host__ __device__ inline size_t cell_smem_doubles(int np, int pts) { return 4 * (size_t)np + 2 * ((size_t)pts + 2) + 50; }
+// f and G with a point of padding on both sides, the warps' totals [3][16],
+// three values that one warp computes for all
+__host__ __device__ inline size_t cell_smem_doubles(int np, int pts) { return 4 * (size_t)np + 2 * ((size_t)pts + 2) + 51; }
 struct CellSmem {
     TriRows tri;
     double *f, *g, *tot;   // f, g: index -1 .. pts
@@ -210,13 +217,18 @@ __device__ __forceinline__ CellSmem carve_cell(double* base, int np, int pts) {
     return s;
 }
 
+// joins the first W warps of the CTA, which do the pointwise work
+template <int W>
+__device__ __forceinline__ void warps_sync() {
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * W) : "memory");
+}
 // The cumulative integrals I4, I2 (k' <= k) and J1 (k' > k) of f at a thread's
 // points, and the whole I4, I2 (S4, S2).  fm, fp: the neighbours.
-template <int PT>
+template <int PT, int W>
 __device__ __forceinline__ void cell_scans(const PointTab<PT>& t, const double (&f)[PT], const double (&fm)[PT],
                                            const double (&fp)[PT], double* tot, double (&I4)[PT], double (&I2)[PT],
                                            double (&J1)[PT], double& S4, double& S2) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double s4 = 0.0, s2 = 0.0, s1 = 0.0;
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
@@ -239,10 +251,11 @@ __device__ __forceinline__ void cell_scans(const PointTab<PT>& t, const double (
     double r1 = __shfl_down_sync(kFull, s1, 1);
     if (lane == 0) { r4 = 0.0; r2 = 0.0; }
     if (lane == 31) r1 = 0.0;
-    __syncthreads();
+    warps_sync<W>();
     double b4 = 0.0, b2 = 0.0, b1 = 0.0;
     S4 = 0.0; S2 = 0.0;
-    for (int w = 0; w < nw; ++w) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
         if (w == warp) { b4 = S4; b2 = S2; }
         S4 += tot[w]; S2 += tot[16 + w];
         if (w > warp) b1 += tot[32 + w];
@@ -260,12 +273,12 @@ __device__ __forceinline__ void cell_scans(const PointTab<PT>& t, const double (
     }
 }
 // a thread's points to shared memory, then its neighbours back
-template <int PT>
+template <int PT, int W>
 __device__ __forceinline__ void neighbours(double* buf, const int k0, const double (&v)[PT], double (&lo)[PT],
                                            double (&hi)[PT]) {
 #pragma unroll
     for (int j = 0; j < PT; ++j) buf[k0 + j] = v[j];
-    __syncthreads();
+    warps_sync<W>();
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
         lo[j] = j > 0 ? v[j > 0 ? j - 1 : 0] : buf[k0 - 1];
