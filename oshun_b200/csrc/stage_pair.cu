@@ -949,7 +949,7 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
                     auto quad = [&](double (&j)[PT], const TS* v, const TS* rf) {
 #pragma unroll
                         for (int k = 0; k < PT; ++k) {
-                            double f = (double)v[k == 0 ? 0 : nb.o2];
+                            double f = (double)v[k == 0 ? 0 : SHIFT ? nb.o2 : 1];
                             if (rf) f = add_rn(f, (double)rf[k == 0 ? pc : pc1]);
                             if (k == 0 ? pv : pv1) j[k] = mul_rn(ldg(a.wj + (k == 0 ? pc : pc1)), f);
                         }
