@@ -2450,17 +2450,18 @@ int oshun_adjoint_vjp(oshun_adjoint a, const double* y, const double* lam_next, 
         const int nsub = (int)((t_new - t_ee) / h->cfg.small_dt) + 1;   // def-FokkerPlanck.cpp:598-599
         const double hsub = (t_new - t_ee) / (double)nsub;
         const double Dt = t_new - t_eb;
-        const long long wsz = adj::coll_ws(h->cfg.nump, h->cfg.l0, nsub);
-        if (wsz * h->cells > a->ws_cap) {
+        const long long need = (long long)nsub * h->pstride;   // the substeps' starts
+        if (need > a->ws_cap) {
             CK(cudaStreamSynchronize(h->stream));
             cudaFree(a->ws);
             a->ws = nullptr;
-            CK(cudaMalloc(&a->ws, sizeof(double) * wsz * h->cells));
-            a->ws_cap = wsz * h->cells;
+            a->ws_cap = 0;
+            CK(cudaMalloc(&a->ws, sizeof(double) * need));
+            a->ws_cap = need;
         }
         const int mmax = h->cfg.if_implicit1D ? 0 : h->cfg.m0;
         CK(launch_collide_adj(adj_tables(h), h->cfg.l0, (int)h->cells, a->y1, a->lam1, 1, 1, nsub, hsub, Dt, a->ws,
-                              wsz, h->stream, h->d_plane_of, h->cfg.m0, mmax));
+                              h->stream, h->d_plane_of, h->cfg.m0, mmax));
     }
     // RK4 transpose
     const adj::Grid1 g = adj_grid(a);

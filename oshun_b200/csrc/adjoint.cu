@@ -314,17 +314,19 @@ __global__ void to_fp64_kernel(const float* __restrict__ src, double* __restrict
 
 // K: the form of collide_cell.cuh (nump <= 256: one thread a point).  16 warps
 // an SM: the e-e sweeps, most of a cell's time, hold far fewer registers than
-// the solves, which spill a little for it.
+// the solves, which spill a little for it.  ws: the substeps' starts of every
+// cell, nsub rows; shared memory for them would leave fewer CTAs an SM (600 cells
+// of 64 points, 90 substeps: a step's transpose 3.34 ms against 1.96; five
+// substeps 0.34 either way).
 template <int K>
 __global__ void __launch_bounds__(32 * point_warps(K), 16 / point_warps(K))
     collide_adj_kernel(const CollTables T, const adjc::StepT st, const double* __restrict__ y, double* __restrict__ lam,
-                       double* __restrict__ ws, const long long wsz, const int smem_ws) {
+                       double* __restrict__ ws) {
     extern __shared__ double smem[];
     const long long x = blockIdx.x;
     const int np = T.np;
-    double* starts = smem_ws ? smem + adjc::cell_doubles(np, blockDim.x) : ws + x * wsz;
-    adjc::collide_cell_T<form_lanes(K), form_run(K), point_warps(K)>(T, st, y + x * np, y + st.pstride + x * np, lam + x * np,
-                                                     lam + st.pstride + x * np, smem, starts);
+    adjc::collide_cell_T<form_lanes(K), form_run(K), point_warps(K)>(
+        T, st, y + x * np, y + st.pstride + x * np, lam + x * np, lam + st.pstride + x * np, smem, ws + x * st.nsub * np);
 }
 
 // out = a0 v0 + a1 v1 and, where acc is given, acc = base + v1
@@ -364,23 +366,17 @@ cudaError_t launch_convert(const float* src, double* dst, long long n, cudaStrea
 }
 
 cudaError_t launch_collide_adj(const CollTables& T, int l0, int nx, const double* y, double* lam, int ee, int eb,
-                               int nsub, double hsub, double Dt, double* ws, long long wsz, cudaStream_t st,
-                               const int* plane_of, int m0, int mmax) {
-    // ws: the substep starts of the cells where a CTA's shared memory does not hold them
-    if (T.np > 256 || (long long)nsub * T.np > wsz) return cudaErrorInvalidValue;
+                               int nsub, double hsub, double Dt, double* ws, cudaStream_t st, const int* plane_of,
+                               int m0, int mmax) {
+    if (T.np > 256) return cudaErrorInvalidValue;
     const int K = collide_form(T.np);
     const adjc::StepT s{l0, m0, mmax, collide_unit_planes(T.np, l0, m0, mmax, 1, 1), ee, eb, nsub, hsub, Dt, plane_of,
                         (long long)nx * T.np};   // nx: the cells of the grid
     return with_form(K, [&](auto form) {
         constexpr int F = decltype(form)::value;
         if constexpr (F <= 32) {
-            const size_t base = sizeof(double) * adjc::cell_doubles(T.np, 32 * point_warps(F));
-            const size_t starts = sizeof(double) * (size_t)nsub * T.np;
-            const int in_smem = base + starts <= 100 * 1024;
-            const size_t smem = base + (in_smem ? starts : 0);
-            const cudaError_t e = ensure_dyn_smem((const void*)collide_adj_kernel<F>, smem);
-            if (e != cudaSuccess) return e;
-            collide_adj_kernel<F><<<nx, 32 * point_warps(F), smem, st>>>(T, s, y, lam, ws, wsz, in_smem);
+            const size_t smem = sizeof(double) * adjc::cell_doubles(T.np, 32 * point_warps(F));
+            collide_adj_kernel<F><<<nx, 32 * point_warps(F), smem, st>>>(T, s, y, lam, ws);
             return cudaGetLastError();
         }
         return cudaErrorInvalidValue;

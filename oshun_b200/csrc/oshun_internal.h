@@ -231,8 +231,9 @@ cudaError_t launch_stage_vjp(const adj::Grid1& g, const double* s, const double*
 // FP64 state vector <-> FP32 planes/fields (the FP32 bulk adjoint)
 cudaError_t launch_convert(const double* src, float* dst, long long n, cudaStream_t st);
 cudaError_t launch_convert(const float* src, double* dst, long long n, cudaStream_t st);
+// ws: nsub rows of every cell
 cudaError_t launch_collide_adj(const adj::CollTables& T, int l0, int nx, const double* y, double* lam, int ee, int eb,
-                               int nsub, double hsub, double Dt, double* ws, long long wsz, cudaStream_t st,
+                               int nsub, double hsub, double Dt, double* ws, cudaStream_t st,
                                const int* plane_of, int m0, int mmax);
 // out = a0 v0 + a1 v1 (v1 may be null) and, where acc is given, acc = base + v1
 cudaError_t launch_rk_combine(double* out, const double* v0, double a0, const double* v1, double a1, double* acc,
