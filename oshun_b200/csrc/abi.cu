@@ -633,10 +633,10 @@ int build_tables(oshun_ctx* h) {
 }
 
 // one stage launch: the state sets it reads and writes (out < 0: no stage
-// output) and its weights in units of the step
+// output), what its slope is multiplied by, dt/div, and what Y takes of that
 struct StageSets {
     int in, B, A, out, kind;
-    double c1, c2;
+    double div, c2;
 };
 template <typename TS>
 StageArgs<TS> stage_launch_args(const oshun_ctx* h, const StageSets& q, double dt) {
@@ -644,7 +644,7 @@ StageArgs<TS> stage_launch_args(const oshun_ctx* h, const StageSets& q, double d
     a.f00_B = h->f00[q.B]; a.pl_B = (const TS*)h->pl[q.B]; a.fld_B = (const TS*)h->fld[q.B];
     a.f00_A = h->f00[q.A]; a.pl_A = (TS*)h->pl[q.A]; a.fld_A = (TS*)h->fld[q.A];
     if (q.out >= 0) { a.f00_out = h->f00[q.out]; a.pl_out = (TS*)h->pl[q.out]; a.fld_out = (TS*)h->fld[q.out]; }
-    a.c1 = dt * q.c1; a.c2 = q.c2;
+    a.c1 = dt / q.div; a.c2 = q.c2;
     return a;
 }
 
@@ -670,10 +670,10 @@ int launch_stage(oshun_ctx* h, const StageSets& q, int parts = kPartAll, const C
 // set B into set A: the stage inputs are B, Sa, Sb, Sa
 StageSets rk4_sets(int k, int B, int A, int Sa, int Sb) {
     switch (k) {
-        case 1: return {B, B, A, Sa, kStageFirst, 0.5, 1.0 / 3.0};
-        case 2: return {Sa, B, A, Sb, kStageMid, 0.5, 2.0 / 3.0};
+        case 1: return {B, B, A, Sa, kStageFirst, 2.0, 1.0 / 3.0};
+        case 2: return {Sa, B, A, Sb, kStageMid, 2.0, 2.0 / 3.0};
         case 3: return {Sb, B, A, Sa, kStageMid, 1.0, 1.0 / 3.0};
-        default: return {Sa, B, A, -1, kStageLast, 1.0 / 6.0, 1.0};
+        default: return {Sa, B, A, -1, kStageLast, 6.0, 1.0};
     }
 }
 
@@ -891,7 +891,7 @@ ImplicitArgs implicit_args(const oshun_ctx* h) {
 int enqueue_rk2(oshun_ctx* h, int S, int T, int U, int parts, const CoefLM* coef, const void* fld_in) {
     int rc = launch_stage(h, {S, S, T, U, kStageFirst, 1.0, 0.5}, parts, coef, fld_in);
     if (rc) return rc;
-    return launch_stage(h, {U, S, T, -1, kStageLast, 0.5, 1.0}, parts, coef, fld_in);
+    return launch_stage(h, {U, S, T, -1, kStageLast, 2.0, 1.0}, parts, coef, fld_in);
 }
 
 // Implicit_E_Field::advance (def-ImplicitE.cpp:471-676) on set cur at RK time t
@@ -2252,7 +2252,7 @@ int launch_stage_vec(oshun_ctx* h, int k, const double* in, const double* B, dou
     a.f00_B = B; a.pl_B = B + ps; a.fld_B = B + pf;
     a.f00_A = A; a.pl_A = A + ps; a.fld_A = A + pf;
     if (out) { a.f00_out = out; a.pl_out = out + ps; a.fld_out = out + pf; }
-    a.c1 = h->cfg.dt * q.c1; a.c2 = q.c2;
+    a.c1 = h->cfg.dt / q.div; a.c2 = q.c2;
     const cudaError_t e = launch_stage_fp64(a, h->mc, h->stream);
     if (e != cudaSuccess) { set_error(std::string("rk stage launch: ") + cudaGetErrorString(e)); return OSHUN_ERR_CUDA; }
     return OSHUN_OK;
