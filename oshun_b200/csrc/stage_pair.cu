@@ -72,6 +72,7 @@ namespace {
 constexpr int kMaxDepth = 12;                 // slots of either ring
 constexpr int kMinSrc = 3, kMinTgt = 3;       // fewest slots a plan may have
 constexpr int kJBuf = 8;                      // tiles whose current sums can be open at once (see consume_tile)
+static_assert(kMaxDepth / 2 + 1 < kJBuf, "sets of current sums");
 
 // a consumer warp's wait: when it runs out the whole warp reports and stops
 // (the lanes decide together), so the code behind a wait has no failure path;
@@ -992,8 +993,10 @@ __device__ __forceinline__ void consume_tile(const StageArgs<TS>& a, const CoefS
     // the cell's current: sums over 32 points to shared memory; the last
     // half-warp of the cell adds them in order and updates E and B.  No
     // barrier joins the consumer warps: a warp whose wait ran out stops on its
-    // own.  A warp can be at most kMaxDepth slots, two or more of them a tile,
-    // ahead of another, so kJBuf sets of sums are enough.
+    // own.  A source slot is filled again only when every warp has released it,
+    // also in slope launches (no operand ring): a warp can be at most kMaxDepth
+    // slots, two or more of them a tile, ahead of one that is still adding, so
+    // kJBuf sets of sums are enough.
     auto total = [&](double (&j)[PT]) -> double {
 #pragma unroll
         for (int off = kSeg / 2; off > 0; off >>= 1)
@@ -1157,9 +1160,7 @@ cudaError_t pair_form(const StageArgs<TS>& a, cudaStream_t s) {
         if (per_sm_ctas > tile_min_blocks<MC>()) per_sm_ctas = tile_min_blocks<MC>();
     }
     const long long resident = (long long)sm_count() * per_sm_ctas;
-    // a slope launch has no operand ring to hold the warps of a CTA within a
-    // tile or two of each other's current sums: one tile a CTA
-    const long long blocks = a.kind == kStageSlope ? tiles : (tiles < resident ? tiles : resident);
+    const long long blocks = tiles < resident ? tiles : resident;
     kernel<<<dim3((unsigned)blocks), dim3(threads), P.total, s>>>(a, P, tx);
     return cudaGetLastError();
 }
