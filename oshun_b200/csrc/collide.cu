@@ -824,17 +824,18 @@ __global__ void __launch_bounds__(32) collide_warp_kernel(const CollideArgs a) {
 //      plane.
 
 // EE_isotropic_conserva::Getslope (def-FokkerPlanck.cpp:192-267): fh = C_ee(fin)
-template <int PT, int W>
+// X: a warp that holds no points takes the logarithm (cell_ee_log)
+template <int PT, int W, int X>
 __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSmem& s, const PointTab<PT>& t,
                                               const int k0, const double (&fin)[PT], double (&fh)[PT]) {
     const int n = a.np;
     double fm[PT], fp[PT], I4[PT], I2[PT], J1[PT], S4, S2;
     neighbours<PT, W>(s.f, k0, fin, fm, fp);
     const double fa = s.f[0], fb = s.f[1];
-    cell_scans<PT, W>(t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
+    cell_scans<PT, W, X>(t, fin, fm, fp, s.tot, I4, I2, J1, S4, S2);
     // the logarithm of the whole cell on the last warp (the first has the fit below): every warp
     // of its own would spend as many FP64 instructions on it as on all the rest of the slope
-    if ((int)threadIdx.x >= 32 * (W - 1)) {
+    if (X == 0 && (int)threadIdx.x >= 32 * (W - 1)) {
         const double norm = a.c_kpre * log_ee(4.0 * M_PI * S2, 4.0 * M_PI * S4, a.density_np);
         if ((threadIdx.x & 31) == 0) s.one[0] = norm;
     }
@@ -852,7 +853,7 @@ __device__ __forceinline__ void cell_ee_slope(const CollideArgs& a, const CellSm
             G[j] = fma_rn(fma_rn(t.U3[j], J1[j], I4[j]), fin[j], i2);
         }
     }
-    neighbours<PT, W>(s.g, k0, G, Gm, Gp);
+    neighbours<PT, W, X>(s.g, k0, G, Gm, Gp);
     const double norm = s.one[0];
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
@@ -1007,7 +1008,7 @@ __device__ __forceinline__ void cell_solves(const CollideArgs& a, const TriRows&
 
 // RK4 substeps of Explicit_EC_FP::loop (RungeKutta4_ee::advance,
 // def-FokkerPlanck.cpp:518-553) on a thread's points of the cell's f00
-template <int PT, int W>
+template <int PT, int W, int X>
 __device__ __forceinline__ void cell_ee(const CollideArgs& a, const StepP& sp, const CellSmem& s, const PointTab<PT>& t,
                                         const int k0, double (&f)[PT]) {
     const double h = sp.hsub;
@@ -1017,7 +1018,7 @@ __device__ __forceinline__ void cell_ee(const CollideArgs& a, const StepP& sp, c
         for (int j = 0; j < PT; ++j) { f0[j] = f[j]; f1[j] = f[j]; }
         // one call site of the slope for the four stages
         for (int st = 0; st < 4; ++st) {
-            cell_ee_slope<PT, W>(a, s, t, k0, f1, fh);
+            cell_ee_slope<PT, W, X>(a, s, t, k0, f1, fh);
             const double w = st < 2 ? 0.5 * h : (st == 2 ? h : h / 6.0);
             const double u = st == 1 ? 2.0 / 3.0 : (st == 3 ? 1.0 : 1.0 / 3.0);
 #pragma unroll
@@ -1027,6 +1028,20 @@ __device__ __forceinline__ void cell_ee(const CollideArgs& a, const StepP& sp, c
                 f[j] = fma_rn(d, u, f[j]);
             }
         }
+    }
+}
+
+// the logarithms of all its slopes, on a warp of their own
+template <int W>
+__device__ __forceinline__ void cell_ee_log(const CollideArgs& a, const StepP& sp, const CellSmem& s) {
+    for (int i = 0; i < 4 * sp.nsub; ++i) {
+        warps_sync<W + 1, 2>();
+        double S4 = 0.0, S2 = 0.0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) { S4 += s.tot[w]; S2 += s.tot[16 + w]; }
+        const double norm = a.c_kpre * log_ee(4.0 * M_PI * S2, 4.0 * M_PI * S4, a.density_np);
+        if ((threadIdx.x & 31) == 0) s.one[0] = norm;
+        warps_sync<W + 1, 3>();
     }
 }
 
@@ -1071,14 +1086,16 @@ __device__ __forceinline__ void point_coeffs(const CollideArgs& a, const CoeffP&
     tri.a[k] = ta; tri.b[k] = tb; tri.c[k] = tc;
 }
 
-// W: the warps that hold the row, PT points a thread; CW: the CTA's.  The CTA's other warps join for the coefficients (a
-// point a thread, whose divisions are a chain each) and the solves.
+// W: the warps that hold the row, PT points a thread; CW: the CTA's.  Of the CTA's other warps one takes the slopes'
+// logarithms, all join for the coefficients (a point a thread, whose divisions are a chain each) and the solves.
 template <typename TP, int G, int R, int PT, int W, int CW>
 __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long long cell, double* smem) {
     const int n = a.np;
-    constexpr int pts = PT * 32 * W;
+    constexpr int pts = PT * 32 * W, X = CW > W ? 1 : 0;
     const CellSmem s = carve_cell(smem, n, pts);
-    if (threadIdx.x < 32 * W) {
+    if (X && threadIdx.x >= 32 * W) {
+        if (a.do_ee && threadIdx.x < 32 * (W + 1)) cell_ee_log<W>(a, step_params(a), s);
+    } else {
         const int k0 = PT * (int)threadIdx.x;
         PointTab<PT> t;
         load_tab<PT>(a, k0, t);
@@ -1088,7 +1105,7 @@ __device__ __forceinline__ void collide_cell(const CollideArgs& a, const long lo
         for (int j = 0; j < PT; ++j) f[j] = k0 + j < n ? a.f00[cell * n + k0 + j] : 0.0;
         if (threadIdx.x == 0) { s.f[-1] = 0.0; s.f[pts] = 0.0; s.g[-1] = 0.0; s.g[pts] = 0.0; }
         if (a.do_ee) {
-            cell_ee<PT, W>(a, sp, s, t, k0, f);
+            cell_ee<PT, W, X>(a, sp, s, t, k0, f);
 #pragma unroll
             for (int j = 0; j < PT; ++j)
                 if (k0 + j < n) a.f00[cell * n + k0 + j] = f[j];
@@ -1246,7 +1263,7 @@ __global__ void __launch_bounds__(32 * form_warps(K), ee_blocks(K)) collide_ee_k
         double f[PT];
 #pragma unroll
         for (int j = 0; j < PT; ++j) f[j] = k0 + j < n ? a.f00[cell * n + k0 + j] : 0.0;
-        cell_ee<PT, form_warps(K)>(a, sp, s, t, k0, f);
+        cell_ee<PT, form_warps(K), 0>(a, sp, s, t, k0, f);
 #pragma unroll
         for (int j = 0; j < PT; ++j)
             if (k0 + j < n) a.f00[cell * n + k0 + j] = f[j];

@@ -20,7 +20,8 @@ constexpr unsigned kFull = 0xffffffffu;
 // One thread a point up to 128 points, two beyond (half the warps' scans and
 // barriers: e-e substeps of 20000 cells of 184 / 200 points 354 / 444 -> 208 / 260
 // us, 1433 cells of 201 points, 15 substeps, f1 and f_lm with them, 575 -> 331,
-// where a warp a cell took 447; 100 cells of 224 points 144 -> 150).  113 to 128 points take runs
+// where a warp a cell took 447; few cells, whose logarithms take a warp without
+// points, 100 of 224 points 114 -> 96).  113 to 128 points take runs
 // of 4 on 32 lanes: with 8 on 16 lanes two planes share a warp, but a row's
 // pieces lie 64 bytes apart (20000 cells, l0 = 1, the f1 call 150 -> 101 us;
 // 5000 cells, 15 planes, their call 143 -> 93; 64 cells of 48 planes 29 -> 33).
@@ -218,13 +219,14 @@ __device__ __forceinline__ CellSmem carve_cell(double* base, int np, int pts) {
 }
 
 // joins the first W warps of the CTA, which do the pointwise work
-template <int W>
+template <int W, int BAR = 1>
 __device__ __forceinline__ void warps_sync() {
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * W) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(32 * W) : "memory");
 }
 // The cumulative integrals I4, I2 (k' <= k) and J1 (k' > k) of f at a thread's
 // points, and the whole I4, I2 (S4, S2).  fm, fp: the neighbours.
-template <int PT, int W>
+// X: one warp more waits for the totals
+template <int PT, int W, int X = 0>
 __device__ __forceinline__ void cell_scans(const PointTab<PT>& t, const double (&f)[PT], const double (&fm)[PT],
                                            const double (&fp)[PT], double* tot, double (&I4)[PT], double (&I2)[PT],
                                            double (&J1)[PT], double& S4, double& S2) {
@@ -251,7 +253,8 @@ __device__ __forceinline__ void cell_scans(const PointTab<PT>& t, const double (
     double r1 = __shfl_down_sync(kFull, s1, 1);
     if (lane == 0) { r4 = 0.0; r2 = 0.0; }
     if (lane == 31) r1 = 0.0;
-    warps_sync<W>();
+    if constexpr (X > 0) warps_sync<W + X, 2>();
+    else warps_sync<W>();
     double b4 = 0.0, b2 = 0.0, b1 = 0.0;
     S4 = 0.0; S2 = 0.0;
 #pragma unroll
@@ -273,12 +276,14 @@ __device__ __forceinline__ void cell_scans(const PointTab<PT>& t, const double (
     }
 }
 // a thread's points to shared memory, then its neighbours back
-template <int PT, int W>
+// (X: one warp more joins)
+template <int PT, int W, int X = 0>
 __device__ __forceinline__ void neighbours(double* buf, const int k0, const double (&v)[PT], double (&lo)[PT],
                                            double (&hi)[PT]) {
 #pragma unroll
     for (int j = 0; j < PT; ++j) buf[k0 + j] = v[j];
-    warps_sync<W>();
+    if constexpr (X > 0) warps_sync<W + X, 3>();
+    else warps_sync<W>();
 #pragma unroll
     for (int j = 0; j < PT; ++j) {
         lo[j] = j > 0 ? v[j > 0 ? j - 1 : 0] : buf[k0 - 1];
