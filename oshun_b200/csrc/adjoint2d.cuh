@@ -1,7 +1,7 @@
 // Transpose of the RK4-stage right-hand side for any grid (1D or 2D, any
 // m0): F'(s)^T c at one stage state s, gathered per source point.  The
 // forward is Actions::Adv as the stage kernels compute it (stage_pipe.cuh
-// couple_src3 / couple_f00_row, field_update): for a source harmonic
+// couple_src3 / couple_f00_row, stage_common.cuh field_update): for a source harmonic
 // (s, M) with values f, momentum stencils G, H (wG/wH/wG00 of
 // adjoint_math.h, the reference's ends), x/y differences dx, dy (times v),
 //   (s+1, M)    += ex_g Ex G + ax_p dx          (s-1, M)    += ex_h Ex H + ax_m dx
