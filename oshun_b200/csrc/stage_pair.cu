@@ -1042,9 +1042,9 @@ inline int tile_cells(int np, int nx, int segments) { return batch_cells(np, nx,
 // >= 3).  FP32 rows of 51 points on 64 x 64 cells, l0 = m0 = 6, two steps 2.18
 // -> 1.60 ms with two, in spite of 376 bytes spilled; FP64 rows of 129 points
 // on 30 x 31 cells, l0 = 4, m0 = 2, 646 -> 407 us (128 bytes spilled).
-template <int MC, typename TS, bool SHIFT>
+template <int MC, typename TS>
 constexpr int points() { return sizeof(TS) == 4 || MC <= 2 ? 2 : 1; }
-template <int MC, typename TS, bool SHIFT>
+template <int MC, typename TS>
 constexpr int consumer_warps() {
     if (MC == 0) return 8;
     if (sizeof(TS) == 8) return MC <= 6 ? 10 : 6;
@@ -1055,9 +1055,9 @@ constexpr int consumer_warps() {
 template <int MC>
 constexpr int tile_min_blocks() { return MC == 0 ? 2 : 1; }
 
-// MC: the problem's m0
-template <int MC, typename TS, bool SHIFT>
-__global__ void __launch_bounds__((consumer_warps<MC, TS, SHIFT>() + 2) * 32, tile_min_blocks<MC>())
+// MC: the problem's m0; PT: points of a thread
+template <int MC, typename TS, bool SHIFT, int PT>
+__global__ void __launch_bounds__((consumer_warps<MC, TS>() + 2) * 32, tile_min_blocks<MC>())
     rk_stage_pair_kernel(const __grid_constant__ StageArgs<TS> a, const __grid_constant__ Plan P, const int tx) {
     extern __shared__ __align__(128) unsigned char smem[];
     const Geo g = make_geo(a.np, a.nx, a.ny, tx);
@@ -1110,13 +1110,13 @@ __global__ void __launch_bounds__((consumer_warps<MC, TS, SHIFT>() + 2) * 32, ti
     Consumer cs;
     cs.start(P, smem);
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-        consume_tile<MC, TS, points<MC, TS, SHIFT>(), SHIFT>(a, scoef, splane, g, P, tile, smem, cs, a.err, wlim);
+        consume_tile<MC, TS, PT, SHIFT>(a, scoef, splane, g, P, tile, smem, cs, a.err, wlim);
 }
 
-template <int MC, typename TS, bool SHIFT>
+template <int MC, typename TS, bool SHIFT, int PT>
 cudaError_t pair_form(const StageArgs<TS>& a, cudaStream_t s) {
-    constexpr int per_warp = points<MC, TS, SHIFT>();        // 32-point segments of a warp
-    constexpr int max_hw = per_warp * consumer_warps<MC, TS, SHIFT>();
+    constexpr int per_warp = PT;                             // 32-point segments of a warp
+    constexpr int max_hw = per_warp * consumer_warps<MC, TS>();
     constexpr int elem = (int)sizeof(TS);
     if ((a.np + 31) / 32 > max_hw) return cudaErrorNotSupported;
     int tx = tile_cells(a.np, a.nx, max_hw);
@@ -1148,7 +1148,7 @@ cudaError_t pair_form(const StageArgs<TS>& a, cudaStream_t s) {
             --tx;
         }
     }
-    const auto kernel = rk_stage_pair_kernel<MC, TS, SHIFT>;
+    const auto kernel = rk_stage_pair_kernel<MC, TS, SHIFT, PT>;
     cudaError_t e = ensure_dyn_smem((const void*)kernel, P.total);
     if (e != cudaSuccess) return e;
     const int threads = P.hw * (32 / per_warp) + 64;
@@ -1167,8 +1167,15 @@ cudaError_t pair_form(const StageArgs<TS>& a, cudaStream_t s) {
 
 template <typename TS, int MC>
 cudaError_t pair_mc(const StageArgs<TS>& a, cudaStream_t s) {
-    if ((a.np * (int)sizeof(TS)) % 16 == 0) return pair_form<MC, TS, false>(a, s);
-    return pair_form<MC, TS, true>(a, s);
+    constexpr int PT = points<MC, TS>();
+    if ((a.np * (int)sizeof(TS)) % 16 == 0) return pair_form<MC, TS, false, PT>(a, s);
+    // odd rows of at most a cell an SM: the chain of one tile is the launch, and
+    // twice the warps of one point a thread are the faster ones (8 x 8 cells, l0 = 6,
+    // m0 = 2, a step, one point / two: 33 points 123 / 130 us, 189 points 129 / 132)
+    if constexpr (sizeof(TS) == 8 && (MC == 1 || MC == 2)) {
+        if (a.cells <= sm_count() && (a.np + 31) / 32 <= consumer_warps<MC, TS>()) return pair_form<MC, TS, true, 1>(a, s);
+    }
+    return pair_form<MC, TS, true, PT>(a, s);
 }
 
 // ---------------------------------------------------------------------------
