@@ -388,14 +388,15 @@ cudaError_t launch_stage_vjp2(const adj2::Grid2& g, const double* s, const doubl
     if (threads > 256) return cudaErrorInvalidValue;
     const size_t smem = sizeof(double) * 3 * 8 * (size_t)(g.m0 + 1) * threads;
     // The window pays where the CTAs that its shared memory leaves on an SM hold
-    // all cells, or are four or have five warps; else gathering, with all the
-    // SM's warps, is the faster one.  A step's vjp, us, window / gather: 144 cells
+    // all cells within three waves, or are four or have five warps; else gathering,
+    // with all the SM's warps, is the faster one.  A step's vjp, us, window / gather: 144 cells
     // of 64 points, l0 = m0 = 8, 957 / 1855; 1024 cells, m0 = 4, l0 = 4, 96 points (six
     // warps) 1224 / 1480, 64 points (six) 944 / 950, 128 points (four) 1795 / 1630; l0 =
     // m0 = 6, 64 points (four) 1919 / 1705, 96 points (three) 3134 / 2843, 32 points
-    // (five) 1147 / 1458; m0 = 8, 32 points (four CTAs) 1769 / 2338.
+    // (five) 1147 / 1458; m0 = 8, 32 points (four CTAs) 1769 / 2338; 391 cells of 117
+    // points, l0 = 7, m0 = 4, 2.6 waves, 2119 / 2177.
     const long long fit = (228 * 1024) / (long long)(smem + 1024);
-    if (smem <= 200 * 1024 && (g.cells <= fit * sm_count() || fit >= 4 || fit * (threads / 32) >= 5)) {
+    if (smem <= 200 * 1024 && (g.cells <= 3 * fit * sm_count() || fit >= 4 || fit * (threads / 32) >= 5)) {
         const cudaError_t e = ensure_dyn_smem((const void*)stage_vjp2_kernel, smem);
         if (e != cudaSuccess) return e;
         stage_vjp2_kernel<<<(unsigned)g.cells, threads, smem, st>>>(g, s, c, out);

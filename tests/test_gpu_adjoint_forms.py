@@ -13,7 +13,7 @@ def test_forms_agree(l0, m0, nump):
     import torch
     from oshun_b200 import workloads
     from oshun_b200.adjoint import Run
-    base, copies, ny = 6, 60, 2
+    base, copies, ny = 6, 80, 2
     cfg, _, _ = workloads.sensitivity1d(nx=16, nump=48, length=4.0)
     gen = torch.Generator(device="cuda").manual_seed(13)
     out = []
