@@ -1272,8 +1272,8 @@ __global__ void __launch_bounds__(32 * form_warps(K), ee_blocks(K)) collide_ee_k
 
 // Coefficients and solves of many cells, one warp a cell: 16 cells an SM under way where CTAs of their own leave 2 to 8,
 // most of whose lanes wait for the one that has the plane.  collide_f1 alone, l0 = 1, 20000 cells, a CTA a cell -> here:
-// 64 points 150 -> 96 us, 128 289 -> 101, 257 1161 -> 250; a whole collision step of 96 points 289 -> 237, of 200
-// 788 -> 530 (of 129 points and more the form has changed since); Weibel (16384 cells of 96 points, 48 planes), the whole step 3.55 -> 3.47 ms, FP32 split 2.68 -> 2.61.
+// 64 points 150 -> 96 us, 128 289 -> 101, 257 1161 -> 250; a whole collision step of 96 points 289 -> 237.  Weibel (16384
+// cells of 96 points, 48 planes), the whole step 3.55 -> 3.47 ms, FP32 split 2.68 -> 2.61.
 template <typename TP, int K>
 __global__ void __launch_bounds__(32, solve_blocks(K)) collide_solve_kernel(const CollideArgs a) {
     extern __shared__ double smem[];
